@@ -158,10 +158,7 @@ def generic_layered() -> dict:
 
 def solve_kernel_name(pol) -> str:
     """The persistent solve kernel a policy launches (cgc_engine.cu launch_solve)."""
-    c = pol.ctas_per_sm or 2
-    if c == 2:
-        return "k_solve"
-    return f"k_solve{c}" + ("w" if pol.bfs_warp_min else "")
+    return {2: "k_solve4", 3: "k_solve5", 4: "k_solve8"}[pol.ctas_per_sm or 2]  # by tile groups per SM
 
 
 def profiled_traffic(workload: int):
@@ -176,13 +173,12 @@ def profiled_traffic(workload: int):
     return None
 
 
-# autotune candidates: pulses, region relabels and sweep pairs per cycle, CTAs per SM, warp-per-tile BFS
-# rounds and exclusive sweeps (which only the 4-CTA kernels are measured to gain from)
-BATCH_CANDIDATES = [dict(local_pulses=L, region_relabels=R, sweeps_per_relabel=K, ctas_per_sm=c, bfs_warp_min=bw,
-                         exclusive=ex)
+# autotune candidates: pulses, region relabels and sweep pairs per cycle, tiles per SM and exclusive sweeps
+# (which only the kernel with the most tiles per SM is measured to gain from)
+BATCH_CANDIDATES = [dict(local_pulses=L, region_relabels=R, sweeps_per_relabel=K, ctas_per_sm=c, exclusive=ex)
                     for (L, R, K) in ((4, 2, 8), (2, 4, 4), (2, 4, 8), (4, 2, 4), (4, 4, 8), (8, 2, 8), (2, 4, 6),
                                       (4, 2, 6))
-                    for c in (2, 3, 4) for bw in ((0, 8) if c > 2 else (0,)) for ex in ((0, 1) if c == 4 else (0,))]
+                    for c in (2, 3, 4) for ex in ((0, 1) if c == 4 else (0,))]
 GRID_SCHEDULES = ((4, 2, 8), (2, 4, 4), (8, 2, 8), (4, 2, 16), (2, 4, 8), (4, 4, 8), (4, 2, 6), (2, 4, 6))
 
 
@@ -442,10 +438,9 @@ def main():
     B = Batch([(v.X, v.Y, v.Z)])
     B.bind_inputs(0, d_in[0].data_ptr(), d_in[1].data_ptr(), [t.data_ptr() for t in d_in[2:]])
     B.bind_outputs(0, d_seg[0].data_ptr(), d_seg[1].data_ptr())
-    cands = [Policy(local_pulses=L, region_relabels=R, sweeps_per_relabel=K, ctas_per_sm=c, learned=lr, bfs_warp_min=bw,
-                    exclusive=ex)
+    cands = [Policy(local_pulses=L, region_relabels=R, sweeps_per_relabel=K, ctas_per_sm=c, learned=lr, exclusive=ex)
              for (L, R, K) in GRID_SCHEDULES
-             for c in (2, 3, 4) for lr in ((0, 1, 3) if have_learned else (0,)) for bw in ((0, 8) if c > 2 else (0,))
+             for c in (2, 3, 4) for lr in ((0, 1, 3) if have_learned else (0,))
              for ex in ((0, 1) if c == 4 else (0,))]
     if args.schedule:
         L, R, K, c, lr = (int(x) for x in args.schedule.split(","))

@@ -87,15 +87,12 @@ std::vector<cgc_options> default_candidates() {
   for (int cta : {2, 3, 4})
     for (int R : {1, 2, 4})
       for (int L : {2, 4, 8})
-        for (int K : {4, 8, 16})
-          for (int bw : {0, 8}) {
-            if (bw && cta == 2) continue;  // warp-per-tile BFS rounds exist at 3 and 4 CTAs/SM
-            cgc_options o{};
-            o.struct_size = sizeof(cgc_options);
-            o.local_pulses = L; o.region_relabels = R; o.sweeps_per_relabel = K; o.ctas_per_sm = cta;
-            o.bfs_warp_min = bw;
-            c.push_back(o);
-          }
+        for (int K : {4, 8, 16}) {
+          cgc_options o{};
+          o.struct_size = sizeof(cgc_options);
+          o.local_pulses = L; o.region_relabels = R; o.sweeps_per_relabel = K; o.ctas_per_sm = cta;
+          c.push_back(o);
+        }
   return c;
 }
 

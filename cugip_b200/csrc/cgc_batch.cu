@@ -100,15 +100,14 @@ int pool_enqueue(Pool& p, const cgc_options* opts, int64_t* flows_dev, cudaStrea
   DevPool& d = p.dp;
   CGC_CUDA(cudaMemsetAsync(d.flow, 0, (size_t)p.ninst * 8, stream));
   CGC_CUDA(cudaMemsetAsync(d.stats, 0, S_NSTATS * 8, stream));
-  CGC_CUDA(cudaMemsetAsync(d.err, 0, 4, stream));
-  CGC_CUDA(cudaMemsetAsync(d.bar, 0, 8, stream));
+  CGC_CUDA(cudaMemsetAsync(d.bar, 0, 8, stream));  // and the error word
   CGC_CUDA(cudaMemsetAsync(d.stamp_bfs, 0, (size_t)d.T * 4, stream));
   CGC_CUDA(cudaMemsetAsync(d.stamp_sw, 0, 2 * (size_t)d.T * 4, stream));
   CGC_CUDA(cudaMemsetAsync(d.stamp_inc, 0, (size_t)d.T * 4, stream));
   k_put_all<<<d.T, 128, 0, stream>>>(d, p.d_in);
   note_launch();
   const SolveParams prm = solve_params(o);
-  if (int rc = launch_solve(p, o, d, prm, stream)) return rc;
+  if (int rc = launch_solve(d, o, prm, p.device, p.sms, stream)) return rc;
   bool any_out = false;
   for (uint8_t* q : p.out_ptrs) any_out = any_out || q;
   if (any_out) {

@@ -230,7 +230,8 @@ __global__ void __launch_bounds__(CSR_THREADS) k_csr_solve(CsrDev D, CsrParams p
     acc += now - tmark;
     tmark = now;
   };
-  auto sync = [&]() { return grid_barrier(D.bar, D.err, prm.limit_ns); };
+  uint32_t bar_target = 0;
+  auto sync = [&]() { return grid_barrier(D.bar, bar_target, prm.limit_ns); };
   // frontier BFS over lists L[k&1] with counters cb[k%3]; `visit` appends
   // to the next frontier; returns the number of rounds, -1 on a failed barrier
   auto bfs = [&](auto&& visit) -> int {
@@ -460,7 +461,6 @@ int graph_create(int32_t n, int64_t m, const int32_t* a, const int32_t* b, const
     const int64_t o_cnt = off; off += al(CC_N * 4);
     const int64_t o_fl = off; off += al(8);
     const int64_t o_sta = off; off += al(CS_N * 8);
-    const int64_t o_err = off; off += al(4);
     const int64_t o_bar = off; off += al(8);
     const int64_t o_seg = off; off += al(n);
     const int64_t o_bs = off; off += al((int64_t)nb * 4);
@@ -487,8 +487,8 @@ int graph_create(int32_t n, int64_t m, const int32_t* a, const int32_t* b, const
     d.cnt = (int32_t*)(base + o_cnt);
     d.flow = (unsigned long long*)(base + o_fl);
     d.stats = (unsigned long long*)(base + o_sta);
-    d.err = (int32_t*)(base + o_err);
     d.bar = (uint32_t*)(base + o_bar);
+    d.err = (int32_t*)(d.bar + 1);
     g->seg = (uint8_t*)(base + o_seg);
     int32_t* bsum = (int32_t*)(base + o_bs);
     if (m > 0) {
@@ -557,8 +557,7 @@ int graph_maxflow(cgc_graph* g, const cgc_options* opts, int64_t* flow) {
     CGC_CUDA(cudaEventRecord(ev[0], g->stream));
     CGC_CUDA(cudaMemsetAsync(d.flow, 0, 8, g->stream));
     CGC_CUDA(cudaMemsetAsync(d.stats, 0, CS_N * 8, g->stream));
-    CGC_CUDA(cudaMemsetAsync(d.err, 0, 4, g->stream));
-    CGC_CUDA(cudaMemsetAsync(d.bar, 0, 8, g->stream));
+    CGC_CUDA(cudaMemsetAsync(d.bar, 0, 8, g->stream));  // and the error word
     CGC_CUDA(cudaMemsetAsync(d.cnt, 0, CC_N * 4, g->stream));
     k_csr_prepare<<<grid_blocks(std::max<int64_t>(d.arcs, d.n), 256), 256, 0, g->stream>>>(d); note_launch();
     CGC_CUDA(cudaGetLastError());

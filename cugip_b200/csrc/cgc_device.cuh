@@ -27,7 +27,7 @@ namespace cgc {
 constexpr int TILE = 8;
 constexpr int TV = 512;            // voxels per tile
 constexpr int INF = 0x3fffffff;    // height of vertices that cannot reach the sink
-constexpr int HALO = 1000;         // 10x10x10 heights with a one-voxel halo
+constexpr int MAX_GROUPS = 8;      // tile groups per CTA of the persistent solve
 
 enum Dir { PX = 0, MX = 1, PY = 2, MY = 3, PZ = 4, MZ = 5 };
 
@@ -94,8 +94,8 @@ struct DevPool {
   unsigned long long* flow;   // ninst: flow value (int64 as two's complement)
   const InstGeo* geo;   // ninst
   unsigned long long* stats;  // S_NSTATS
-  int32_t* err;         // first error code raised on the device
-  uint32_t* bar;        // grid barrier: [0] arrivals, [1] generation
+  int32_t* err;         // first error code raised on the device (bar + 1)
+  uint32_t* bar;        // grid barrier: [0] arrivals, [1] the error word
   unsigned long long* trace;  // 2*TRACE_CAP words of phase records (may be null)
   // learned scheduler (null unless used)
   __nv_bfloat16* sfeat;       // T*16 tile features
@@ -121,7 +121,6 @@ struct SolveParams {
   int trace_cycles;      // record scheduling traces for the first trace_cycles relabel cycles
   int64_t max_sweeps;    // cap on sweeps (parity steps)
   uint64_t limit_ns;     // bounded barrier wait
-  int bfs_warp_min = 0;  // BFS rounds with at least this many tiles per CTA run a warp per tile (0: never)
   int exclusive = 0;     // 1: exclusive sweeps (cgc_options.exclusive), 0: parity sweeps
   int incremental = 0;   // 1: global relabels after the first of a solve are incremental (cgc_options.relabel)
 };
@@ -131,11 +130,9 @@ __global__ void k_put_tlinks(DevPool P, int inst, const int32_t* __restrict__ ca
 __global__ void k_put_nlinks(DevPool P, int inst, int axis, const int32_t* __restrict__ fwd,
                              const int32_t* __restrict__ bwd);
 __global__ void k_prepare(DevPool P);
-__global__ void k_solve(DevPool P, SolveParams prm);
-__global__ void k_solve3(DevPool P, SolveParams prm);
 __global__ void k_solve4(DevPool P, SolveParams prm);
-__global__ void k_solve3w(DevPool P, SolveParams prm);
-__global__ void k_solve4w(DevPool P, SolveParams prm);
+__global__ void k_solve5(DevPool P, SolveParams prm);
+__global__ void k_solve8(DevPool P, SolveParams prm);
 __global__ void k_segments(DevPool P, int inst, int which, uint8_t* out, uint8_t mask, uint8_t bg);
 // kernels of cgc_batch.cu
 __global__ void k_put_all(DevPool P, const int32_t* const* __restrict__ in);

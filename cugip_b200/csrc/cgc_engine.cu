@@ -186,11 +186,21 @@ __global__ void k_mask_remap(const uint8_t* __restrict__ src, uint8_t* __restric
   }
 }
 
-// Host-driven schedule: one launch per sweep / BFS round.
-__global__ void __launch_bounds__(512, 2) k_sweep_list(DevPool P, const int32_t* list, const int32_t* cnt, int L, int R) {
-  __shared__ SweepShared S;
+// Host-driven schedule: one launch per sweep / BFS round; 512 threads (sweeps),
+// a tile group (BFS) or a warp (reachability) per list entry.
+__global__ void __launch_bounds__(WIDE) k_sweep_list(DevPool P, const int32_t* list, const int32_t* cnt, int L, int R) {
+  __shared__ WideShared S;
+  const auto tg = TileGroup<WIDE>::of_thread();
   const int n = *cnt;
-  for (int i = blockIdx.x; i < n; i += gridDim.x) sweep_tile<false>(P, list[i], L, R, S, 0, nullptr, nullptr, 0, nullptr, nullptr);
+  for (int i = blockIdx.x; i < n; i += gridDim.x) {
+    const int p = sweep_tile_wide<false>(P, tg, list[i], L, R, false, S, 0, nullptr, nullptr, 0, nullptr, nullptr,
+                                         SweepExtra(), nullptr);
+    if (tg.q == 0) {
+      atomicAdd(P.stats + S_TILES_SWEPT, 1ull);
+      atomicAdd(P.stats + S_PULSES, (unsigned long long)p);
+    }
+    tg.sync();
+  }
 }
 
 __global__ void k_compact(DevPool P, int parity, int32_t* list, int32_t* cnt) {
@@ -208,11 +218,16 @@ __global__ void k_bfs_queue(DevPool P, uint32_t id0, int32_t* list0, int32_t* cn
   bfs_queue_tile(P, blockIdx.x * blockDim.x + threadIdx.x, id0, list0, cnt0);
 }
 
-__global__ void __launch_bounds__(512, 2) k_bfs_round(DevPool P, const int32_t* list, const int32_t* cnt, uint32_t id_next,
-                                                      int32_t* list_next, int32_t* cnt_next) {
-  __shared__ BfsShared S;
+__global__ void __launch_bounds__(GROUP) k_bfs_round(DevPool P, const int32_t* list, const int32_t* cnt, uint32_t id_next,
+                                                     int32_t* list_next, int32_t* cnt_next) {
+  __shared__ __align__(16) BfsShared S;
+  const auto tg = TileGroup<GROUP>::of_thread();
   const int n = *cnt;
-  for (int i = blockIdx.x; i < n; i += gridDim.x) bfs_tile(P, list[i], S, id_next, list_next, cnt_next);
+  for (int i = blockIdx.x; i < n; i += gridDim.x) {
+    const int v = bfs_tile(P, tg, list[i], S, id_next, list_next, cnt_next);
+    if (tg.q == 0 && v) atomicAdd(P.stats + S_TILES_BFS, 1ull);
+    tg.sync();
+  }
 }
 
 __global__ void __launch_bounds__(512) k_reach_init(DevPool P, uint32_t id0, int32_t* list0, int32_t* cnt0) {
@@ -221,17 +236,11 @@ __global__ void __launch_bounds__(512) k_reach_init(DevPool P, uint32_t id0, int
     reach_init_tile_w(P, t, id0, list0, cnt0);
 }
 
-__global__ void __launch_bounds__(512, 2) k_reach_round(DevPool P, const int32_t* list, const int32_t* cnt, uint32_t id_next,
-                                                        int32_t* list_next, int32_t* cnt_next) {
-  __shared__ ReachShared S;
-  const int n = *cnt;
-  for (int i = blockIdx.x; i < n; i += gridDim.x) reach_tile(P, list[i], S, id_next, list_next, cnt_next);
-}
-
-// ---------------------------------------------------------------------------
-// Grid-wide barrier of the persistent solve (bounded waits, cgc_sync.cuh).
-__device__ __forceinline__ bool grid_sync(const DevPool& P, uint64_t limit_ns) {
-  return grid_barrier(P.bar, P.err, limit_ns);
+__global__ void __launch_bounds__(GROUP) k_reach_round(DevPool P, const int32_t* list, const int32_t* cnt, uint32_t id_next,
+                                                       int32_t* list_next, int32_t* cnt_next) {
+  const int n = *cnt, nw = gridDim.x * (blockDim.x >> 5);
+  for (int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += nw)
+    reach_tile_w(P, list[i], id_next, list_next, cnt_next);
 }
 
 __device__ __forceinline__ int ld_cnt(const int32_t* p) { return *(volatile const int32_t*)p; }
@@ -244,7 +253,8 @@ __device__ __forceinline__ int ld_cnt(const int32_t* p) { return *(volatile cons
 // lists (la: na entries, lb: nb).  Four grid barriers.  Returns false when a
 // barrier failed.
 __device__ __forceinline__ bool sched_stage(const DevPool& P, const SolveParams& prm, int cycle, bool learned,
-                                            bool tracing, const int32_t* la, int na, const int32_t* lb, int nb) {
+                                            bool tracing, const int32_t* la, int na, const int32_t* lb, int nb,
+                                            uint32_t& bar_target) {
   const int G = gridDim.x, b = blockIdx.x, tid = threadIdx.x;
   const int gw = b * (blockDim.x >> 5) + (tid >> 5), nw = G * (blockDim.x >> 5);
   // zeros for the inactive tiles, a thread per tile
@@ -266,127 +276,135 @@ __device__ __forceinline__ bool sched_stage(const DevPool& P, const SolveParams&
     const int t = __ldcg(i < na ? la + i : lb + (i - na));
     sched_features_warp(P, t, P.sfeat, tracing ? P.tfeat + ((int64_t)cycle * P.T + t) * SCHED_C : nullptr);
   }
-  if (!grid_sync(P, prm.limit_ns)) return false;
+  if (!grid_barrier(P.bar, bar_target, prm.limit_ns)) return false;
   if (!learned) return true;
   const PoolSpace sp{&P};
   for (int layer = 0; layer < 3; ++layer) {
     sched_layer(sp, layer, pool_io(P, layer), gw, nw, nullptr);
-    if (!grid_sync(P, prm.limit_ns)) return false;
+    if (!grid_barrier(P.bar, bar_target, prm.limit_ns)) return false;
   }
   return true;
 }
 
-// BFS rounds with many tiles run a warp per tile on the first BFS_WARPS warps
-// of each CTA (one WarpBfsSmem slice each).
-constexpr int BFS_WARPS = 8;
-
-union SolveShared {
+// Shared memory of one tile group.
+union TileShared {  // size a multiple of 16: the members are aligned
   SweepShared sw;
   BfsShared bfs;
-  WarpBfsSmem wbfs[BFS_WARPS];
-  ReachShared rc;
-  SchedShared sched;
 };
 
-// The whole solve in one cooperative launch; a CTA of 512 threads is the unit
-// that visits a tile.
-template <bool BFSW = false>
-__device__ __forceinline__ void solve_body(const DevPool& P, const SolveParams& prm, SolveShared& S) {
+// Bookkeeping of a CTA that one thread updates: kept out of the registers,
+// which the visits need.
+struct SolveBook {
+  unsigned long long tmark, t_launch, ns_bfs, ns_sweep, ns_reach, ns_sched;  // CTA 0
+  int ntrace;                                                               // CTA 0
+  unsigned visits_sw[MAX_GROUPS], pulses[MAX_GROUPS], visits_bfs[MAX_GROUPS], visits_chk[MAX_GROUPS];
+  int next[2 * MAX_GROUPS];  // for_entries
+};
+
+// a list entry, loaded ahead of the test that may discard it
+__device__ __forceinline__ int ld_ahead(const int32_t* p) {
+  int v;
+  asm volatile("ld.global.cg.s32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+
+// The whole solve in one cooperative launch of one CTA per SM: its groups of
+// 128 threads each visit a tile at a time, and a grid barrier has one arrival
+// per SM.
+__device__ __forceinline__ void solve_body(const DevPool& P, const SolveParams& prm, TileShared* groups) {
+  __shared__ SolveBook book;
   const int G = gridDim.x, b = blockIdx.x, tid = threadIdx.x;
-  const bool leader = tid == 0;
+  const auto tg = TileGroup<GROUP>::of_thread();
+  const int q = tg.q, grp = tid / GROUP;
+  TileShared& S = groups[grp];
   // warps of the grid, for the passes that visit every tile with a warp
   const int gw = b * (int)(blockDim.x >> 5) + (tid >> 5), nw = G * (int)(blockDim.x >> 5);
-  // Hands out the n entries of a round.  The first entry of CTA b is entry b;
-  // later ones come from the round's counter (C_TAKE0 + round % 3, the next
-  // round's slot is cleared meanwhile) through an atomic issued when the
-  // current visit starts and read when it ends, so visits of uneven cost
-  // spread over the CTAs.
-  __shared__ int s_next;
+  uint32_t bar_target = 0;
+  auto sync = [&]() { return grid_barrier(P.bar, bar_target, prm.limit_ns); };
+  if (tid < MAX_GROUPS) book.visits_sw[tid] = book.pulses[tid] = book.visits_bfs[tid] = book.visits_chk[tid] = 0;
+  if (tid == 0) {
+    book.tmark = book.t_launch = globaltimer_ns();
+    book.ns_bfs = book.ns_sweep = book.ns_reach = book.ns_sched = 0;
+    book.ntrace = 0;
+  }
+  auto list = [&](int k) { return P.lists + (int64_t)k * P.T; };  // 0..2: BFS rounds, 3..6: sweeps
+  // Hands out the n entries of a round to the groups.  Group g of CTA b starts
+  // with entry g * G + b, so the first G entries go to distinct SMs; later ones
+  // come from the round's counter (C_TAKE0 + round % 3, the next round's slot
+  // is cleared meanwhile) through an atomic issued when the current visit
+  // starts and read when it ends, so visits of uneven cost spread over the
+  // groups.  The barrier between visits also lets the next one reuse S.
+  // t0: the group's first entry, if it has one.
   int round_no = 0;
-  auto for_entries = [&](int n, auto&& visit) {
+  auto first_entry = [&](const int32_t* lst) {
+    const int i = grp * G + b;
+    return i < P.T ? ld_ahead(lst + i) : 0;
+  };
+  auto for_entries = [&](const int32_t* lst, int t0, int n, auto&& visit) {
     if (!CGC_IN_BOUNDS(P, n, P.T + 1)) n = P.T;  // a list holds at most T entries
     int32_t* take = P.cnt + C_TAKE0 + round_no % 3;
     if (b == 0 && tid == 0) P.cnt[C_TAKE0 + (round_no + 1) % 3] = 0;
     ++round_no;
-    int i = b;
+    const int first = G * (int)(blockDim.x / GROUP);
+    int i = grp * G + b, j = 2 * grp;
     while (i < n) {
       int nx = 0;
-      if (tid == 0) nx = atomicAdd(take, 1);
-      visit(i);
-      if (tid == 0) s_next = G + nx;
-      __syncthreads();
-      i = s_next;
-      __syncthreads();
+      if (q == 0 && n > first) nx = atomicAdd(take, 1);
+      visit(t0);
+      if (n <= first) break;
+      if (q == 0) book.next[j] = first + nx;
+      tg.sync();
+      i = book.next[j];
+      j ^= 1;
+      if (i < n) t0 = __ldcg(lst + i);
     }
   };
-  int32_t* const bl[3] = {P.lists, P.lists + P.T, P.lists + 2 * P.T};
-  int32_t* const sl[4] = {P.lists + 3 * P.T, P.lists + 4 * P.T, P.lists + 5 * P.T, P.lists + 6 * P.T};
   int32_t* const bc = P.cnt + C_BFS0;
   int32_t* const sc = P.cnt + C_SW0;
   uint32_t bfs_id = 1;
-  int64_t s = 0;        // sweep index; sweep s uses list s&3 and stamp id s+1
-  int64_t sweeps = 0;
-  long long rounds = 0, relabels = 0;
-  unsigned long long ns_bfs = 0, ns_sweep = 0, ns_reach = 0, ns_sched = 0;
-  int traced = 0;
-  uint64_t tmark = globaltimer_ns();
-  const uint64_t t_launch = tmark;
-  int ntrace = 0;
+  int s = 0;        // sweep index; sweep s uses list 3 + (s & 3) and stamp id s + 1
+  int sweeps = 0, rounds = 0, relabels = 0, traced = 0;
   // block 0 records one phase step (after the barrier that ended it)
   auto record = [&](unsigned long long kind, long long index, int tiles) {
-    if (b == 0 && tid == 0 && P.trace && ntrace < TRACE_CAP) {
-      P.trace[2 * ntrace] = (kind << 56) | ((unsigned long long)(index & 0xffffffffll) << 24) | (unsigned)(tiles & 0xffffff);
-      P.trace[2 * ntrace + 1] = globaltimer_ns() - t_launch;
-      ++ntrace;
+    if (b == 0 && tid == 0 && P.trace && book.ntrace < TRACE_CAP) {
+      const int i = book.ntrace++;
+      P.trace[2 * i] = (kind << 56) | ((unsigned long long)(index & 0xffffffffll) << 24) | (unsigned)(tiles & 0xffffff);
+      P.trace[2 * i + 1] = globaltimer_ns() - book.t_launch;
     }
   };
   auto lap = [&](unsigned long long& acc) {
-    const uint64_t now = globaltimer_ns();
-    acc += now - tmark;
-    tmark = now;
+    if (b == 0 && tid == 0) {
+      const uint64_t now = globaltimer_ns();
+      acc += now - book.tmark;
+      book.tmark = now;
+    }
   };
   // Tile rounds of one relabel pass: round 0 visits the entries of list0
-  // (count *cnt0), round k > 0 the tiles round k - 1 queued in bl[k % 3]
+  // (count *cnt0), round k > 0 the tiles round k - 1 queued in list k % 3
   // (bc[1], bc[2] zero on entry).  inval: invalidation visits, otherwise BFS
   // visits.  False when a grid barrier gave up.
-  auto relabel_rounds = [&](int32_t* list0, int32_t* cnt0, bool inval) -> bool {
+  auto relabel_rounds = [&](const int32_t* list0, int32_t* cnt0, bool inval) -> bool {
     int k = 0;
     for (;;) {
-      int32_t* const lst = k == 0 ? list0 : bl[k % 3];
-      int n = ld_cnt(k == 0 ? cnt0 : bc + k % 3);
+      const int32_t* lst = k == 0 ? list0 : list(k % 3);
+      const int t0 = first_entry(lst);
+      const int n = ld_cnt(k == 0 ? cnt0 : bc + k % 3);
       if (n == 0) break;
-      if (!CGC_IN_BOUNDS(P, n, P.T + 1)) n = P.T;  // a list holds at most T entries
       if (b == 0 && tid == 0) bc[(k + 2) % 3] = 0;
       if (inval) {
-        const uint32_t id_inc = (uint32_t)(relabels + 1);
-        for_entries(n, [&](int i) {
-          inval_tile(P, __ldcg(lst + i), S.bfs, bfs_id + k + 1, bl[(k + 1) % 3], bc + (k + 1) % 3, id_inc, sl[0],
-                     P.cnt + C_INC);
+        for_entries(lst, t0, n, [&](int t) {
+          const int v = inval_tile(P, tg, t, S.bfs, bfs_id + k + 1, list((k + 1) % 3), bc + (k + 1) % 3,
+                                   (uint32_t)(relabels + 1), list(3), P.cnt + C_INC);
+          if (q == 0) book.visits_chk[grp] += v;
         });
-      } else if (BFSW && n / G >= prm.bfs_warp_min) {
-        // Throughput-bound round: a warp per tile (no block barriers, a
-        // tile's relaxation costs one warp's issue slots instead of 16),
-        // entries handed out like for_entries, per warp.
-        int32_t* take = P.cnt + C_TAKE0 + round_no % 3;
-        if (b == 0 && tid == 0) P.cnt[C_TAKE0 + (round_no + 1) % 3] = 0;
-        ++round_no;
-        const int wid = tid >> 5;
-        if (wid < BFS_WARPS) {
-          int i = b * BFS_WARPS + wid;
-          while (i < n) {
-            int nx = 0;
-            if ((tid & 31) == 0) nx = atomicAdd(take, 1);
-            bfs_tile_w(P, __ldcg(lst + i), S.wbfs[wid], bfs_id + k + 1, bl[(k + 1) % 3], bc + (k + 1) % 3);
-            i = G * BFS_WARPS + __shfl_sync(0xffffffffu, nx, 0);
-          }
-        }
       } else {
-        for_entries(n, [&](int i) {
-          bfs_tile(P, __ldcg(lst + i), S.bfs, bfs_id + k + 1, bl[(k + 1) % 3], bc + (k + 1) % 3);
+        for_entries(lst, t0, n, [&](int t) {
+          const int v = bfs_tile(P, tg, t, S.bfs, bfs_id + k + 1, list((k + 1) % 3), bc + (k + 1) % 3);
+          if (q == 0) book.visits_bfs[grp] += v;
         });
       }
       ++k;
-      if (!grid_sync(P, prm.limit_ns)) return false;
+      if (!sync()) return false;
       record(TR_BFS_ROUND, rounds + k, n);
     }
     bfs_id += k + 1;
@@ -407,27 +425,27 @@ __device__ __forceinline__ void solve_body(const DevPool& P, const SolveParams& 
       P.cnt[C_INC] = 0;
     }
     round_no = 0;
-    if (!grid_sync(P, prm.limit_ns)) return;
+    if (!sync()) return;
     if (!inc) {
-      for (int t = gw; t < P.T; t += nw) bfs_init_tile_w(P, t);  // a warp per tile in both shapes
-      if (!grid_sync(P, prm.limit_ns)) return;
-      for (int t0 = b * blockDim.x; t0 < P.T; t0 += G * blockDim.x) bfs_queue_tile(P, t0 + tid, bfs_id, bl[0], bc + 0);
-      if (!grid_sync(P, prm.limit_ns)) return;
-      if (!relabel_rounds(bl[0], bc + 0, false)) return;
+      for (int t = gw; t < P.T; t += nw) bfs_init_tile_w(P, t);  // a warp per tile
+      if (!sync()) return;
+      for (int t0 = b * blockDim.x; t0 < P.T; t0 += G * blockDim.x) bfs_queue_tile(P, t0 + tid, bfs_id, list(0), bc + 0);
+      if (!sync()) return;
+      if (!relabel_rounds(list(0), bc + 0, false)) return;
     } else {
       // invalidation from the tiles the last cycle queued, then BFS rounds
-      // from the tiles with dropped voxels (listed in sl[0], free until the
+      // from the tiles with dropped voxels (listed in list 3, free until the
       // sweep lists are rebuilt below)
       for (int t0 = b * blockDim.x; t0 < P.T; t0 += G * blockDim.x)
-        inval_queue_tile(P, t0 + tid, c0, prm.exclusive != 0, bfs_id, bl[0], bc + 0);
-      if (!grid_sync(P, prm.limit_ns)) return;
-      if (!relabel_rounds(bl[0], bc + 0, true)) return;
+        inval_queue_tile(P, t0 + tid, c0, prm.exclusive != 0, bfs_id, list(0), bc + 0);
+      if (!sync()) return;
+      if (!relabel_rounds(list(0), bc + 0, true)) return;
       if (b == 0 && tid == 0) bc[0] = bc[1] = bc[2] = 0;
-      if (!grid_sync(P, prm.limit_ns)) return;
-      if (!relabel_rounds(sl[0], P.cnt + C_INC, false)) return;
+      if (!sync()) return;
+      if (!relabel_rounds(list(3), P.cnt + C_INC, false)) return;
     }
     ++relabels;
-    lap(ns_bfs);
+    lap(book.ns_bfs);
     // ------------------------------------------------ active tiles -> parity lists
     s += 2;  // fresh stamp ids for the lists built here
     c0 = (uint32_t)s;
@@ -436,23 +454,23 @@ __device__ __forceinline__ void solve_body(const DevPool& P, const SolveParams& 
       const bool a = t < P.T && __ldcg(P.act + t);
       const int par = a ? __ldcg(P.tpar + t) : 0;
       if (prm.exclusive) {  // one list: the whole active set is queued for sweep s
-        if (a) P.stamp_sw[(s & 1) * P.T + t] = (uint32_t)(s + 1);
-        warp_append(P, a, t, sl[s & 3], sc + (s & 3));
+        if (a) P.stamp_sw[(int64_t)(s & 1) * P.T + t] = (uint32_t)(s + 1);
+        warp_append(P, a, t, list(3 + (s & 3)), sc + (s & 3));
       } else {              // one list per parity, for sweeps s and s + 1
         if (a) P.stamp_sw[t] = (uint32_t)(s + par + 1);
-        warp_append(P, a && par == 0, t, sl[s & 3], sc + (s & 3));
-        warp_append(P, a && par == 1, t, sl[(s + 1) & 3], sc + ((s + 1) & 3));
+        warp_append(P, a && par == 0, t, list(3 + (s & 3)), sc + (s & 3));
+        warp_append(P, a && par == 1, t, list(3 + ((s + 1) & 3)), sc + ((s + 1) & 3));
       }
     }
-    if (!grid_sync(P, prm.limit_ns)) return;
+    if (!sync()) return;
     const int nact = ld_cnt(sc + (s & 3)) + ld_cnt(sc + ((s + 1) & 3));
     record(TR_RELABEL_DONE, relabels, nact);
-    if (b == 0 && tid == 0 && P.trace && ntrace < TRACE_CAP) {  // flow at this relabel (after the barrier)
+    if (b == 0 && tid == 0 && P.trace && book.ntrace < TRACE_CAP) {  // flow at this relabel (after the barrier)
       unsigned long long f = 0;
       for (int i = 0; i < P.ninst; ++i) f += __ldcg(P.flow + i);
-      P.trace[2 * ntrace] = ((unsigned long long)TR_FLOW << 56) | ((unsigned long long)(relabels & 0xffffffffll) << 24);
-      P.trace[2 * ntrace + 1] = f;
-      ++ntrace;
+      const int i = book.ntrace++;
+      P.trace[2 * i] = ((unsigned long long)TR_FLOW << 56) | ((unsigned long long)relabels << 24);
+      P.trace[2 * i + 1] = f;
     }
     if (nact == 0) break;
     if (sweeps >= prm.max_sweeps) {
@@ -460,40 +478,33 @@ __device__ __forceinline__ void solve_body(const DevPool& P, const SolveParams& 
       break;
     }
     // ------------------------------------------------ learned scheduler
-    const int cycle = (int)relabels - 1;
+    const int cycle = relabels - 1;
     const bool tracing = prm.trace_cycles > cycle;
     if (tracing) traced = cycle + 1;
-    // Priorities (deferral) only pay off while active tiles outnumber the
-    // CTAs: with fewer, a sweep lasts one tile visit whatever the order.
-    // Budgets can still shorten that visit, so learned = 3 runs the stage in
-    // every cycle, with each tile's budget capped at the schedule's L (a
-    // budget may only end a visit early).
-    const bool throughput = nact > 2 * G;
+    // Priorities (deferral) only pay off while active tiles outnumber what
+    // runs at a time: with fewer, a sweep lasts one tile visit whatever the
+    // order.  Budgets can still shorten that visit, so learned = 3 runs the
+    // stage in every cycle, with each tile's budget capped at the schedule's L
+    // (a budget may only end a visit early).
+    const bool throughput = nact > 2 * G * (int)(blockDim.x / GROUP);
     const bool learned = prm.learned && (throughput || prm.learned == 3);
     if (learned || tracing) {
-      if (!sched_stage(P, prm, cycle, learned, tracing, sl[s & 3], ld_cnt(sc + (s & 3)), sl[(s + 1) & 3],
-                       prm.exclusive ? 0 : ld_cnt(sc + ((s + 1) & 3))))
+      if (!sched_stage(P, prm, cycle, learned, tracing, list(3 + (s & 3)), ld_cnt(sc + (s & 3)), list(3 + ((s + 1) & 3)),
+                       prm.exclusive ? 0 : ld_cnt(sc + ((s + 1) & 3)), bar_target))
         return;
-      lap(ns_sched);
+      lap(book.ns_sched);
     }
     // ------------------------------------------------ sweeps
-    SweepExtra ex;
-    if (tracing) {
-      ex.tr_pulses = P.tpulses + (int64_t)cycle * P.T;
-      ex.tr_sink = P.tsink + (int64_t)cycle * P.T;
-    }
     int idle = 0;  // consecutive sweeps in which no tile delivered flow to the sink
     for (int j = 0; j < 2 * prm.K; ++j, ++s) {
+      const int32_t* const lst = list(3 + (s & 3));
+      const int t0 = first_entry(lst), tw = b < P.T ? ld_ahead(lst + b) : 0;
       const int n = ld_cnt(sc + (s & 3));
       if (n == 0 && (prm.exclusive || ld_cnt(sc + ((s + 1) & 3)) == 0)) break;
       if (b == 0 && tid == 0) {
         sc[(s + 3) & 3] = 0;
-        P.cnt[C_SINKT0 + (int)((s + 1) % 3)] = 0;
+        P.cnt[C_SINKT0 + (s + 1) % 3] = 0;
       }
-      ex.sink_tiles = P.cnt + C_SINKT0 + (int)(s % 3);
-      // the learned scheduler defers low-priority tiles during the first half
-      // of the cycle; every active tile is swept in the second half
-      const bool may_defer = learned && throughput && (prm.learned == 1 || prm.learned == 3) && j < prm.K;
       // Parity sweeps: sweep s uses stamp id s + 1; a visited tile queues the
       // tiles it pushed into for sweep s + 1 and itself, of the same parity,
       // for sweep s + 2.  Exclusive sweeps: every queued tile runs unless it
@@ -503,77 +514,100 @@ __device__ __forceinline__ void solve_body(const DevPool& P, const SolveParams& 
       // the parity schedule; everything is queued for sweep s + 1, with the
       // stamps in half (s+1)&1 of stamp_sw, so half s&1 -- this sweep's list --
       // does not change during the sweep.
-      uint32_t* const stamp_q = prm.exclusive ? P.stamp_sw + ((s + 1) & 1) * P.T : P.stamp_sw;
-      const uint32_t id_self = (uint32_t)(prm.exclusive ? s + 2 : s + 3);
-      int32_t* const list_self = sl[(prm.exclusive ? s + 1 : s + 2) & 3];
-      int32_t* const cnt_self = sc + ((prm.exclusive ? s + 1 : s + 2) & 3);
-      for_entries(n, [&](int i) {
-        const int t = __ldcg(sl[s & 3] + i);
-        if (may_defer && !__ldcg(P.sprio + t)) {
-          if (leader && atomicExch(stamp_q + t, id_self) != id_self) list_self[atomicAdd(cnt_self, 1)] = t;
+      auto sweep_visit = [&](const auto vg, auto& sh, int t) {
+        uint32_t* const stamp_q = prm.exclusive ? P.stamp_sw + (int64_t)((s + 1) & 1) * P.T : P.stamp_sw;
+        const int sn = s + 1, ss = prm.exclusive ? s + 1 : s + 2;  // the sweeps the neighbours and the tile queue for
+        // the learned scheduler defers low-priority tiles during the first half
+        // of the cycle; every active tile is swept in the second half
+        if (learned && throughput && prm.learned != 2 && j < prm.K && !__ldcg(P.sprio + t)) {
+          if (vg.q == 0) queue_tile(P, stamp_q, t, (uint32_t)(ss + 1), list(3 + (ss & 3)), sc + (ss & 3));
           return;
         }
-        if (prm.exclusive && (int)__ldcg(P.tpar + t) != (int)(s & 1)) {  // uniform over the block
+        if (prm.exclusive && (int)__ldcg(P.tpar + t) != (s & 1)) {  // uniform over the group
           bool queued_nb = false;
-          if (tid < 6) {
-            const int nb = __ldcg(P.nbr + tid * P.T + t);
-            queued_nb = nb >= 0 && __ldcg(P.stamp_sw + (s & 1) * P.T + nb) == (uint32_t)(s + 1);
+          if (vg.q < 6) {
+            const int nb = __ldcg(P.nbr + vg.q * P.T + t);
+            queued_nb = nb >= 0 && __ldcg(P.stamp_sw + (int64_t)(s & 1) * P.T + nb) == (uint32_t)(s + 1);
           }
-          if (__syncthreads_or(queued_nb)) {  // wait one sweep
-            if (leader) queue_tile(P, stamp_q, t, (uint32_t)(s + 2), sl[(s + 1) & 3], sc + ((s + 1) & 3));
+          if (vg.any(queued_nb)) {  // wait one sweep
+            if (vg.q == 0) queue_tile(P, stamp_q, t, (uint32_t)(sn + 1), list(3 + (sn & 3)), sc + (sn & 3));
             return;
           }
         }
         const int L = !learned ? prm.L
                       : prm.learned == 3 ? min((int)__ldcg(P.sbudget + t), prm.L) : (int)__ldcg(P.sbudget + t);
-        sweep_tile<true>(P, t, L, prm.R, S.sw, (uint32_t)(s + 2), sl[(s + 1) & 3], sc + ((s + 1) & 3), id_self,
-                         list_self, cnt_self, ex, stamp_q);
-      });
+        SweepExtra ex;
+        if (prm.stall > 0) ex.sink_tiles = P.cnt + C_SINKT0 + s % 3;
+        if (tracing) {
+          ex.tr_pulses = P.tpulses + (int64_t)cycle * P.T;
+          ex.tr_sink = P.tsink + (int64_t)cycle * P.T;
+        }
+        int np;
+        if constexpr (decltype(vg)::width == WIDE)
+          np = sweep_tile_wide<true>(P, vg, t, L, prm.R, j == 0, sh, (uint32_t)(sn + 1), list(3 + (sn & 3)), sc + (sn & 3),
+                                     (uint32_t)(ss + 1), list(3 + (ss & 3)), sc + (ss & 3), ex, stamp_q);
+        else
+          np = sweep_tile(P, vg, t, L, prm.R, j == 0, sh, (uint32_t)(sn + 1), list(3 + (sn & 3)), sc + (sn & 3),
+                                (uint32_t)(ss + 1), list(3 + (ss & 3)), sc + (ss & 3), ex, stamp_q);
+        if (vg.q == 0) {
+          ++book.visits_sw[grp];
+          book.pulses[grp] += (unsigned)np;
+        }
+      };
+      // At most one tile per SM: 512 threads per visit.  A visit then lasts
+      // about 12k cycles instead of 18k (256^3 tail); with two tiles per SM one
+      // after the other it gains nothing over two groups side by side.
+      if (n <= G) {
+        const auto wide = TileGroup<WIDE>::of_thread();
+        if (tid < WIDE && b < n) sweep_visit(wide, *reinterpret_cast<WideShared*>(groups), tw);
+      } else {
+        for_entries(lst, t0, n, [&](int t) { sweep_visit(tg, S.sw, t); });
+      }
       ++sweeps;
-      if (!grid_sync(P, prm.limit_ns)) return;
+      if (!sync()) return;
       record(TR_SWEEP, sweeps, n);
       // Early relabel: after stall consecutive non-empty sweeps of each parity
       // delivered no flow to the sink.  Empty sweeps do not count, so every
       // cycle performs at least one push or relabel; labels never decrease
       // (an exact relabel only raises valid labels), so the solve still ends.
-      if (n > 0) idle = ld_cnt(P.cnt + C_SINKT0 + (int)(s % 3)) ? 0 : idle + 1;
+      if (prm.stall > 0 && n > 0) idle = ld_cnt(P.cnt + C_SINKT0 + s % 3) ? 0 : idle + 1;
       if (prm.stall > 0 && idle >= 2 * prm.stall) { ++s; break; }
     }
-    lap(ns_sweep);
+    lap(book.ns_sweep);
   }
-  lap(ns_bfs);
+  lap(book.ns_bfs);
   // ------------------------------------------------ source-side reachability
-  if (b == 0 && tid == 0) {
-    bc[0] = bc[1] = bc[2] = 0;
-    P.cnt[C_TAKE0] = P.cnt[C_TAKE0 + 1] = P.cnt[C_TAKE0 + 2] = 0;
-  }
-  round_no = 0;
-  if (!grid_sync(P, prm.limit_ns)) return;
-  for (int t = gw; t < P.T; t += nw) reach_init_tile_w(P, t, bfs_id, bl[0], bc + 0);
-  if (!grid_sync(P, prm.limit_ns)) return;
-  int k = 0;
-  for (;;) {
+  if (b == 0 && tid == 0) bc[0] = bc[1] = bc[2] = 0;
+  if (!sync()) return;
+  for (int t = gw; t < P.T; t += nw) reach_init_tile_w(P, t, bfs_id, list(0), bc + 0);
+  if (!sync()) return;
+  for (int k = 0;;) {
     const int n = ld_cnt(bc + k % 3);
     if (n == 0) break;
     if (b == 0 && tid == 0) bc[(k + 2) % 3] = 0;
-    for_entries(n, [&](int i) {
-      reach_tile(P, __ldcg(bl[k % 3] + i), S.rc, bfs_id + k + 1, bl[(k + 1) % 3], bc + (k + 1) % 3);
-    });
+    for (int i = (tid >> 5) * G + b; i < n; i += nw)  // a warp per tile
+      reach_tile_w(P, __ldcg(list(k % 3) + i), bfs_id + k + 1, list((k + 1) % 3), bc + (k + 1) % 3);
     ++k;
-    if (!grid_sync(P, prm.limit_ns)) return;
+    if (!sync()) return;
     record(TR_REACH_ROUND, k, n);
   }
+  if (q == 0) {
+    atomicAdd(P.stats + S_TILES_SWEPT, (unsigned long long)book.visits_sw[grp]);
+    atomicAdd(P.stats + S_PULSES, (unsigned long long)book.pulses[grp]);
+    atomicAdd(P.stats + S_TILES_BFS, (unsigned long long)book.visits_bfs[grp]);
+    atomicAdd(P.stats + S_TILES_CHECK, (unsigned long long)book.visits_chk[grp]);
+  }
   if (b == 0 && tid == 0) {
+    lap(book.ns_reach);
     P.stats[S_SWEEPS] = (unsigned long long)sweeps;
     P.stats[S_RELABELS] = (unsigned long long)relabels;
     P.stats[S_ROUNDS] = (unsigned long long)rounds;
-    lap(ns_reach);
-    P.stats[S_NS_BFS] = ns_bfs;
-    P.stats[S_NS_SWEEP] = ns_sweep;
-    P.stats[S_NS_REACH] = ns_reach;
-    P.stats[S_TRACE_N] = (unsigned long long)ntrace;
+    P.stats[S_NS_BFS] = book.ns_bfs;
+    P.stats[S_NS_SWEEP] = book.ns_sweep;
+    P.stats[S_NS_REACH] = book.ns_reach;
+    P.stats[S_TRACE_N] = (unsigned long long)book.ntrace;
     P.stats[S_TRACE_CYC] = (unsigned long long)traced;
-    P.stats[S_NS_SCHED] = ns_sched;
+    P.stats[S_NS_SCHED] = book.ns_sched;
   }
 }
 
@@ -599,7 +633,19 @@ int coop_launch_ordered(int device, cudaStream_t stream, const std::function<int
   return CGC_OK;
 }
 
-int launch_solve(Pool& p, const cgc_options& o, const DevPool& d, const SolveParams& prm, cudaStream_t stream) {
+// Tile groups per SM.  More groups hide more latency while tiles are plenty
+// (512x512x128 tubes, sweeps: 4.2 ms at 4 groups, 3.8 at 5, 3.7 at 8); fewer
+// leave each visit more registers and issue slots, which the tail of a solve
+// wants (256^3 balls, kernel: 5.1, 5.2, 5.8 ms).
+static int solve_groups(const cgc_options& o) { return o.ctas_per_sm == 4 ? 8 : o.ctas_per_sm == 3 ? 5 : 4; }
+
+static void (*solve_kernel(int groups))(DevPool, SolveParams) {
+  return groups == 8 ? k_solve8 : groups == 5 ? k_solve5 : k_solve4;
+}
+
+int launch_solve(const DevPool& d, const cgc_options& o, const SolveParams& prm, int device, int sms, cudaStream_t stream) {
+  const int groups = solve_groups(o);
+  auto* kernel = solve_kernel(groups);
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
@@ -607,15 +653,13 @@ int launch_solve(Pool& p, const cgc_options& o, const DevPool& d, const SolvePar
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   cfg.stream = stream;
-  const bool three = o.ctas_per_sm == 3, four = o.ctas_per_sm == 4;
-  cfg.gridDim = dim3(four ? p.coop_blocks4 : three ? p.coop_blocks3 : p.coop_blocks);
-  cfg.blockDim = dim3(512);
-  cfg.dynamicSmemBytes = 0;
-  const bool bw = prm.bfs_warp_min > 0;
-  int rc = coop_launch_ordered(p.device, stream, [&]() -> int {
-    if (four) CGC_CUDA(cudaLaunchKernelEx(&cfg, bw ? k_solve4w : k_solve4, d, prm));
-    else if (three) CGC_CUDA(cudaLaunchKernelEx(&cfg, bw ? k_solve3w : k_solve3, d, prm));
-    else CGC_CUDA(cudaLaunchKernelEx(&cfg, k_solve, d, prm));
+  cfg.gridDim = dim3(sms);
+  cfg.blockDim = dim3(groups * GROUP);
+  cfg.dynamicSmemBytes = groups * sizeof(TileShared);
+  // a property of the function on the current device, set before its first launch there
+  CGC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes));
+  int rc = coop_launch_ordered(device, stream, [&]() -> int {
+    CGC_CUDA(cudaLaunchKernelEx(&cfg, kernel, d, prm));
     return CGC_OK;
   });
   if (rc) return rc;
@@ -623,29 +667,17 @@ int launch_solve(Pool& p, const cgc_options& o, const DevPool& d, const SolvePar
   return ok();
 }
 
-// The solve kernel at 2 CTAs per SM (64 registers), at 3 (40 registers, a
-// few spills) and at 4 (2048 threads, 32 registers).
-__global__ void __launch_bounds__(512, 2) k_solve(DevPool P, SolveParams prm) {
-  __shared__ SolveShared S;
-  solve_body(P, prm, S);
+// The solve kernel with 4, 5 or 8 tile groups per SM (128, 96 and 64 registers
+// per thread).
+extern __shared__ __align__(16) unsigned char solve_smem[];
+__global__ void __launch_bounds__(4 * GROUP, 1) k_solve4(DevPool P, SolveParams prm) {
+  solve_body(P, prm, reinterpret_cast<TileShared*>(solve_smem));
 }
-__global__ void __launch_bounds__(512, 3) k_solve3(DevPool P, SolveParams prm) {
-  __shared__ SolveShared S;
-  solve_body(P, prm, S);
+__global__ void __launch_bounds__(5 * GROUP, 1) k_solve5(DevPool P, SolveParams prm) {
+  solve_body(P, prm, reinterpret_cast<TileShared*>(solve_smem));
 }
-__global__ void __launch_bounds__(512, 4) k_solve4(DevPool P, SolveParams prm) {
-  __shared__ SolveShared S;
-  solve_body(P, prm, S);
-}
-// The same with warp-per-tile BFS rounds (SolveParams::bfs_warp_min); separate
-// kernels, so that the others do not carry that code's registers.
-__global__ void __launch_bounds__(512, 3) k_solve3w(DevPool P, SolveParams prm) {
-  __shared__ SolveShared S;
-  solve_body<true>(P, prm, S);
-}
-__global__ void __launch_bounds__(512, 4) k_solve4w(DevPool P, SolveParams prm) {
-  __shared__ SolveShared S;
-  solve_body<true>(P, prm, S);
+__global__ void __launch_bounds__(8 * GROUP, 1) k_solve8(DevPool P, SolveParams prm) {
+  solve_body(P, prm, reinterpret_cast<TileShared*>(solve_smem));
 }
 
 // Output kernels (linear layout of one instance).  k_segments, a thread per
@@ -765,7 +797,6 @@ int pool_create(int32_t count, const int32_t* ext, void* stream, Pool** out) {
   const int64_t o_fl = off; off += al((int64_t)count * 8);
   const int64_t o_geo = off; off += al((int64_t)count * sizeof(InstGeo));
   const int64_t o_st = off; off += al(S_NSTATS * 8);
-  const int64_t o_err = off; off += al(4);
   const int64_t o_bar = off; off += al(8);
   const int64_t o_tr = off; off += al(2 * TRACE_CAP * 8);
   CGC_CUDA(cudaMalloc(&p->dbuf, off));
@@ -780,7 +811,7 @@ int pool_create(int32_t count, const int32_t* ext, void* stream, Pool** out) {
   d.stamp_inc = (uint32_t*)(base + o_si);
   d.lists = (int32_t*)(base + o_li); d.cnt = (int32_t*)(base + o_cnt);
   d.flow = (unsigned long long*)(base + o_fl); d.geo = (InstGeo*)(base + o_geo);
-  d.stats = (unsigned long long*)(base + o_st); d.err = (int32_t*)(base + o_err); d.bar = (uint32_t*)(base + o_bar);
+  d.stats = (unsigned long long*)(base + o_st); d.bar = (uint32_t*)(base + o_bar); d.err = (int32_t*)(d.bar + 1);
   d.trace = (unsigned long long*)(base + o_tr);
 
   // tile tables
@@ -820,20 +851,8 @@ int pool_create(int32_t count, const int32_t* ext, void* stream, Pool** out) {
   cudaDeviceProp prop;
   CGC_CUDA(cudaGetDeviceProperties(&prop, p->device));
   p->sms = prop.multiProcessorCount;
-  int occ = 0;
-  CGC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_solve, 512, 0));
-  p->coop_blocks = std::max(1, occ) * p->sms;
-  int occ3 = 0;
-  CGC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ3, k_solve3, 512, 0));
-  p->coop_blocks3 = std::max(1, occ3) * p->sms;
-  int occ4 = 0, occ3w = 0, occ4w = 0;
-  CGC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ4, k_solve4, 512, 0));
-  CGC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ3w, k_solve3w, 512, 0));
-  CGC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ4w, k_solve4w, 512, 0));
-  p->coop_blocks4 = std::max(1, std::min(occ4, occ4w)) * p->sms;
-  p->coop_blocks3 = std::min(p->coop_blocks3, std::max(1, occ3w) * p->sms);
   int occ2 = 0;
-  CGC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ2, k_sweep_list, 512, 0));
+  CGC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ2, k_sweep_list, WIDE, 0));
   p->sweep_blocks = std::max(1, occ2) * p->sms;
   CGC_CUDA(cudaStreamSynchronize(p->stream));
   *out = p.release();
@@ -950,7 +969,6 @@ SolveParams solve_params(const cgc_options& o) {
   prm.trace_cycles = o.trace_cycles > 0 ? o.trace_cycles : 0;
   prm.max_sweeps = (int64_t)o.max_sweeps;
   prm.limit_ns = wait_limit_ns(o);
-  prm.bfs_warp_min = o.ctas_per_sm >= 3 ? o.bfs_warp_min : 0;  // kernels k_solve3w / k_solve4w
   prm.exclusive = o.exclusive ? 1 : 0;
   prm.incremental = o.relabel == 2 ? 1 : 0;
   return prm;
@@ -976,8 +994,8 @@ static int host_bfs(Pool& p, uint32_t& id, int64_t& rounds) {
     if (n == 0) { id += k + 1; break; }
     CGC_CUDA(cudaMemsetAsync(d.cnt + C_BFS0 + (k + 1) % 3, 0, 4, p.stream));
     const int gb = std::min(n, p.sweep_blocks);
-    if (REACH) { k_reach_round<<<gb, 512, 0, p.stream>>>(d, bl[k % 3], d.cnt + C_BFS0 + k % 3, id + k + 1, bl[(k + 1) % 3], d.cnt + C_BFS0 + (k + 1) % 3); note_launch(); }
-    else { k_bfs_round<<<gb, 512, 0, p.stream>>>(d, bl[k % 3], d.cnt + C_BFS0 + k % 3, id + k + 1, bl[(k + 1) % 3], d.cnt + C_BFS0 + (k + 1) % 3); note_launch(); }
+    if (REACH) { k_reach_round<<<gb, GROUP, 0, p.stream>>>(d, bl[k % 3], d.cnt + C_BFS0 + k % 3, id + k + 1, bl[(k + 1) % 3], d.cnt + C_BFS0 + (k + 1) % 3); note_launch(); }
+    else { k_bfs_round<<<gb, GROUP, 0, p.stream>>>(d, bl[k % 3], d.cnt + C_BFS0 + k % 3, id + k + 1, bl[(k + 1) % 3], d.cnt + C_BFS0 + (k + 1) % 3); note_launch(); }
     CGC_CUDA(cudaGetLastError());
     ++rounds;
   }
@@ -1028,8 +1046,7 @@ int pool_solve_async(Pool& p, const cgc_options* opts) {
   CGC_CUDA(cudaEventRecord(p.ev[0], p.stream));
   CGC_CUDA(cudaMemsetAsync(d.flow, 0, (size_t)p.ninst * 8, p.stream));
   CGC_CUDA(cudaMemsetAsync(d.stats, 0, S_NSTATS * 8, p.stream));
-  CGC_CUDA(cudaMemsetAsync(d.err, 0, 4, p.stream));
-  CGC_CUDA(cudaMemsetAsync(d.bar, 0, 8, p.stream));
+  CGC_CUDA(cudaMemsetAsync(d.bar, 0, 8, p.stream));  // and the error word
   CGC_CUDA(cudaMemsetAsync(d.stamp_bfs, 0, (size_t)d.T * 4, p.stream));
   CGC_CUDA(cudaMemsetAsync(d.stamp_sw, 0, 2 * (size_t)d.T * 4, p.stream));
   CGC_CUDA(cudaMemsetAsync(d.stamp_inc, 0, (size_t)d.T * 4, p.stream));
@@ -1053,7 +1070,7 @@ int pool_solve_async(Pool& p, const cgc_options* opts) {
   int rc = CGC_OK;
   if (o.persistent > 0) {
     CGC_CUDA(cudaEventRecord(p.ev[2], p.stream));
-    rc = launch_solve(p, o, d, prm, p.stream);
+    rc = launch_solve(d, o, prm, p.device, p.sms, p.stream);
     CGC_CUDA(cudaEventRecord(p.ev[3], p.stream));
   } else {
     // the host loop reads counters back every round; a preparation error
@@ -1080,7 +1097,7 @@ int pool_solve_async(Pool& p, const cgc_options* opts) {
           CGC_CUDA(cudaMemsetAsync(d.cnt + C_SW0 + par, 0, 4, p.stream));
           k_compact<<<(d.T + 255) / 256, 256, 0, p.stream>>>(d, par, sl + par * d.T, d.cnt + C_SW0 + par); note_launch();
         }
-        k_sweep_list<<<p.sweep_blocks, 512, 0, p.stream>>>(d, sl + par * d.T, d.cnt + C_SW0 + par, o.local_pulses, o.region_relabels); note_launch();
+        k_sweep_list<<<p.sweep_blocks, WIDE, 0, p.stream>>>(d, sl + par * d.T, d.cnt + C_SW0 + par, o.local_pulses, o.region_relabels); note_launch();
         CGC_CUDA(cudaGetLastError());
         ++sweeps;
       }

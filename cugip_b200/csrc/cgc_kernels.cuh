@@ -1,9 +1,15 @@
 // Tile routines and kernels of the grid push-relabel engine (sm_100a).
 //
-// One CTA of 512 threads owns one 8x8x8 tile at a time; thread l owns voxel
-// (l&7, (l>>3)&7, l>>6).  The voxel's own state (excess, height, sink
-// residual, six out-residuals) lives in registers; heights of the tile plus a
-// one-voxel halo live in shared memory so that neighbours can be read.
+// A tile group of 128 threads owns one 8x8x8 tile at a time; thread q owns the
+// four voxels 4q..4q+3 (half an x row: x = 4(q&1).., y = (q>>1)&7, z = q>>4).
+// Their state (excess, height, sink residual, six out-residuals) lives in
+// registers; heights of the tile plus a one-voxel halo live in shared memory
+// so that neighbours can be read.  What bounds a visit is the latency of its
+// steps -- a chain of shared-memory round trips and block barriers -- and, when
+// many tiles are active, the instructions they issue.  Rows of four make both
+// small: a y or z neighbour row is one 16-byte shared load for four voxels, the
+// x neighbours are registers or one shuffle, y exchanges stay inside a warp
+// (warp w owns the planes z = 2w, 2w+1), and a barrier joins 4 warps.
 //
 // Push sweep (replaces the per-level push of
 // include/cugip/advanced_operations/detail/graph_cut_push.hpp:160-186,236-318,
@@ -36,12 +42,7 @@
 
 namespace cgc {
 
-__device__ __forceinline__ int halo_index(int x, int y, int z) { return (z + 1) * 100 + (y + 1) * 10 + (x + 1); }
-
-// offsets of the 6 neighbours in the halo array and inside a tile
-__device__ __forceinline__ int hoff(int d) {
-  return d == PX ? 1 : d == MX ? -1 : d == PY ? 10 : d == MY ? -10 : d == PZ ? 100 : -100;
-}
+// offset of the neighbour along d inside a tile
 __device__ __forceinline__ int loff(int d) {
   return d == PX ? 1 : d == MX ? -1 : d == PY ? 8 : d == MY ? -8 : d == PZ ? 64 : -64;
 }
@@ -51,10 +52,6 @@ __device__ __forceinline__ int xoff(int d) {
 }
 __device__ __forceinline__ bool inside(int d, int x, int y, int z) {
   return d == PX ? x < 7 : d == MX ? x > 0 : d == PY ? y < 7 : d == MY ? y > 0 : d == PZ ? z < 7 : z > 0;
-}
-// entry of voxel (x,y,z) on face d in the order of for_halo_entry (a + 8b)
-__device__ __forceinline__ int face_entry(int d, int x, int y, int z) {
-  return (d == PX || d == MX) ? y + 8 * z : (d == PY || d == MY) ? x + 8 * z : x + 8 * y;
 }
 // bit mask of the faces of the tile the voxel lies on
 __device__ __forceinline__ int face_bits(int x, int y, int z) {
@@ -86,32 +83,99 @@ static __device__ __noinline__ bool bound_fail(const DevPool& P, long long i) {
 #define CGC_IN_BOUNDS(P, i, lim) true
 #endif
 
-// Face f of the halo: thread k in [0,64) of face f writes halo entry (a,b) of
-// that face from the neighbouring tile (INF outside the grid).
-template <typename F>
-__device__ __forceinline__ void for_halo_entry(int l, F&& fn) {
-  if (l < 384) {
-    const int f = l >> 6, k = l & 63, a = k & 7, b = k >> 3;
-    int hi, src;
-    switch (f) {
-      case PX: hi = (b + 1) * 100 + (a + 1) * 10 + 9; src = 8 * a + 64 * b; break;
-      case MX: hi = (b + 1) * 100 + (a + 1) * 10;     src = 7 + 8 * a + 64 * b; break;
-      case PY: hi = (b + 1) * 100 + 90 + (a + 1);     src = a + 64 * b; break;
-      case MY: hi = (b + 1) * 100 + (a + 1);          src = a + 56 + 64 * b; break;
-      case PZ: hi = 900 + (b + 1) * 10 + (a + 1);     src = a + 8 * b; break;
-      default: hi = (b + 1) * 10 + (a + 1);           src = a + 8 * b + 448; break;
-    }
-    fn(f, hi, src);
+constexpr unsigned FULL = 0xffffffffu;
+
+// The W threads that visit a tile together, with a named barrier of their own
+// (barrier 0 is __syncthreads of the whole CTA): groups of 128, numbered in the
+// CTA, or the CTA's first 512 threads.
+constexpr int GROUP = 128, WIDE = 512;
+template <int W>
+struct TileGroup {
+  static constexpr int width = W;
+  int q;    // thread of the group
+  int bar;  // named barrier
+  __device__ __forceinline__ static TileGroup of_thread() {
+    if (W == WIDE) return TileGroup{(int)threadIdx.x, 15};
+    return TileGroup{(int)(threadIdx.x & (W - 1)), 1 + (int)(threadIdx.x / W)};
   }
+  __device__ __forceinline__ void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(W) : "memory"); }
+  __device__ __forceinline__ bool any(bool p) const {
+    int r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\tbar.red.or.pred q, %2, %3, p;\n\t"
+        "selp.s32 %0, 1, 0, q;\n\t}"
+        : "=r"(r)
+        : "r"((int)p), "r"(bar), "n"(W)
+        : "memory");
+    return r != 0;
+  }
+};
+
+// Heights of a tile with its y and z halo rows in shared memory: row (y, z),
+// y and z in [-1, 8], is 8 ints at hrow(y, z).  The x halo is one register per
+// thread (the neighbour left of x = 0 or right of x = 7).
+constexpr int HROWS = 100;
+__device__ __forceinline__ int hrow(int y, int z) { return ((z + 1) * 10 + (y + 1)) * 8; }
+
+__device__ __forceinline__ int4 ld4(const int* p) { return *reinterpret_cast<const int4*>(p); }
+__device__ __forceinline__ void st4(int* p, const int (&v)[4]) {
+  *reinterpret_cast<int4*>(p) = make_int4(v[0], v[1], v[2], v[3]);
+}
+__device__ __forceinline__ void ldcg4(const int32_t* p, int (&v)[4]) {
+  const int4 a = __ldcg(reinterpret_cast<const int4*>(p));
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+}
+__device__ __forceinline__ int at(const int4& v, int k) { return k == 0 ? v.x : k == 1 ? v.y : k == 2 ? v.z : v.w; }
+
+// Halo of tile t: 64 threads each load half a y or z halo row into sh0 (and
+// sh1 if given), every thread returns its x halo height (INF outside the grid).
+__device__ __forceinline__ int load_halo_heights(const DevPool& P, const int t, const int q, int* sh0, int* sh1) {
+  const int half = q & 1, k = (q >> 1) & 7;
+  const int nx = __ldcg(P.nbr + (half ? PX : MX) * P.T + t);
+  if (q < 64) {
+    const int f = PY + (q >> 4);
+    const int nt = __ldcg(P.nbr + f * P.T + t);
+    int4 v = make_int4(INF, INF, INF, INF);
+    const int src = (f == PY ? 64 * k : f == MY ? 64 * k + 56 : f == PZ ? 8 * k : 8 * k + 448) + 4 * half;
+    const int dst = (f == PY ? hrow(8, k) : f == MY ? hrow(-1, k) : f == PZ ? hrow(k, 8) : hrow(k, -1)) + 4 * half;
+    if (nt >= 0 && CGC_IN_BOUNDS(P, nt, P.T)) v = __ldcg(reinterpret_cast<const int4*>(P.h + (int64_t)nt * TV + src));
+    *reinterpret_cast<int4*>(sh0 + dst) = v;
+    if (sh1) *reinterpret_cast<int4*>(sh1 + dst) = v;
+  }
+  return (nx >= 0 && CGC_IN_BOUNDS(P, nx, P.T)) ? __ldcg(P.h + (int64_t)nx * TV + 8 * (q >> 1) + (half ? 0 : 7)) : INF;
 }
 
-__device__ __forceinline__ void load_halo_heights(const DevPool& P, int t, int (*sh)[HALO]) {
-  for_halo_entry(threadIdx.x, [&](int f, int hi, int src) {
-    const int nt = __ldcg(P.nbr + f * P.T + t);
-    const int v = (nt >= 0 && CGC_IN_BOUNDS(P, nt, P.T)) ? __ldcg(P.h + (int64_t)nt * TV + src) : INF;
-    sh[0][hi] = v;
-    sh[1][hi] = v;
-  });
+// Cost of a closed edge in the relaxation: INF + CLOSED does not overflow, and
+// any height plus CLOSED is above INF.
+constexpr int CLOSED = 0x40000000;
+
+// One in-place Bellman-Ford step of the thread's four voxels on the heights S
+// (d[] is the thread's copy of its row): d = min(d, 1 + neighbour) over the
+// open edges (c[dir][k] is 1 for an open edge, CLOSED otherwise, so an edge is
+// one add-min instruction and needs no predicate).  Values only drop, so
+// reading a neighbour's old or new value is both correct and the fixed point
+// is the same.  Returns whether d dropped (and then the row was stored).
+__device__ __forceinline__ bool relax_row(int* S, const int row, const int half, const int hx, int (&d)[4],
+                                          const int (&c)[6][4]) {
+  const int4 yp = ld4(S + row + 8), ym = ld4(S + row - 8), zp = ld4(S + row + 80), zm = ld4(S + row - 80);
+  const int xo = __shfl_xor_sync(FULL, half ? d[0] : d[3], 1);
+  int n[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    n[k] = min(__viaddmin_s32(at(yp, k), c[PY][k], d[k]), __viaddmin_s32(at(ym, k), c[MY][k], at(zp, k) + c[PZ][k]));
+    n[k] = __viaddmin_s32(at(zm, k), c[MZ][k], n[k]);
+  }
+  n[0] = __viaddmin_s32(half ? xo : hx, c[MX][0], n[0]);
+  n[3] = __viaddmin_s32(half ? hx : xo, c[PX][3], n[3]);
+#pragma unroll
+  for (int k = 1; k < 4; ++k) n[k] = __viaddmin_s32(n[k - 1], c[MX][k], n[k]);
+#pragma unroll
+  for (int k = 2; k >= 0; --k) n[k] = __viaddmin_s32(n[k + 1], c[PX][k], n[k]);
+  const bool ch = ((n[0] ^ d[0]) | (n[1] ^ d[1]) | (n[2] ^ d[2]) | (n[3] ^ d[3])) != 0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) d[k] = n[k];
+  if (ch) st4(S + row, d);
+  return ch;
 }
 
 // warp-aggregated append of `pred` items to list/cnt
@@ -154,214 +218,633 @@ __device__ __forceinline__ long long block_sum64(long long v, long long* red) {
   return s;
 }
 
-// Shared state is double buffered (pulse / iteration parity), so one
-// pulse needs two barriers and one BFS iteration needs one.
-struct SweepShared {
-  int h[2][HALO];
-  int out[2][6][TV];
-  int facc[6][64];          // flow pushed out of the tile per face entry (for_halo_entry order)
-  unsigned long long sink;  // flow delivered to the sink by this visit
-  int nb[6];                // face neighbours of the tile (-1 outside)
-  int flags;
-  int lastout;  // last pulse (1-based) that moved flow out of the tile or into the sink
+// Shared state of one tile group.
+struct alignas(16) SweepShared {
+  int h[2][HROWS * 8];  // heights, double buffered by pulse
+  int out[2][TV];       // flow pushed along +z / -z in this pulse; zero between pulses
+  int facc[6][64];      // flow pushed out of the tile per face entry
+  unsigned char face[8];  // faces that flow left through
+  int lastout;          // last pulse (1-based) that moved flow out of the tile or into the sink
 };
 
-struct BfsShared {
-  int h[2][HALO];
-  int flags;
+struct alignas(16) BfsShared {
+  int h[HROWS * 8];
+  unsigned char face[8];  // BFS / invalidation: faces whose heights changed
+  unsigned char act;      // an excess voxel that reaches the sink
+  unsigned char any;      // a voxel was dropped
 };
 
-struct ReachShared {
-  unsigned char rc[2][HALO];
-  unsigned char m[HALO];
-  int flags;
-};
-
-// ---------------------------------------------------------------------------
-// One visit of the push sweep to tile t (L pulses at most).
-//   APPEND: queue the tile itself (if still active) for sweep id_self and the
-//   tiles it pushed into for sweep id_next (persistent schedule); otherwise
-//   only the act[] flags are maintained (host-driven schedule).
 // optional per-visit bookkeeping of the persistent schedule
 struct SweepExtra {
-  int32_t* sink_tiles = nullptr;  // counter of tiles that delivered sink flow in this sweep
+  int32_t* sink_tiles = nullptr;  // nonzero after a sweep in which some tile delivered sink flow
   uint8_t* tr_pulses = nullptr;   // trace: pulses of the first visit in this cycle
   uint8_t* tr_sink = nullptr;     // trace: delivered sink flow in this cycle
 };
 
-//   stamp_q: the stamps the queued tiles get (null: P.stamp_sw).
-template <bool APPEND>
-__device__ inline void sweep_tile(const DevPool& P, const int t, const int L, const int R, SweepShared& S,
-                           const uint32_t id_next, int32_t* list_next, int32_t* cnt_next,
-                           const uint32_t id_self, int32_t* list_self, int32_t* cnt_self,
-                           const SweepExtra ex = SweepExtra(), uint32_t* stamp_q = nullptr) {
-  if (!stamp_q) stamp_q = P.stamp_sw;
-  if (!CGC_IN_BOUNDS(P, t, P.T)) return;  // uniform over the block
-  const int l = threadIdx.x;
-  const int x = l & 7, y = (l >> 3) & 7, z = l >> 6;
-  const int64_t g = (int64_t)t * TV + l;
+// ---------------------------------------------------------------------------
+// One visit of the push sweep to tile t (L pulses at most per region-relabel
+// round, R rounds) by one tile group; returns the pulses it ran.
+//   The tile itself (if still active) is queued for sweep id_self and the tiles
+//   it pushed into for sweep id_next, with the stamps stamp_q.
+//   exact: the labels are exact (no push or relabel since the last global
+//   relabel), so the first region relabel would change nothing and is left out.
+// The caller synchronises the group before S is used again.
+//
+// A pulse pushes in the order sink, +x, -x (through the thread's row, so flow
+// crosses four voxels), row ends (shuffle), +-y (shuffles inside the warp), +-z
+// (shared memory); flow received earlier in the pulse may be pushed on by a
+// later direction, since labels do not change until the pulse's relabel.  Two
+// barriers per pulse.
+__device__ __forceinline__ int sweep_tile(const DevPool& P, const TileGroup<GROUP> tg, const int t, const int L, const int R,
+                                          const bool exact, SweepShared& S, const uint32_t id_next, int32_t* list_next,
+                                          int32_t* cnt_next, const uint32_t id_self, int32_t* list_self,
+                                          int32_t* cnt_self, const SweepExtra ex, uint32_t* stamp_q) {
+  if (!CGC_IN_BOUNDS(P, t, P.T)) return 0;  // uniform over the group
+  const int q = tg.q, half = q & 1, y = (q >> 1) & 7, z = q >> 4;
+  const int row = hrow(y, z) + 4 * half;
+  const int64_t g = (int64_t)t * TV + 4 * q;
   const int64_t Np = P.Np;
-  int e = __ldcg(P.e + g), h = __ldcg(P.h + g), rT = __ldcg(P.rT + g);
-  int r[6];
+  int e[4], h[4], rT[4], r[6][4];
+  ldcg4(P.h + g, h);
+  ldcg4(P.e + g, e);
+  ldcg4(P.rT + g, rT);
 #pragma unroll
-  for (int d = 0; d < 6; ++d) r[d] = __ldcg(P.r + d * Np + g);
-  const int hi = halo_index(x, y, z);
-  S.h[0][hi] = h;
-  load_halo_heights(P, t, S.h);
+  for (int d = 0; d < 6; ++d) ldcg4(P.r + d * Np + g, r[d]);
+  st4(S.h[0] + row, h);
+  const int hx = load_halo_heights(P, t, q, S.h[0], S.h[1]);
   const int inst = __ldcg(P.tinst + t);
   const int hdead = P.geo[inst].hdead;
-  if (l < 6) S.nb[l] = __ldcg(P.nbr + l * P.T + t);  // read by the write-back
-  if (l < 384) (&S.facc[0][0])[l] = 0;
-  if (l == 0) { S.flags = 0; S.lastout = 0; S.sink = 0ull; }
-  __syncthreads();
+  {
+    const int zero[4] = {0, 0, 0, 0};
+    st4(&S.out[0][4 * q], zero);
+    st4(&S.out[1][4 * q], zero);
+    if (q < 96) st4(&S.facc[0][0] + 4 * q, zero);
+  }
+  if (q < 8) S.face[q] = 0;
+  if (q == 0) S.lastout = 0;
+  if (R <= 0 || exact) tg.sync();  // the region relabel has its own
 
-  int sink = 0;
+  // some voxel of the thread holds excess and may still reach the sink
+  auto active = [&]() {
+    return (e[0] > 0 && h[0] < INF) || (e[1] > 0 && h[1] < INF) || (e[2] > 0 && h[2] < INF) || (e[3] > 0 && h[3] < INF);
+  };
+  long long sink = 0;
   int pulses = 0;
   int cur = 0;
+  bool dirty = false, dirty_h = false;  // the thread's excess and residuals / heights differ from memory
+  bool any = true;
   for (int round = 0;; ++round) {
-    if (R > 0) {
+    if (R > 0 && !(exact && round == 0)) {
       // Region relabel: exact distance d(v) to the sink or to the (frozen)
       // halo inside the tile, then h = max(h, d).  d is a lower bound of the
       // true distance and max(h, d) keeps every residual edge valid, so this
       // is an ordinary (multi-step) relabel; d = INF means v cannot reach the
       // sink at all.
-      int dd = (rT > 0) ? 1 : INF;
-      S.h[cur][hi] = dd;
-      __syncthreads();
+      int dd[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) dd[k] = rT[k] > 0 ? 1 : INF;
+      st4(S.h[cur] + row, dd);
+      int c[6][4];
+#pragma unroll
+      for (int d = 0; d < 6; ++d)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) c[d][k] = r[d][k] > 0 ? 1 : CLOSED;
+      tg.sync();
       for (int it = 0; it < 600; ++it) {  // Bellman-Ford: < 512 steps in a tile
-        int mn = dd;
-#pragma unroll
-        for (int d = 0; d < 6; ++d)
-          if (r[d] > 0) mn = min(mn, S.h[cur][hi + hoff(d)] + 1);
-        S.h[cur ^ 1][hi] = mn;
-        const int any = __syncthreads_or(mn < dd);
-        dd = mn;
-        cur ^= 1;
-        if (!any) break;
+        const bool ch = relax_row(S.h[cur], row, half, hx, dd, c);
+        if (!tg.any(ch)) break;
       }
-      int hn = max(h, dd);
-      if (hn >= hdead) hn = INF;
-      h = hn;
-      S.h[cur][hi] = h;
-      __syncthreads();
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        int hn = max(h[k], dd[k]);
+        if (hn >= hdead) hn = INF;
+        dirty_h = dirty_h || hn != h[k];
+        h[k] = hn;
+      }
+      st4(S.h[cur] + row, h);
+      tg.sync();
     }
-    int any = 1;
     for (int p = 0; p < L; ++p) {
-      int hn[6];
+      // labels of the neighbours, fixed during the pulse
+      const int* H = S.h[cur];
+      const int4 yp = ld4(H + row + 8), ym = ld4(H + row - 8), zp = ld4(H + row + 80), zm = ld4(H + row - 80);
+      const int xo = __shfl_xor_sync(FULL, half ? h[0] : h[3], 1);
+      const int hl = half ? xo : hx, hr = half ? hx : xo;
+      bool act = active();
+      if (__any_sync(FULL, act)) {
+        dirty = dirty || act;
+        int out = 0;  // > 0: flow left the tile or went into the sink
+        // amount voxel k pushes along d to a neighbour of height hn (a voxel
+        // at INF has no neighbour at INF - 1)
+        auto push = [&](int d, int k, int hn) {
+          const int dl = hn + 1 == h[k] ? min(e[k], r[d][k]) : 0;
+          e[k] -= dl;
+          r[d][k] -= dl;
+          return dl;
+        };
 #pragma unroll
-      for (int d = 0; d < 6; ++d) hn[d] = S.h[cur][hi + hoff(d)];
-      bool moved_out = false;
-      const bool act = e > 0 && h < INF;
-      if (act && rT > 0 && h == 1) {
-        const int dl = min(e, rT);
-        e -= dl; rT -= dl; sink += dl;
-        moved_out = dl > 0;
-      }
-      // pushes; in-tile amounts (0 included) go to S.out for the receiver,
-      // amounts across a face to the face accumulator (this voxel is its
-      // only writer)
-#pragma unroll
-      for (int d = 0; d < 6; ++d) {
-        int dl = 0;
-        if (act && e > 0 && r[d] > 0 && hn[d] == h - 1) {
-          dl = min(e, r[d]);
-          e -= dl; r[d] -= dl;
+        for (int k = 0; k < 4; ++k) {  // a voxel with a sink residual is at height 1: the labelling is valid
+          const int dl = min(e[k], rT[k]);
+          e[k] -= dl;
+          rT[k] -= dl;
+          sink += dl;
+          out |= dl;
         }
-        if (inside(d, x, y, z)) {
-          S.out[cur][d][l] = dl;
-        } else if (dl > 0) {
-          S.facc[d][face_entry(d, x, y, z)] += dl;
-          moved_out = true;
-        }
-      }
-      if (moved_out) S.lastout = pulses + 1;  // same value from every writer of this pulse
-      __syncthreads();
 #pragma unroll
-      for (int d = 0; d < 6; ++d) {
-        if (inside(d, x, y, z)) {
-          const int din = S.out[cur][d ^ 1][l + loff(d)];
-          e += din; r[d] += din;
-        }
-      }
-      int hnew = h;
-      if (e > 0 && h < INF) {
-        // the labels of the pulse start, read again from S.h[cur] (the new
-        // ones go to the other buffer) rather than kept in registers
-        bool adm = (rT > 0 && h == 1);
-        int mn = (rT > 0) ? 0 : INF;
+        for (int k = 0; k < 3; ++k)
+          if (h[k + 1] + 1 == h[k]) {
+            const int dl = min(e[k], r[PX][k]);
+            e[k] -= dl;
+            r[PX][k] -= dl;
+            e[k + 1] += dl;
+            r[MX][k + 1] += dl;
+          }
 #pragma unroll
-        for (int d = 0; d < 6; ++d) {
-          if (r[d] > 0) {
-            const int hd = S.h[cur][hi + hoff(d)];
-            adm = adm || (hd == h - 1);
-            mn = min(mn, hd);
+        for (int k = 3; k > 0; --k)
+          if (h[k - 1] + 1 == h[k]) {
+            const int dl = min(e[k], r[MX][k]);
+            e[k] -= dl;
+            r[MX][k] -= dl;
+            e[k - 1] += dl;
+            r[PX][k - 1] += dl;
+          }
+        {  // row ends: one leaves the tile, the other goes to the row's other half
+          const int ar = push(PX, 3, hr), al = push(MX, 0, hl);
+          const int in = __shfl_xor_sync(FULL, half ? al : ar, 1);
+          if (half) { e[0] += in; r[MX][0] += in; } else { e[3] += in; r[PX][3] += in; }
+          dirty = dirty || in > 0;
+          const int w = half ? ar : al;
+          if (w > 0) {
+            const int f = half ? PX : MX;
+            S.facc[f][y + 8 * z] += w;  // this thread is the entry's only writer
+            S.face[f] = 1;
+            out = 1;
           }
         }
-        if (!adm) {
-          hnew = (mn >= INF) ? INF : mn + 1;
-          if (hnew >= hdead) hnew = INF;
+        {  // y: the warp holds all rows of its planes
+          int up[4], dn[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            up[k] = push(PY, k, at(yp, k));
+            dn[k] = push(MY, k, at(ym, k));
+          }
+          const int wu = up[0] | up[1] | up[2] | up[3], wd = dn[0] | dn[1] | dn[2] | dn[3];
+          if (__any_sync(FULL, (wu | wd) > 0)) {
+            const bool hi = y == 7, lo = y == 0;
+            if (hi ? wu > 0 : lo && wd > 0) {
+              int* fa = &S.facc[hi ? PY : MY][4 * half + 8 * z];
+#pragma unroll
+              for (int k = 0; k < 4; ++k) fa[k] += hi ? up[k] : dn[k];
+              S.face[hi ? PY : MY] = 1;
+              out = 1;
+            }
+            int got = 0;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              int a = __shfl_up_sync(FULL, up[k], 2), b = __shfl_down_sync(FULL, dn[k], 2);
+              a = lo ? 0 : a;
+              b = hi ? 0 : b;
+              e[k] += a + b;
+              r[MY][k] += a;
+              r[PY][k] += b;
+              got |= a | b;
+            }
+            dirty = dirty || got > 0;
+          }
+        }
+        {  // z: through shared memory; the receiver clears what it took
+          int up[4], dn[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            up[k] = push(PZ, k, at(zp, k));
+            dn[k] = push(MZ, k, at(zm, k));
+          }
+          if ((up[0] | up[1] | up[2] | up[3]) > 0) {
+            if (z < 7) {
+              st4(&S.out[0][4 * q], up);
+            } else {
+              int* fa = &S.facc[PZ][4 * half + 8 * y];
+#pragma unroll
+              for (int k = 0; k < 4; ++k) fa[k] += up[k];
+              S.face[PZ] = 1;
+              out = 1;
+            }
+          }
+          if ((dn[0] | dn[1] | dn[2] | dn[3]) > 0) {
+            if (z > 0) {
+              st4(&S.out[1][4 * q], dn);
+            } else {
+              int* fa = &S.facc[MZ][4 * half + 8 * y];
+#pragma unroll
+              for (int k = 0; k < 4; ++k) fa[k] += dn[k];
+              S.face[MZ] = 1;
+              out = 1;
+            }
+          }
+        }
+        if (out > 0) {
+          dirty = true;
+          S.lastout = pulses + 1;  // same value from every writer of this pulse
         }
       }
+      tg.sync();
+      {
+        const int zero[4] = {0, 0, 0, 0};
+        if (z > 0) {
+          int* o = &S.out[0][4 * q - 64];
+          const int4 a = ld4(o);
+          if (a.x | a.y | a.z | a.w) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) { e[k] += at(a, k); r[MZ][k] += at(a, k); }
+            st4(o, zero);
+            dirty = true;
+          }
+        }
+        if (z < 7) {
+          int* o = &S.out[1][4 * q + 64];
+          const int4 a = ld4(o);
+          if (a.x | a.y | a.z | a.w) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) { e[k] += at(a, k); r[PZ][k] += at(a, k); }
+            st4(o, zero);
+            dirty = true;
+          }
+        }
+      }
+      // Relabel: the labelling is valid, so the lowest residual neighbour mn is
+      // at h - 1 or higher (the sink counts as height 0), and 1 + mn is h itself
+      // where the voxel still has an admissible edge.
+      bool still = false;
+      if (__any_sync(FULL, active())) {
+        int hn[4], ch = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          int mn = rT[k] > 0 ? 0 : INF;
+          if (r[PX][k] > 0) mn = min(mn, k < 3 ? h[k < 3 ? k + 1 : 3] : hr);
+          if (r[MX][k] > 0) mn = min(mn, k > 0 ? h[k > 0 ? k - 1 : 0] : hl);
+          if (r[PY][k] > 0) mn = min(mn, at(yp, k));
+          if (r[MY][k] > 0) mn = min(mn, at(ym, k));
+          if (r[PZ][k] > 0) mn = min(mn, at(zp, k));
+          if (r[MZ][k] > 0) mn = min(mn, at(zm, k));
+          int v = mn + 1;
+          if (v >= hdead) v = INF;
+          hn[k] = e[k] > 0 && h[k] < INF ? v : h[k];
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          ch |= hn[k] ^ h[k];
+          h[k] = hn[k];
+        }
+        dirty_h = dirty_h || ch != 0;
+        still = active();
+      }
       ++pulses;
-      S.h[cur ^ 1][hi] = hnew;
-      any = __syncthreads_or(e > 0 && hnew < INF);
-      h = hnew;
+      st4(S.h[cur ^ 1] + row, h);
+      any = tg.any(still);
       cur ^= 1;
       if (!any) break;
     }
     if (!any || round + 1 >= max(R, 1)) break;
   }
 
-  // write back the tile
-  P.e[g] = e; P.h[g] = h; P.rT[g] = rT;
-  unsigned m = ((rT > 0) ? 64u : 0u) | ((e > 0) ? 128u : 0u);
-#pragma unroll
-  for (int d = 0; d < 6; ++d) { P.r[d * Np + g] = r[d]; m |= (r[d] > 0 ? 1u : 0u) << d; }
-  P.rmask[g] = (uint8_t)m;
-  // flow that left the tile: excess and reverse residual of the neighbour,
-  // one face entry per thread (the pulses ended with a barrier)
-  for_halo_entry(l, [&](int f, int, int src) {
-    const int a = (&S.facc[0][0])[l];
-    if (a > 0) {
-      const int nt = S.nb[f];
-      if (nt < 0) { raise_error(P, CGC_ERR_OVERFLOW); return; }  // capacity leaving the grid
-      if (!CGC_IN_BOUNDS(P, nt, P.T)) return;
-      const int64_t ng = (int64_t)nt * TV + src;
-      atomicAdd(P.e + ng, a);
-      atomicAdd(P.r + (f ^ 1) * Np + ng, a);
-      atomicOr((unsigned*)(P.rmask + (ng & ~(int64_t)3)), (128u | (1u << (f ^ 1))) << (8 * (int)(ng & 3)));
-      atomicOr(&S.flags, 1 << f);
-    }
-  });
-  // sink flow of the visit: warp sums into one shared total before the barrier
-  unsigned long long ws = (unsigned long long)sink;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) ws += __shfl_down_sync(0xffffffffu, ws, o);
-  if ((l & 31) == 0 && ws) atomicAdd(&S.sink, ws);
-  const int still = __syncthreads_or(e > 0 && h < INF);
-  const unsigned long long total = S.sink;
-  if (l == 0) {
-    P.act[t] = (uint8_t)(still ? 1 : 0);
-    if (total) {
-      atomicAdd(P.flow + inst, total);
-      if (ex.sink_tiles) atomicAdd(ex.sink_tiles, 1);
-      if (ex.tr_sink) ex.tr_sink[t] = 1;
-    }
+  // The queue updates first: they are chains of two dependent atomics, and the
+  // rest of the write-back runs beside them.
+  if (q == 64) {
+    P.act[t] = (uint8_t)(any ? 1 : 0);
+    if (any) queue_tile(P, stamp_q, t, id_self, list_self, cnt_self);
     // trace label: productive pulses of the tile's first visit in the cycle
     // (255 marks a visited tile that moved nothing out)
     if (ex.tr_pulses && ex.tr_pulses[t] == 0) ex.tr_pulses[t] = (uint8_t)(S.lastout > 0 ? min(S.lastout, 254) : 255);
-    atomicAdd(P.stats + S_TILES_SWEPT, 1ull);
-    atomicAdd(P.stats + S_PULSES, (unsigned long long)pulses);
   }
-  // the tile re-queues itself from another warp than thread 0's face chain,
-  // so the two dependent atomic chains overlap
-  if (APPEND && l == 32 && still) queue_tile(P, stamp_q, t, id_self, list_self, cnt_self);
-  if (l < 6 && ((S.flags >> l) & 1) && CGC_IN_BOUNDS(P, S.nb[l], P.T)) {
-    const int nt = S.nb[l];
-    P.act[nt] = 1;
-    if (APPEND) queue_tile(P, stamp_q, nt, id_next, list_next, cnt_next);
+  if (q >= 32 && q < 38 && S.face[q - 32]) {
+    const int nt = __ldcg(P.nbr + (q - 32) * P.T + t);
+    if (nt < 0) {
+      raise_error(P, CGC_ERR_OVERFLOW);  // capacity leaving the grid
+    } else if (CGC_IN_BOUNDS(P, nt, P.T)) {
+      P.act[nt] = 1;
+      queue_tile(P, stamp_q, nt, id_next, list_next, cnt_next);
+    }
   }
-  __syncthreads();
+  // the tile's planes, where they changed
+  if (dirty_h) st4(P.h + g, h);
+  if (dirty) {
+    st4(P.e + g, e);
+    st4(P.rT + g, rT);
+    unsigned m4 = 0;
+#pragma unroll
+    for (int d = 0; d < 6; ++d) st4(P.r + d * Np + g, r[d]);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      unsigned m = (rT[k] > 0 ? 64u : 0u) | (e[k] > 0 ? 128u : 0u);
+#pragma unroll
+      for (int d = 0; d < 6; ++d) m |= (r[d][k] > 0 ? 1u : 0u) << d;
+      m4 |= m << (8 * k);
+    }
+    *reinterpret_cast<unsigned*>(P.rmask + g) = m4;
+  }
+  // flow that left the tile: excess and reverse residual of the neighbour
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    const int i = q + GROUP * j, f = i >> 6, a = i & 7, b = (i >> 3) & 7;
+    const int w = (&S.facc[0][0])[i];
+    if (w > 0) {
+      const int nt = __ldcg(P.nbr + f * P.T + t);
+      if (nt < 0 || !CGC_IN_BOUNDS(P, nt, P.T)) continue;  // reported above
+      const int src = f == PX ? 8 * a + 64 * b : f == MX ? 7 + 8 * a + 64 * b : f == PY ? a + 64 * b
+                    : f == MY ? a + 56 + 64 * b : f == PZ ? a + 8 * b : a + 8 * b + 448;
+      const int64_t ng = (int64_t)nt * TV + src;
+      atomicAdd(P.e + ng, w);
+      atomicAdd(P.r + (f ^ 1) * Np + ng, w);
+      atomicOr((unsigned*)(P.rmask + (ng & ~(int64_t)3)), (128u | (1u << (f ^ 1))) << (8 * (int)(ng & 3)));
+    }
+  }
+  if (__any_sync(FULL, sink > 0)) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sink += __shfl_down_sync(FULL, sink, o);
+    if ((q & 31) == 0) {
+      atomicAdd(P.flow + inst, (unsigned long long)sink);
+      if (ex.sink_tiles) atomicAdd(ex.sink_tiles, 1);
+      if (ex.tr_sink) ex.tr_sink[t] = 1;
+    }
+  }
+  return pulses;
+}
+
+// ---------------------------------------------------------------------------
+// The same visit by 512 threads, one voxel each, for sweeps that leave most of
+// the chip idle.  With one tile on an SM, a warp runs one instruction in about
+// seven cycles (its chain of dependent instructions), so the fewest
+// instructions per warp win, not the fewest in total: a relaxation step is 20
+// of them instead of 60, and a warp without an active voxel skips a pulse.
+//   APPEND: queue tiles as above (persistent schedule); otherwise only the
+//   act[] flags are maintained (host-driven schedule).
+constexpr int WH = HROWS * 8 + 128;  // a buffer of heights: the rows, then the x halo (left of x = 0, right of x = 7)
+struct alignas(16) WideShared {
+  int h[2][WH];      // double buffered by pulse
+  int out[6][TV];    // flow pushed along d in this pulse; zero between pulses
+  int facc[6][64];   // flow pushed out of the tile per face entry
+  int inbox[16];     // per warp: last pulse (1-based) in which flow was pushed to its voxels
+  int moved[8];      // last pulse in which flow left through face d; [6]: into the sink
+  int nb[6];
+};
+
+// Predicated shared-memory updates for the six directions at once: branches
+// around them cost more than the updates, and so would waiting for one
+// predicate after the other.
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+// where v[d] > 0: *to[d] += v[d], *tell[d] = s
+__device__ __forceinline__ void push_out6(const uint32_t (&to)[6], const uint32_t (&tell)[6], const int (&v)[6], int s) {
+  asm volatile(
+      "{\n\t.reg .pred p<6>;\n\t"
+      "setp.gt.s32 p0, %12, 0;\n\tsetp.gt.s32 p1, %13, 0;\n\tsetp.gt.s32 p2, %14, 0;\n\t"
+      "setp.gt.s32 p3, %15, 0;\n\tsetp.gt.s32 p4, %16, 0;\n\tsetp.gt.s32 p5, %17, 0;\n\t"
+      "@p0 red.shared.add.s32 [%0], %12;\n\t@p1 red.shared.add.s32 [%1], %13;\n\t"
+      "@p2 red.shared.add.s32 [%2], %14;\n\t@p3 red.shared.add.s32 [%3], %15;\n\t"
+      "@p4 red.shared.add.s32 [%4], %16;\n\t@p5 red.shared.add.s32 [%5], %17;\n\t"
+      "@p0 st.shared.s32 [%6], %18;\n\t@p1 st.shared.s32 [%7], %18;\n\t@p2 st.shared.s32 [%8], %18;\n\t"
+      "@p3 st.shared.s32 [%9], %18;\n\t@p4 st.shared.s32 [%10], %18;\n\t@p5 st.shared.s32 [%11], %18;\n\t}" ::"r"(to[0]),
+      "r"(to[1]), "r"(to[2]), "r"(to[3]), "r"(to[4]), "r"(to[5]), "r"(tell[0]), "r"(tell[1]), "r"(tell[2]), "r"(tell[3]),
+      "r"(tell[4]), "r"(tell[5]), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(s)
+      : "memory");
+}
+// v[d] = the flow pushed towards the voxel whose slot of direction 0 is at
+// `from` (0 where on[d] is 0: no such neighbour in the tile)
+__device__ __forceinline__ void take6(uint32_t from, const bool (&on)[6], int (&v)[6]) {
+  asm volatile(
+      "{\n\t.reg .pred p<6>;\n\t"
+      "setp.ne.s32 p0, %7, 0;\n\tsetp.ne.s32 p1, %8, 0;\n\tsetp.ne.s32 p2, %9, 0;\n\t"
+      "setp.ne.s32 p3, %10, 0;\n\tsetp.ne.s32 p4, %11, 0;\n\tsetp.ne.s32 p5, %12, 0;\n\t"
+      "mov.s32 %0, 0;\n\tmov.s32 %1, 0;\n\tmov.s32 %2, 0;\n\tmov.s32 %3, 0;\n\tmov.s32 %4, 0;\n\tmov.s32 %5, 0;\n\t"
+      "@p0 ld.shared.s32 %0, [%6+2052];\n\t@p1 ld.shared.s32 %1, [%6+-4];\n\t"
+      "@p2 ld.shared.s32 %2, [%6+6176];\n\t@p3 ld.shared.s32 %3, [%6+4064];\n\t"
+      "@p4 ld.shared.s32 %4, [%6+10496];\n\t@p5 ld.shared.s32 %5, [%6+7936];\n\t}"
+      : "=&r"(v[0]), "=&r"(v[1]), "=&r"(v[2]), "=&r"(v[3]), "=&r"(v[4]), "=&r"(v[5])
+      : "r"(from), "r"((int)on[0]), "r"((int)on[1]), "r"((int)on[2]), "r"((int)on[3]), "r"((int)on[4]), "r"((int)on[5])
+      : "memory");
+}
+// clears the slots that take6 found flow in
+__device__ __forceinline__ void clear6(uint32_t from, const int (&v)[6]) {
+  asm volatile(
+      "{\n\t.reg .pred p<6>;\n\t"
+      "setp.gt.s32 p0, %1, 0;\n\tsetp.gt.s32 p1, %2, 0;\n\tsetp.gt.s32 p2, %3, 0;\n\t"
+      "setp.gt.s32 p3, %4, 0;\n\tsetp.gt.s32 p4, %5, 0;\n\tsetp.gt.s32 p5, %6, 0;\n\t"
+      "@p0 st.shared.s32 [%0+2052], 0;\n\t@p1 st.shared.s32 [%0+-4], 0;\n\t"
+      "@p2 st.shared.s32 [%0+6176], 0;\n\t@p3 st.shared.s32 [%0+4064], 0;\n\t"
+      "@p4 st.shared.s32 [%0+10496], 0;\n\t@p5 st.shared.s32 [%0+7936], 0;\n\t}" ::"r"(from),
+      "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5])
+      : "memory");
+}
+// the offsets above: slot of direction d ^ 1 of the neighbour along d
+static_assert(4 * (MX * TV + 1) == 2052 && 4 * (PX * TV - 1) == -4 && 4 * (MY * TV + 8) == 6176 &&
+              4 * (PY * TV - 8) == 4064 && 4 * (MZ * TV + 64) == 10496 && 4 * (PZ * TV - 64) == 7936, "take6 / clear6");
+
+template <bool APPEND>
+__device__ __forceinline__ int sweep_tile_wide(const DevPool& P, const TileGroup<WIDE> tg, const int t, const int L,
+                                               const int R, const bool exact, WideShared& S, const uint32_t id_next,
+                                               int32_t* list_next, int32_t* cnt_next, const uint32_t id_self,
+                                               int32_t* list_self, int32_t* cnt_self, const SweepExtra ex,
+                                               uint32_t* stamp_q) {
+  if (!CGC_IN_BOUNDS(P, t, P.T)) return 0;  // uniform over the group
+  const int l = tg.q, lane = l & 31, wid = l >> 5;
+  const int x = l & 7, y = (l >> 3) & 7, z = l >> 6;
+  const int64_t g = (int64_t)t * TV + l, Np = P.Np;
+  int h = __ldcg(P.h + g), e = __ldcg(P.e + g), rT = __ldcg(P.rT + g);
+  int r[6];
+#pragma unroll
+  for (int d = 0; d < 6; ++d) r[d] = __ldcg(P.r + d * Np + g);
+  if (l >= 64 && l < 128) {  // y and z halo rows, 16 bytes per thread
+    const int i = l - 64, half = i & 1, k = (i >> 1) & 7, f = PY + (i >> 4);
+    const int nt = __ldcg(P.nbr + f * P.T + t);
+    const int src = (f == PY ? 64 * k : f == MY ? 64 * k + 56 : f == PZ ? 8 * k : 8 * k + 448) + 4 * half;
+    const int dst = (f == PY ? hrow(8, k) : f == MY ? hrow(-1, k) : f == PZ ? hrow(k, 8) : hrow(k, -1)) + 4 * half;
+    int4 v = make_int4(INF, INF, INF, INF);
+    if (nt >= 0 && CGC_IN_BOUNDS(P, nt, P.T)) v = __ldcg(reinterpret_cast<const int4*>(P.h + (int64_t)nt * TV + src));
+    *reinterpret_cast<int4*>(S.h[0] + dst) = v;
+    *reinterpret_cast<int4*>(S.h[1] + dst) = v;
+  } else if (l >= 128 && l < 256) {  // x halo
+    const int i = l - 128, f = i < 64 ? MX : PX, k = i & 63;
+    const int nt = __ldcg(P.nbr + f * P.T + t);
+    const int v = (nt >= 0 && CGC_IN_BOUNDS(P, nt, P.T)) ? __ldcg(P.h + (int64_t)nt * TV + 8 * k + (f == MX ? 7 : 0)) : INF;
+    S.h[0][HROWS * 8 + i] = v;
+    S.h[1][HROWS * 8 + i] = v;
+  } else if (l >= 256 && l < 262) {
+    S.nb[l - 256] = __ldcg(P.nbr + (l - 256) * P.T + t);
+  }
+  const int inst = __ldcg(P.tinst + t);
+  const int hdead = P.geo[inst].hdead;
+  const int hi = hrow(y, z) + x;
+  int off[6];  // neighbours in a buffer of heights
+  off[PX] = x < 7 ? hi + 1 : HROWS * 8 + 64 + (l >> 3);
+  off[MX] = x > 0 ? hi - 1 : HROWS * 8 + (l >> 3);
+  off[PY] = hi + 8; off[MY] = hi - 8;
+  off[PZ] = hi + 80; off[MZ] = hi - 80;
+  const bool in[6] = {x < 7, x > 0, y < 7, y > 0, z < 7, z > 0};
+  // where a push along d goes: the voxel's slot for the neighbour (and the
+  // neighbour's warp is told), or the face entry, whose only writer this is
+  uint32_t to[6], tell[6];
+#pragma unroll
+  for (int d = 0; d < 6; ++d) {
+    to[d] = smem_addr(in[d] ? &S.out[d][l] : &S.facc[d][d < 2 ? l >> 3 : d < 4 ? x + 8 * z : l & 63]);
+    tell[d] = smem_addr(in[d] ? &S.inbox[(l + loff(d)) >> 5] : &S.moved[d]);
+  }
+  const uint32_t from = smem_addr(&S.out[0][l]);
+  S.h[0][hi] = h;
+#pragma unroll
+  for (int d = 0; d < 6; ++d) S.out[d][l] = 0;
+  if (l < 384) (&S.facc[0][0])[l] = 0;
+  if (l < 24) S.inbox[l] = 0;  // and moved[]
+  tg.sync();
+
+  int sink = 0, pulses = 0, cur = 0;
+  bool dirty = false, any = true;
+  const int h0 = h;
+  for (int round = 0;; ++round) {
+    if (R > 0 && !(exact && round == 0)) {  // region relabel, as in sweep_tile
+      int dd = rT > 0 ? 1 : INF, c[6];
+      int* const H = S.h[cur];
+      H[hi] = dd;
+#pragma unroll
+      for (int d = 0; d < 6; ++d) c[d] = r[d] > 0 ? 1 : CLOSED;
+      tg.sync();
+      for (int it = 0; it < 600; ++it) {  // Bellman-Ford: < 512 steps in a tile, two per barrier
+        const int d0 = dd;
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const int a = __viaddmin_s32(H[off[0]], c[0], __viaddmin_s32(H[off[1]], c[1], dd));
+          const int b = __viaddmin_s32(H[off[2]], c[2], H[off[3]] + c[3]);
+          const int n = min(__viaddmin_s32(H[off[4]], c[4], a), __viaddmin_s32(H[off[5]], c[5], b));
+          if (n < dd) H[hi] = n;
+          dd = n;
+          __syncwarp();
+        }
+        if (!tg.any(dd < d0)) break;
+      }
+      h = max(h, dd);
+      if (h >= hdead) h = INF;
+      H[hi] = h;
+      tg.sync();
+    }
+    for (int p = 0; p < L; ++p) {
+      const int* H = S.h[cur];
+      ++pulses;
+      // (a voxel at INF has no neighbour at INF - 1 and no sink residual)
+      if (__any_sync(FULL, e > 0 && h < INF)) {
+        int hn[6];
+#pragma unroll
+        for (int d = 0; d < 6; ++d) hn[d] = H[off[d]];
+        const int e0 = e;
+        const int ds = min(e, rT);  // a voxel with a sink residual is at height 1: the labelling is valid
+        e -= ds;
+        rT -= ds;
+        sink += ds;
+        if (ds > 0) S.moved[6] = pulses;  // same value from every writer of this pulse
+        int dl[6];
+#pragma unroll
+        for (int d = 0; d < 6; ++d) dl[d] = hn[d] + 1 == h ? r[d] : 0;
+#pragma unroll
+        for (int d = 0; d < 6; ++d) {
+          dl[d] = min(e, dl[d]);
+          e -= dl[d];
+          r[d] -= dl[d];
+        }
+        push_out6(to, tell, dl, pulses);
+        dirty = dirty || e != e0;
+      }
+      tg.sync();
+      if (S.inbox[wid] == pulses) {  // uniform over the warp
+        int v[6], got = 0;
+        take6(from, in, v);
+        clear6(from, v);
+#pragma unroll
+        for (int d = 0; d < 6; ++d) {
+          e += v[d];
+          r[d] += v[d];
+          got |= v[d];
+        }
+        dirty = dirty || got > 0;
+      }
+      // Relabel, from the labels of the pulse's start: the labelling is valid,
+      // so the lowest residual neighbour mn is at h - 1 or higher (the sink
+      // counts as height 0), and 1 + mn is h itself where the voxel still has
+      // an admissible edge.
+      bool act = e > 0 && h < INF;
+      if (__any_sync(FULL, act)) {
+        int c[6];
+#pragma unroll
+        for (int d = 0; d < 6; ++d) {
+          const int hn = H[off[d]];
+          c[d] = r[d] > 0 ? hn : INF;
+        }
+        const int mn = min(min(min(c[0], c[1]), min(c[2], c[3])), min(c[4], c[5]));
+        int v = (rT > 0 ? 0 : mn) + 1;
+        if (v >= hdead) v = INF;
+        if (act) h = v;
+        act = act && v < INF;
+      }
+      S.h[cur ^ 1][hi] = h;
+      any = tg.any(act);
+      cur ^= 1;
+      if (!any) break;
+    }
+    if (!any || round + 1 >= max(R, 1)) break;
+  }
+
+  // write-back, the queue updates' chains of two dependent atomics first
+  if (l == 480) {
+    P.act[t] = (uint8_t)(any ? 1 : 0);
+    if (APPEND && any) queue_tile(P, stamp_q, t, id_self, list_self, cnt_self);
+    if (ex.tr_pulses && ex.tr_pulses[t] == 0) {
+      int last = 0;
+      for (int d = 0; d < 7; ++d) last = max(last, S.moved[d]);
+      ex.tr_pulses[t] = (uint8_t)(last > 0 ? min(last, 254) : 255);
+    }
+  }
+  if (l >= 448 && l < 454 && S.moved[l - 448]) {
+    const int nt = S.nb[l - 448];
+    if (nt < 0) {
+      raise_error(P, CGC_ERR_OVERFLOW);  // capacity leaving the grid
+    } else if (CGC_IN_BOUNDS(P, nt, P.T)) {
+      if (APPEND) queue_tile(P, stamp_q, nt, id_next, list_next, cnt_next);
+      P.act[nt] = 1;
+    }
+  }
+  if (l < 384) {  // flow that left the tile: excess and reverse residual of the neighbour
+    const int w = (&S.facc[0][0])[l];
+    if (w > 0) {
+      const int f = l >> 6, a = l & 7, b = (l >> 3) & 7, nt = S.nb[f];
+      if (nt >= 0 && CGC_IN_BOUNDS(P, nt, P.T)) {
+        const int src = f == PX ? 8 * a + 64 * b : f == MX ? 7 + 8 * a + 64 * b : f == PY ? a + 64 * b
+                      : f == MY ? a + 56 + 64 * b : f == PZ ? a + 8 * b : a + 8 * b + 448;
+        const int64_t ng = (int64_t)nt * TV + src;
+        atomicAdd(P.e + ng, w);
+        atomicAdd(P.r + (f ^ 1) * Np + ng, w);
+        atomicOr((unsigned*)(P.rmask + (ng & ~(int64_t)3)), (128u | (1u << (f ^ 1))) << (8 * (int)(ng & 3)));
+      }
+    }
+  }
+  if (h != h0) P.h[g] = h;
+  if (dirty) {
+    P.e[g] = e;
+    P.rT[g] = rT;
+    unsigned m = (rT > 0 ? 64u : 0u) | (e > 0 ? 128u : 0u);
+#pragma unroll
+    for (int d = 0; d < 6; ++d) {
+      P.r[d * Np + g] = r[d];
+      m |= (r[d] > 0 ? 1u : 0u) << d;
+    }
+    P.rmask[g] = (uint8_t)m;
+  }
+  if (__any_sync(FULL, sink > 0)) {
+    long long s = sink;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(FULL, s, o);
+    if (lane == 0) {
+      atomicAdd(P.flow + inst, (unsigned long long)s);
+      if (ex.sink_tiles) atomicAdd(ex.sink_tiles, 1);
+      if (ex.tr_sink) ex.tr_sink[t] = 1;
+    }
+  }
+  return pulses;
 }
 
 // Upload of tile t of an instance from its linear (x-fastest) device inputs
@@ -615,48 +1098,58 @@ __device__ __forceinline__ void bfs_queue_tile(const DevPool& P, const int t, co
 }
 
 // One BFS visit: relax h(v) = min(h(v), 1 + h(u)) over residual edges v->u
-// until the tile is stable; re-queue face neighbours whose halo changed.
-__device__ inline void bfs_tile(const DevPool& P, const int t, BfsShared& S, const uint32_t id_next,
-                         int32_t* list_next, int32_t* cnt_next) {
-  if (!CGC_IN_BOUNDS(P, t, P.T)) return;  // uniform over the block
-  if (__ldcg(P.tflag + t) & TF_DEAD) return;  // uniform over the block; nothing can change
-  const int l = threadIdx.x;
-  const int nb = l < 6 ? __ldcg(P.nbr + l * P.T + t) : -1;  // face neighbour, for the re-queue
-  const int x = l & 7, y = (l >> 3) & 7, z = l >> 6;
-  const int64_t g = (int64_t)t * TV + l;
-  int h = __ldcg(P.h + g);
-  const int h0 = h;
-  const unsigned m = __ldcg(P.rmask + g);
-  const bool has_excess = (m & 128u) != 0;
-  const int hi = halo_index(x, y, z);
-  S.h[0][hi] = h;
-  load_halo_heights(P, t, S.h);
-  if (l == 0) S.flags = 0;
-  __syncthreads();
-  int cur = 0;
-  for (int it = 0; it < 1024; ++it) {  // converges in < 512 steps (path length in a tile)
-    int mn = h;
+// until the tile is stable; re-queue face neighbours whose halo changed.  The
+// face and activity flags are set as heights drop (they never rise again), so
+// the barrier that ends the relaxation also publishes them.  The caller
+// synchronises the group before S is used again; returns 1 for a visited tile.
+__device__ __forceinline__ int bfs_tile(const DevPool& P, const TileGroup<GROUP> tg, const int t, BfsShared& S,
+                                        const uint32_t id_next, int32_t* list_next, int32_t* cnt_next) {
+  if (!CGC_IN_BOUNDS(P, t, P.T)) return 0;  // uniform over the group
+  const int q = tg.q, half = q & 1, y = (q >> 1) & 7, z = q >> 4;
+  const int row = hrow(y, z) + 4 * half;
+  const int64_t g = (int64_t)t * TV + 4 * q;
+  const int dead = __ldcg(P.tflag + t) & TF_DEAD;
+  int h[4];
+  ldcg4(P.h + g, h);
+  const unsigned m = __ldcg(reinterpret_cast<const unsigned*>(P.rmask + g));
+  const int hx = load_halo_heights(P, t, q, S.h, nullptr);
+  if (dead) return 0;  // uniform over the group; nothing can change
+  const int nb = q >= 32 && q < 38 ? __ldcg(P.nbr + (q - 32) * P.T + t) : -1;  // face neighbour, for the re-queue
+  st4(S.h + row, h);
+  if (q < 8) S.face[q] = 0;
+  if (q == 8) S.act = 0;
+  tg.sync();
+  // faces the thread's voxels lie on: its own row end, y and z
+  const int fx = half ? PX : MX, kx = half ? 3 : 0;
+  bool changed = false;
+  int c[6][4];
 #pragma unroll
-    for (int d = 0; d < 6; ++d)
-      if ((m >> d) & 1u) mn = min(mn, S.h[cur][hi + hoff(d)] + 1);
-    S.h[cur ^ 1][hi] = mn;
-    const int any = __syncthreads_or(mn < h);
-    h = mn;
-    cur ^= 1;
-    if (!any) break;
+  for (int d = 0; d < 6; ++d)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) c[d][k] = ((m >> (8 * k + d)) & 1u) ? 1 : CLOSED;
+  for (int it = 0; it < 1024; ++it) {  // converges in < 512 steps (path length in a tile)
+    const int hxe = kx ? h[3] : h[0];
+    const bool ch = relax_row(S.h, row, half, hx, h, c);
+    if (ch) {
+      changed = true;
+      if ((kx ? h[3] : h[0]) < hxe) S.face[fx] = 1;
+      if (y == 7) S.face[PY] = 1;
+      if (y == 0) S.face[MY] = 1;
+      if (z == 7) S.face[PZ] = 1;
+      if (z == 0) S.face[MZ] = 1;
+    }
+    if (it == 0 || ch) {
+      bool act = false;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) act = act || (((m >> (8 * k + 7)) & 1u) && h[k] < INF);
+      if (act) S.act = 1;
+    }
+    if (!tg.any(ch)) break;
   }
-  if (h < h0) {
-    P.h[g] = h;
-    const int fb = face_bits(x, y, z);
-    if (fb) atomicOr(&S.flags, fb);
-  }
-  const int act = __syncthreads_or(has_excess && h < INF);
-  if (l == 0) {
-    P.act[t] = (uint8_t)(act ? 1 : 0);  // heights only drop in later visits: the last visit's value is final
-    atomicAdd(P.stats + S_TILES_BFS, 1ull);
-  }
-  if (l < 6 && ((S.flags >> l) & 1) && nb >= 0) queue_tile(P, P.stamp_bfs, nb, id_next, list_next, cnt_next);
-  __syncthreads();
+  if (q >= 32 && q < 38 && S.face[q - 32] && nb >= 0) queue_tile(P, P.stamp_bfs, nb, id_next, list_next, cnt_next);
+  if (changed) st4(P.h + g, h);
+  if (q == 0) P.act[t] = S.act;  // heights only drop in later visits: the last visit's value is final
+  return 1;
 }
 
 // ---------------------------------------------------------------------------
@@ -705,101 +1198,151 @@ __device__ __forceinline__ void inval_queue_tile(const DevPool& P, const int t, 
 // tile is stable (drops are monotone, so in-place updates are safe and the
 // result is the largest supported set); re-queue the face neighbours of
 // dropped face voxels, and list the tile once (stamp_inc) for the BFS rounds.
-__device__ inline void inval_tile(const DevPool& P, const int t, BfsShared& S, const uint32_t id_next,
-                                  int32_t* list_next, int32_t* cnt_next, const uint32_t id_bfs, int32_t* list_bfs,
-                                  int32_t* cnt_bfs) {
-  if (!CGC_IN_BOUNDS(P, t, P.T)) return;  // uniform over the block
-  const int l = threadIdx.x;
-  const int nb = l < 6 ? __ldcg(P.nbr + l * P.T + t) : -1;  // face neighbour, for the re-queue
-  const int x = l & 7, y = (l >> 3) & 7, z = l >> 6;
-  const int64_t g = (int64_t)t * TV + l;
-  int h = __ldcg(P.h + g);
-  const unsigned m = __ldcg(P.rmask + g);
-  const int hi = halo_index(x, y, z);
-  S.h[0][hi] = h;
-  load_halo_heights(P, t, S.h);
-  if (l == 0) S.flags = 0;
-  __syncthreads();
+// The caller synchronises the group before S is used again.
+__device__ __forceinline__ int inval_tile(const DevPool& P, const TileGroup<GROUP> tg, const int t, BfsShared& S,
+                                          const uint32_t id_next, int32_t* list_next, int32_t* cnt_next,
+                                          const uint32_t id_bfs, int32_t* list_bfs, int32_t* cnt_bfs) {
+  if (!CGC_IN_BOUNDS(P, t, P.T)) return 0;  // uniform over the group
+  const int q = tg.q, half = q & 1, y = (q >> 1) & 7, z = q >> 4;
+  const int row = hrow(y, z) + 4 * half;
+  const int64_t g = (int64_t)t * TV + 4 * q;
+  int h[4];
+  ldcg4(P.h + g, h);
+  const unsigned m = __ldcg(reinterpret_cast<const unsigned*>(P.rmask + g));
+  const int hx = load_halo_heights(P, t, q, S.h, nullptr);
+  const int nb = q >= 32 && q < 38 ? __ldcg(P.nbr + (q - 32) * P.T + t) : -1;  // face neighbour, for the re-queue
+  st4(S.h + row, h);
+  if (q < 8) S.face[q] = 0;
+  if (q == 8) S.any = 0;
+  tg.sync();
   bool dropped = false;
   for (int it = 0; it < 1024; ++it) {  // a drop per step climbs one height: < 512 steps in a tile
-    bool drop = false;
-    if (h < INF && !((m & 64u) && h == 1)) {
-      bool sup = false;
+    const int4 yp = ld4(S.h + row + 8), ym = ld4(S.h + row - 8), zp = ld4(S.h + row + 80), zm = ld4(S.h + row - 80);
+    const int xo = __shfl_xor_sync(FULL, half ? h[0] : h[3], 1);
+    bool ch = false;
 #pragma unroll
-      for (int d = 0; d < 6; ++d)
-        if ((m >> d) & 1u) sup = sup || S.h[0][hi + hoff(d)] == h - 1;
-      drop = !sup;
+    for (int k = 0; k < 4; ++k) {
+      const unsigned mk = m >> (8 * k);
+      const int hm = h[k] - 1;
+      const int r = k < 3 ? h[k < 3 ? k + 1 : 3] : (half ? hx : xo);
+      const int l = k > 0 ? h[k > 0 ? k - 1 : 0] : (half ? xo : hx);
+      const bool sup = ((mk & 64u) && hm == 0) || ((mk & 1u) && r == hm) || ((mk & 2u) && l == hm) ||
+                       ((mk & 4u) && at(yp, k) == hm) || ((mk & 8u) && at(ym, k) == hm) ||
+                       ((mk & 16u) && at(zp, k) == hm) || ((mk & 32u) && at(zm, k) == hm);
+      if (h[k] < INF && !sup) {
+        h[k] = INF;
+        ch = true;
+        if (k == (half ? 3 : 0)) S.face[half ? PX : MX] = 1;
+      }
     }
-    if (drop) {
-      h = INF;
-      S.h[0][hi] = INF;
+    if (ch) {
+      st4(S.h + row, h);
       dropped = true;
+      S.any = 1;
+      if (y == 7) S.face[PY] = 1;
+      if (y == 0) S.face[MY] = 1;
+      if (z == 7) S.face[PZ] = 1;
+      if (z == 0) S.face[MZ] = 1;
     }
-    if (!__syncthreads_or(drop)) break;
+    if (!tg.any(ch)) break;
   }
-  if (dropped) {
-    P.h[g] = INF;
-    const int fb = face_bits(x, y, z);
-    if (fb) atomicOr(&S.flags, fb);
-  }
-  const int any = __syncthreads_or(dropped);
-  if (l == 0) atomicAdd(P.stats + S_TILES_CHECK, 1ull);
-  if (l == 32 && any) queue_tile(P, P.stamp_inc, t, id_bfs, list_bfs, cnt_bfs);
-  if (l < 6 && ((S.flags >> l) & 1) && nb >= 0) queue_tile(P, P.stamp_bfs, nb, id_next, list_next, cnt_next);
-  __syncthreads();
+  if (q == 0 && S.any) queue_tile(P, P.stamp_inc, t, id_bfs, list_bfs, cnt_bfs);
+  if (q >= 32 && q < 38 && S.face[q - 32] && nb >= 0) queue_tile(P, P.stamp_bfs, nb, id_next, list_next, cnt_next);
+  if (dropped) st4(P.h + g, h);
+  return 1;
 }
 
 // ---------------------------------------------------------------------------
 // Source-side reachability (canonical cut) after the maximum preflow:
 // closure of {v : e(v) > 0} over residual edges, seeded by reach_init_tile_w
-// (a warp per tile).
-__device__ inline void reach_tile(const DevPool& P, const int t, ReachShared& S, const uint32_t id_next,
-                           int32_t* list_next, int32_t* cnt_next) {
-  if (!CGC_IN_BOUNDS(P, t, P.T)) return;  // uniform over the block
-  const int l = threadIdx.x;
-  const int nb = l < 6 ? __ldcg(P.nbr + l * P.T + t) : -1;  // face neighbour, for the re-queue
-  const int x = l & 7, y = (l >> 3) & 7, z = l >> 6;
-  const int64_t g = (int64_t)t * TV + l;
-  int rc = __ldcg(P.reach + g);
-  const int rc0 = rc;
-  const int hi = halo_index(x, y, z);
-  S.rc[0][hi] = (unsigned char)rc;
-  S.m[hi] = __ldcg(P.rmask + g);
-  for_halo_entry(l, [&](int f, int hh, int src) {
-    const int nt = __ldcg(P.nbr + f * P.T + t);
-    unsigned char rv = 0, mv = 0;
-    if (nt >= 0 && CGC_IN_BOUNDS(P, nt, P.T)) {
-      rv = __ldcg(P.reach + (int64_t)nt * TV + src);
-      mv = __ldcg(P.rmask + (int64_t)nt * TV + src);
-    }
-    S.rc[0][hh] = rv; S.rc[1][hh] = rv; S.m[hh] = mv;
-  });
-  if (l == 0) S.flags = 0;
-  __syncthreads();
-  int cur = 0;
-  for (int it = 0; it < 1024; ++it) {
-    bool ch = false;
-    if (!rc) {
+// (a warp per tile).  One warp visits a tile, with the reach set and the
+// residual masks as bits: lane l owns the rows y = 2(l&3), +1 of plane z = l>>2
+// (16 voxels, bit = 8 (y&1) + x), so a step of the closure is a few shifts and
+// shuffles, without shared memory or barriers.
+__device__ __forceinline__ unsigned byte_bits(unsigned w, int bit) {  // bit `bit` of each byte of w -> bits 0..3
+  w = (w >> bit) & 0x01010101u;
+  return (w * 0x01020408u) >> 24 & 15u;  // byte k -> bit k
+}
+
+__device__ __forceinline__ void reach_tile_w(const DevPool& P, const int t, const uint32_t id_next, int32_t* list_next,
+                                             int32_t* cnt_next) {
+  if (!CGC_IN_BOUNDS(P, t, P.T)) return;  // uniform over the warp
+  const int lane = threadIdx.x & 31, j = lane & 3, z = lane >> 2;
+  const int64_t g = (int64_t)t * TV + 16 * lane;
+  const uint4 rc4 = __ldcg(reinterpret_cast<const uint4*>(P.reach + g));
+  const uint4 m4 = __ldcg(reinterpret_cast<const uint4*>(P.rmask + g));
+  const int nb = lane < 6 ? __ldcg(P.nbr + lane * P.T + t) : -1;
+  int nt[6];
 #pragma unroll
-      for (int d = 0; d < 6; ++d) {
-        const int u = hi + hoff(d);
-        if (S.rc[cur][u] && ((S.m[u] >> (d ^ 1)) & 1u)) ch = true;
-      }
+  for (int d = 0; d < 6; ++d) nt[d] = __shfl_sync(FULL, nb, d);
+  // flow of reachability into this lane's voxels through the tile's faces: a
+  // reached voxel of the neighbour with a residual edge towards the tile
+  unsigned in = 0;
+  auto row_in = [&](int f, int src) {  // 8 voxels of a neighbour's row at src
+    const int64_t ng = (int64_t)nt[f] * TV + src;
+    const uint2 a = __ldcg(reinterpret_cast<const uint2*>(P.reach + ng));
+    const uint2 b = __ldcg(reinterpret_cast<const uint2*>(P.rmask + ng));
+    const int bit = f ^ 1;
+    return byte_bits(a.x, 0) & byte_bits(b.x, bit) | (byte_bits(a.y, 0) & byte_bits(b.y, bit)) << 4;
+  };
+#pragma unroll
+  for (int d = 0; d < 6; ++d)
+    if (nt[d] >= 0 && !CGC_IN_BOUNDS(P, nt[d], P.T)) nt[d] = -1;
+  if (nt[PY] >= 0 && j == 3) in |= row_in(PY, 64 * z) << 8;
+  if (nt[MY] >= 0 && j == 0) in |= row_in(MY, 64 * z + 56);
+  if (nt[PZ] >= 0 && z == 7) in |= row_in(PZ, 16 * j) | row_in(PZ, 16 * j + 8) << 8;
+  if (nt[MZ] >= 0 && z == 0) in |= row_in(MZ, 448 + 16 * j) | row_in(MZ, 448 + 16 * j + 8) << 8;
+#pragma unroll
+  for (int s = 0; s < 2; ++s) {  // x faces: the voxel next to each row end
+    if (nt[PX] >= 0) {
+      const int64_t ng = (int64_t)nt[PX] * TV + 16 * lane + 8 * s;
+      if (__ldcg(P.reach + ng) && ((__ldcg(P.rmask + ng) >> MX) & 1)) in |= 0x80u << (8 * s);
     }
-    if (ch) rc = 1;
-    S.rc[cur ^ 1][hi] = (unsigned char)rc;
-    const int any = __syncthreads_or(ch);
-    cur ^= 1;
-    if (!any) break;
+    if (nt[MX] >= 0) {
+      const int64_t ng = (int64_t)nt[MX] * TV + 16 * lane + 8 * s + 7;
+      if (__ldcg(P.reach + ng) && ((__ldcg(P.rmask + ng) >> PX) & 1)) in |= 0x01u << (8 * s);
+    }
   }
-  if (rc && !rc0) {
-    P.reach[g] = 1;
-    const int fb = face_bits(x, y, z);
-    if (fb) atomicOr(&S.flags, fb);
+  auto bits16 = [](const uint4& w, int bit) {
+    return byte_bits(w.x, bit) | byte_bits(w.y, bit) << 4 | byte_bits(w.z, bit) << 8 | byte_bits(w.w, bit) << 12;
+  };
+  const unsigned r0 = bits16(rc4, 0);
+  unsigned M[6];
+#pragma unroll
+  for (int d = 0; d < 6; ++d) M[d] = bits16(m4, d);
+  unsigned r = r0 | in;
+  for (int it = 0; it < 1024; ++it) {  // < 512 steps
+    unsigned n = r | (r & M[PX] & 0x7f7fu) << 1;
+    n |= (n & M[MX] & 0xfefeu) >> 1;
+    const unsigned yp = n & M[PY], ym = n & M[MY];
+    const unsigned yu = __shfl_up_sync(FULL, yp, 1), yd = __shfl_down_sync(FULL, ym, 1);
+    const unsigned zu = __shfl_up_sync(FULL, n & M[PZ], 4), zd = __shfl_down_sync(FULL, n & M[MZ], 4);
+    n |= (yp & 0xffu) << 8 | (ym >> 8 & 0xffu);
+    if (j > 0) n |= yu >> 8 & 0xffu;
+    if (j < 3) n |= (yd & 0xffu) << 8;
+    if (z > 0) n |= zu;
+    if (z < 7) n |= zd;
+    const bool ch = n != r;
+    r = n;
+    if (!__any_sync(FULL, ch)) break;
   }
-  __syncthreads();
-  if (l < 6 && ((S.flags >> l) & 1) && nb >= 0) queue_tile(P, P.stamp_bfs, nb, id_next, list_next, cnt_next);
-  __syncthreads();
+  const unsigned fresh = r & ~r0;
+  unsigned faces = 0;
+  if (fresh) {
+    // only voxels with a residual edge through the face can reach the neighbour
+    faces = ((fresh & M[PX] & 0x8080u) ? 1u << PX : 0u) | ((fresh & M[MX] & 0x0101u) ? 1u << MX : 0u) |
+            ((j == 3 && (fresh & M[PY] & 0xff00u)) ? 1u << PY : 0u) | ((j == 0 && (fresh & M[MY] & 0xffu)) ? 1u << MY : 0u) |
+            ((z == 7 && (fresh & M[PZ])) ? 1u << PZ : 0u) | ((z == 0 && (fresh & M[MZ])) ? 1u << MZ : 0u);
+    unsigned w[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const unsigned b = r >> (4 * k);
+      w[k] = (b & 1u) | (b & 2u) << 7 | (b & 4u) << 14 | (b & 8u) << 21;
+    }
+    *reinterpret_cast<uint4*>(P.reach + g) = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+  faces = __reduce_or_sync(FULL, faces);
+  if (lane < 6 && ((faces >> lane) & 1) && nb >= 0) queue_tile(P, P.stamp_bfs, nb, id_next, list_next, cnt_next);
 }
 
 }  // namespace cgc

@@ -66,8 +66,7 @@ constexpr int64_t kOffCnt = kOffLists + al256(7 * kMaxTiles * 4);
 constexpr int64_t kOffFlow = kOffCnt + al256(C_NCOUNTERS * 4);
 constexpr int64_t kOffGeo = kOffFlow + al256(8);
 constexpr int64_t kOffStats = kOffGeo + al256(sizeof(InstGeo));
-constexpr int64_t kOffErr = kOffStats + al256(S_NSTATS * 8);
-constexpr int64_t kOffBar = kOffErr + al256(4);
+constexpr int64_t kOffBar = kOffStats + al256(S_NSTATS * 8);  // barrier count, error word
 constexpr int64_t kScratchBytes = kOffBar + al256(8);
 
 }  // namespace
@@ -82,7 +81,7 @@ namespace {
 struct DeviceSetup {
   bool ready = false;
   unsigned char* scratch = nullptr;  // device address of g_noalloc_scratch
-  int coop_blocks = 0;
+  int sms = 0;
 };
 std::mutex g_setup_mutex;
 DeviceSetup g_setup[kMaxDevices];
@@ -97,12 +96,11 @@ int setup_device(int dev, DeviceSetup** out) {
     cudaError_t e = cudaGetSymbolAddress(&ptr, g_noalloc_scratch);
     if (e != cudaSuccess)
       return fail(CGC_ERR_CUDA, std::string("cudaGetSymbolAddress(g_noalloc_scratch): ") + cudaGetErrorString(e));
-    int occ = 0, sms = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_solve, 512, 0);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    int sms = 0;
+    e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return fail(CGC_ERR_CUDA, std::string("noalloc set-up: ") + cudaGetErrorString(e));
     s.scratch = static_cast<unsigned char*>(ptr);
-    s.coop_blocks = (occ > 0 ? occ : 1) * sms;
+    s.sms = sms;
     s.ready = true;
   }
   *out = &s;
@@ -167,8 +165,8 @@ extern "C" int cgc_grid_maxflow_noalloc(int32_t X, int32_t Y, int32_t Z, const i
   P.stamp_inc = (uint32_t*)(base + kOffStampI);
   P.lists = (int32_t*)(base + kOffLists); P.cnt = (int32_t*)(base + kOffCnt);
   P.flow = (unsigned long long*)(base + kOffFlow); P.geo = (const InstGeo*)(base + kOffGeo);
-  P.stats = (unsigned long long*)(base + kOffStats); P.err = (int32_t*)(base + kOffErr);
-  P.bar = (uint32_t*)(base + kOffBar);
+  P.stats = (unsigned long long*)(base + kOffStats);
+  P.bar = (uint32_t*)(base + kOffBar); P.err = (int32_t*)(P.bar + 1);
   // the residual planes are addressed as r + d*Np: use the actual Np (the
   // 6 planes of this grid fit in the 6*kMaxVoxels bytes reserved for them)
 
@@ -198,10 +196,9 @@ extern "C" int cgc_grid_maxflow_noalloc(int32_t X, int32_t Y, int32_t Z, const i
   o.trace_cycles = 0;
   o.exclusive = 0;  // the scratch holds one half of stamps
   const SolveParams prm = solve_params(o);
-  void* args[] = {(void*)&P, (void*)&prm};
   // a preparation error (overflowing capacities) makes every CTA leave at its
   // first barrier
-  NA_CUDA(cudaLaunchCooperativeKernel((const void*)k_solve, dim3(su->coop_blocks), dim3(512), args, 0, st));
+  if ((rc = launch_solve(P, o, prm, dev, su->sms, st))) return rc;
   if (source_side) {
     k_segments<<<(unsigned)((G.hdead + 254) / 256 < 65535 ? (G.hdead + 254) / 256 : 65535), 256, 0, st>>>(
         P, 0, CGC_SEG_SOURCE_MIN, source_side, 1, 0);
@@ -214,7 +211,7 @@ extern "C" int cgc_grid_maxflow_noalloc(int32_t X, int32_t Y, int32_t Z, const i
   }
   struct { unsigned long long flow; int32_t err; } res;
   NA_CUDA(cudaMemcpyAsync(&res.flow, base + kOffFlow, 8, cudaMemcpyDeviceToHost, st));
-  NA_CUDA(cudaMemcpyAsync(&res.err, base + kOffErr, 4, cudaMemcpyDeviceToHost, st));
+  NA_CUDA(cudaMemcpyAsync(&res.err, base + kOffBar + 4, 4, cudaMemcpyDeviceToHost, st));
   NA_CUDA(cudaStreamSynchronize(st));
   if (res.err) {
     const char* what = res.err == CGC_ERR_OVERFLOW ? "capacities may overflow int32 excess/residuals"

@@ -61,9 +61,6 @@ struct Pool {
   int32_t* pinned_cnt = nullptr; // host-pinned counters
   bool solved = false;
   int sms = 148;
-  int coop_blocks = 0;           // co-resident CTAs of k_solve
-  int coop_blocks3 = 0;          // co-resident CTAs of k_solve3
-  int coop_blocks4 = 0;          // co-resident CTAs of k_solve4
   int sweep_blocks = 0;
   cgc_stats st{};
   std::vector<int64_t> flows;
@@ -123,7 +120,7 @@ int pool_solve_wait(Pool& p);
 // cooperative launch of this library on the device has ended
 int coop_launch_ordered(int device, cudaStream_t stream, const std::function<int()>& launch);
 // cooperative launch of the persistent solve kernel selected by the options
-int launch_solve(Pool& p, const cgc_options& o, const DevPool& d, const SolveParams& prm, cudaStream_t stream);
+int launch_solve(const DevPool& d, const cgc_options& o, const SolveParams& prm, int device, int sms, cudaStream_t stream);
 int pool_segments(Pool& p, int inst, int which, uint8_t* out, uint8_t mask, uint8_t bg, bool host);
 int pool_residuals(Pool& p, int inst, int32_t* const res[6], int32_t* resT, int32_t* excess);
 int pool_trace(Pool& p, int64_t* out, int32_t cap, int32_t* count);

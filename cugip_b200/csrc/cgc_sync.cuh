@@ -11,34 +11,38 @@ __device__ __forceinline__ uint64_t sync_globaltimer_ns() {
   return t;
 }
 
-// bar[0] counts arrivals, bar[1] is the generation.  Waits are bounded: after
-// `limit_ns` the waiting CTA records CGC_ERR_TIMEOUT in *err and every CTA
-// leaves at its next barrier.  Returns false once an error was recorded.
-__device__ __forceinline__ bool grid_barrier(uint32_t* bar, int32_t* err, uint64_t limit_ns) {
+// The barrier's two words: bar[0] counts arrivals (zeroed before the launch),
+// bar[1] is the launch's error word.  `target` is the arrival count that ends
+// the CTA's next barrier (0 before the first one; kept per CTA, in a register).
+// Waits are bounded: after `limit_ns` the waiting CTA records CGC_ERR_TIMEOUT,
+// and every CTA leaves at this barrier or the next one, since a waiting CTA
+// also watches the error word.  Returns false once an error was recorded.
+//
+// A barrier costs one release-add and the poll that sees the last one: there
+// is no reset and no second round trip for a generation, and both words come
+// with one 8-byte load.
+__device__ __forceinline__ bool grid_barrier(uint32_t* bar, uint32_t& target, uint64_t limit_ns) {
+  __shared__ int s_ok;
+  target += gridDim.x;
   __syncthreads();
   if (threadIdx.x == 0) {
-    volatile uint32_t* gen = bar + 1;
-    const uint32_t g0 = *gen;
-    __threadfence();
-    const uint32_t arrived = atomicAdd(bar, 1u) + 1u;
-    if (arrived == gridDim.x) {
-      atomicExch(bar, 0u);
-      __threadfence();
-      atomicAdd(bar + 1, 1u);
-    } else {
-      const uint64_t t0 = sync_globaltimer_ns();
-      while (*gen == g0) {
-        __nanosleep(64);
-        if (sync_globaltimer_ns() - t0 > limit_ns) {
-          atomicCAS(err, 0, CGC_ERR_TIMEOUT);
-          break;
-        }
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+    const uint64_t t0 = sync_globaltimer_ns();
+    uint32_t n, err;
+    for (;;) {
+      asm volatile("ld.relaxed.gpu.global.v2.u32 {%0, %1}, [%2];" : "=r"(n), "=r"(err) : "l"(bar) : "memory");
+      if (err != 0 || (int32_t)(n - target) >= 0) break;
+      if (sync_globaltimer_ns() - t0 > limit_ns) {
+        atomicCAS(bar + 1, 0u, (uint32_t)CGC_ERR_TIMEOUT);
+        err = CGC_ERR_TIMEOUT;
+        break;
       }
     }
-    __threadfence();
+    asm volatile("fence.acq_rel.gpu;" ::: "memory");
+    s_ok = err == 0;
   }
   __syncthreads();
-  return *(volatile int32_t*)err == 0;
+  return s_ok != 0;
 }
 
 }  // namespace cgc
