@@ -10,10 +10,10 @@
 //   * CSR built on the device: per-vertex degree count, exclusive scan,
 //     atomic scatter of the two arcs of every edge with reverse-arc links.
 //     The original arc capacities are kept, so a graph can be solved again.
-//   * one cooperative launch per solve: exact global relabel (BFS from the
-//     vertices with a sink residual over reverse residual arcs, heights set by
-//     CAS), then up to K synchronous pulses over a deduplicated active-vertex
-//     list: a push step with fixed labels (a vertex pushes along arcs to
+//   * one cooperative launch per solve, 4 to 16 lanes per vertex: exact global
+//     relabel (BFS from the vertices with a sink residual over reverse residual
+//     arcs, heights set by CAS), then up to K synchronous pulses over a
+//     deduplicated active-vertex list: a push step with fixed labels (a vertex pushes along arcs to
 //     neighbours one level lower; excess and reverse residuals of the
 //     neighbour by atomics) and a relabel step (1 + the lowest residual
 //     neighbour; labels only grow, so concurrent relabels keep them valid).
@@ -38,7 +38,7 @@
 namespace cgc {
 namespace {
 
-constexpr int CSR_THREADS = 256;
+constexpr int CSR_THREADS = 1024;  // solve: one CTA per SM
 constexpr int SCAN_BLOCK = 1024;
 
 enum CsrStat { CS_PULSES = 0, CS_RELABELS, CS_LEVELS, CS_PUSHES, CS_BFS_VISITS, CS_NS_BFS, CS_NS_PUSH, CS_NS_REACH, CS_N = 16 };
@@ -61,6 +61,7 @@ struct CsrDev {
   int32_t* reach;            // n: source side
   uint32_t* stamp;           // n: last list the vertex was queued for
   int32_t* list;             // 2n: two vertex lists
+  int2* front;               // 2n: two BFS frontiers (arc ranges of their vertices)
   int32_t* cnt;              // CC_N counters
   unsigned long long* flow;  // 1
   unsigned long long* stats; // CS_N
@@ -76,8 +77,21 @@ struct CsrParams {
 
 __device__ __forceinline__ int ldv(const int32_t* p) { return *(volatile const int32_t*)p; }
 
+// loaded ahead of the test that may discard it
+__device__ __forceinline__ int ld_early(const int32_t* p) {
+  int v;
+  asm volatile("ld.global.cg.s32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ int2 ld_early(const int2* p) {
+  int2 v;
+  asm volatile("ld.global.cg.v2.s32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+  return v;
+}
+
 // warp-aggregated append (all lanes of the warp call it)
-__device__ __forceinline__ void csr_append(bool pred, int32_t item, int32_t* list, int32_t* cnt) {
+template <typename T>
+__device__ __forceinline__ void csr_append(bool pred, T item, T* list, int32_t* cnt) {
   const unsigned mask = __ballot_sync(0xffffffffu, pred);
   if (!mask) return;
   const int lane = threadIdx.x & 31;
@@ -213,34 +227,72 @@ __global__ void k_csr_prepare(CsrDev D) {
   if ((threadIdx.x & 31) == 0 && through) atomicAdd(D.flow, (unsigned long long)through);
 }
 
-__global__ void __launch_bounds__(CSR_THREADS) k_csr_solve(CsrDev D, CsrParams prm) {
+// W lanes work on a vertex: they read its arcs W at a time, so a vertex costs
+// a few dependent memory round trips instead of one chain per arc.  A round of
+// the BFS or a pulse is bound by those round trips (about 0.3 us each) and by
+// the grid barrier (one CTA per SM, one arrival each), not by bytes.  A thread
+// per vertex and a loop over its arcs took 15 us per BFS round and 32 us per
+// pulse on the layered graph of 100 x 1024 vertices, this takes 4 and 10 (solve
+// 13.7 -> 3.9 ms); random graph of 200 k vertices, 800 k edges: 5.6 -> 2.1 ms.
+// W is 16, 8 or 4 by the average degree (graph_create), so that few lanes idle.
+// Spreading a short list's vertices over all SMs was not faster (BFS 2.9 -> 3.0 ms).
+template <int W>
+__global__ void __launch_bounds__(CSR_THREADS, 1) k_csr_solve(CsrDev D, CsrParams prm) {
+  constexpr unsigned FULL = 0xffffffffu;
   const int n = D.n;
   const int lane = threadIdx.x & 31;
+  const int sub = threadIdx.x & (W - 1);       // lane of the vertex
   const int gt = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+  const int slot = gt / W, slots = nt / W;     // vertices of a list: slot, slot + slots, ...
+  const int wslot = (gt - lane) / W;           // the warp's first slot: loops over a list are uniform over a warp
   int32_t* const L[2] = {D.list, D.list + n};
   int32_t* const cb = D.cnt + CC_BFS0;    // 3 rotating counters of the BFS frontiers
   int32_t* const cp = D.cnt + CC_PULSE0;  // 3 rotating counters of the pulse lists
   const bool lead = gt == 0;
   uint32_t sid = 0;
-  long long pulses = 0, relabels = 0, levels = 0;
+  int pulses = 0, relabels = 0, levels = 0;
+  long long flow = 0;  // delivered to the sink by this thread
   unsigned long long ns_bfs = 0, ns_push = 0, ns_reach = 0;
   uint64_t tmark = sync_globaltimer_ns();
   auto lap = [&](unsigned long long& acc) {
+    if (!lead) return;
     const uint64_t now = sync_globaltimer_ns();
     acc += now - tmark;
     tmark = now;
   };
   uint32_t bar_target = 0;
   auto sync = [&]() { return grid_barrier(D.bar, bar_target, prm.limit_ns); };
-  // frontier BFS over lists L[k&1] with counters cb[k%3]; `visit` appends
-  // to the next frontier; returns the number of rounds, -1 on a failed barrier
-  auto bfs = [&](auto&& visit) -> int {
+  // Frontier BFS.  A frontier holds the arc ranges of its vertices, loaded
+  // while the vertex is claimed, so the next round starts with the arcs.
+  // take(arc, head, k) says whether the arc's head joins the next frontier;
+  // returns the number of rounds, -1 on a failed barrier.
+  auto arcs_of = [&](int v) { return make_int2(__ldg(D.row + v), __ldg(D.row + v + 1)); };
+  auto bfs = [&](auto&& take) -> int {
     int k = 0;
     for (;;) {
+      const int2* lc = D.front + (k & 1) * (int64_t)n;
+      int2* ln = D.front + ((k + 1) & 1) * (int64_t)n;
+      int2 f = slot < n ? ld_early(lc + slot) : make_int2(0, 0);
       const int nf = ldv(cb + k % 3);
       if (nf == 0) return k;
       if (lead) cb[(k + 2) % 3] = 0;
-      for (int i = gt; i < nf; i += nt) visit(L[k & 1][i], k, L[(k + 1) & 1], cb + (k + 1) % 3);
+      for (int i0 = wslot, i = slot; i0 < nf;) {
+        int a = i < nf ? f.x + sub : 0;
+        const int a1 = i < nf ? f.y : 0;
+        for (; __any_sync(FULL, a < a1); a += W) {
+          bool ok = a < a1;
+          int2 r = make_int2(0, 0);
+          if (ok) {
+            const int v = __ldg(D.to + a);
+            r = arcs_of(v);
+            ok = take(a, v, k);
+          }
+          csr_append(ok, r, ln, cb + (k + 1) % 3);
+        }
+        i0 += slots;
+        i += slots;
+        if (i < nf) f = __ldcg(lc + i);
+      }
       ++k;
       if (!sync()) return -1;
     }
@@ -253,17 +305,13 @@ __global__ void __launch_bounds__(CSR_THREADS) k_csr_solve(CsrDev D, CsrParams p
     for (int v = gt; v - lane < n; v += nt) {
       const bool seed = v < n && __ldcg(D.rT + v) > 0;
       if (v < n) D.h[v] = seed ? 1 : INF;
-      csr_append(seed, v, L[0], cb + 0);
+      csr_append(seed, seed ? arcs_of(v) : make_int2(0, 0), D.front, cb + 0);
     }
     if (!sync()) return;
-    const int rounds = bfs([&](int u, int k, int32_t* next, int32_t* cnext) {
-      const int lev = k + 2;  // the frontier of round k has height k + 1
-      const int a1 = D.row[u + 1];
-      for (int a = D.row[u]; a < a1; ++a) {
-        const int v = D.to[a];
-        if (__ldcg(D.res + D.rev[a]) > 0 && ldv(D.h + v) == INF && atomicCAS(D.h + v, INF, lev) == INF)
-          next[atomicAdd(cnext, 1)] = v;
-      }
+    const int rounds = bfs([&](int a, int v, int k) {
+      const int r = __ldcg(D.res + __ldg(D.rev + a));
+      // the frontier of round k has height k + 1
+      return ldv(D.h + v) == INF && r > 0 && atomicCAS(D.h + v, INF, k + 2) == INF;
     });
     if (rounds < 0) return;
     levels += rounds;
@@ -284,65 +332,96 @@ __global__ void __launch_bounds__(CSR_THREADS) k_csr_solve(CsrDev D, CsrParams p
     }
     // ------------------------------------------------ pulses
     for (int p = 0; p < prm.K; ++p) {
+      const int32_t* lc = L[p & 1];
+      int32_t* ln = L[(p + 1) & 1];
+      int v = slot < n ? ld_early(lc + slot) : 0;
       const int ncur = ldv(cp + p % 3);
       if (ncur == 0) break;
       if (lead) cp[(p + 2) % 3] = 0;
       ++sid;
-      const int32_t* lc = L[p & 1];
-      int32_t* ln = L[(p + 1) & 1];
       int32_t* cn = cp + (p + 1) % 3;
-      // push step: labels fixed
-      for (int i = gt; i < ncur; i += nt) {
-        const int v = lc[i];
-        int ev = __ldcg(D.e + v);
-        const int hv = __ldcg(D.h + v);
-        if (ev <= 0 || hv >= INF) continue;
+      // push step: labels fixed; the vertex's lanes split its excess among the
+      // admissible arcs by a saturating prefix sum
+      for (int i0 = wslot, i = slot; i0 < ncur; i0 += slots, i += slots) {
+        int a = 0, a1 = 0, ev = 0, hv = INF, rt = 0;
+        if (i < ncur) {
+          if (i != slot) v = __ldcg(lc + i);
+          a = __ldg(D.row + v) + sub;
+          a1 = __ldg(D.row + v + 1);
+          ev = __ldcg(D.e + v);
+          hv = __ldcg(D.h + v);
+          rt = __ldcg(D.rT + v);
+        }
+        if (ev <= 0 || hv >= INF) { ev = 0; a1 = 0; }
         const int e0 = ev;
-        const int rt = __ldcg(D.rT + v);
-        if (rt > 0 && hv == 1) {
+        if (rt > 0 && hv == 1 && ev > 0) {
           const int dl = min(ev, rt);
-          D.rT[v] = rt - dl;
           ev -= dl;
-          atomicAdd(D.flow, (unsigned long long)dl);
+          if (sub == 0) {
+            D.rT[v] = rt - dl;
+            flow += dl;
+          }
         }
-        const int a1 = D.row[v + 1];
-        for (int a = D.row[v]; a < a1 && ev > 0; ++a) {
-          const int r = __ldcg(D.res + a);
-          if (r <= 0) continue;
-          const int u = D.to[a];
-          if (__ldcg(D.h + u) != hv - 1) continue;
-          const int dl = min(ev, r);
-          D.res[a] = r - dl;  // only v writes this arc in this step
-          atomicAdd(D.res + D.rev[a], dl);
-          atomicAdd(D.e + u, dl);
-          ev -= dl;
-          if (atomicExch(D.stamp + u, sid) != sid) ln[atomicAdd(cn, 1)] = u;
+        for (; __any_sync(FULL, a < a1 && ev > 0); a += W) {
+          unsigned cap = 0;
+          int r = 0, u = 0, rv = 0;
+          if (a < a1 && ev > 0) {
+            r = __ldcg(D.res + a);
+            u = __ldg(D.to + a);
+            rv = __ldg(D.rev + a);
+            if (r > 0 && __ldcg(D.h + u) == hv - 1) cap = (unsigned)min(r, ev);
+          }
+          unsigned s = cap;
+#pragma unroll
+          for (int o = 1; o < W; o <<= 1) {
+            const unsigned x = __shfl_up_sync(FULL, s, o, W);
+            if (sub >= o) s = min(s + x, (unsigned)ev);
+          }
+          unsigned below = __shfl_up_sync(FULL, s, 1, W);
+          if (sub == 0) below = 0;
+          const int dl = (int)(s - below);
+          ev -= (int)__shfl_sync(FULL, s, W - 1, W);
+          bool fresh = false;
+          if (dl > 0) {
+            D.res[a] = r - dl;  // only v writes this arc in this step
+            atomicAdd(D.res + rv, dl);
+            atomicAdd(D.e + u, dl);
+            fresh = atomicExch(D.stamp + u, sid) != sid;
+          }
+          csr_append(fresh, u, ln, cn);
         }
-        if (ev != e0) atomicSub(D.e + v, e0 - ev);
-        if (ev > 0 && atomicExch(D.stamp + v, sid) != sid) ln[atomicAdd(cn, 1)] = v;
+        if (sub == 0 && ev != e0) atomicSub(D.e + v, e0 - ev);
+        csr_append(sub == 0 && ev > 0 && atomicExch(D.stamp + v, sid) != sid, v, ln, cn);
       }
       if (!sync()) return;
-      // relabel step: an active vertex without an admissible arc moves to one
-      // above its lowest residual neighbour
+      // relabel step: an active vertex moves to one above its lowest residual
+      // neighbour (which is its own height while it has an admissible arc);
+      // labels only grow, so concurrent relabels keep them valid
+      v = slot < n ? ld_early(ln + slot) : 0;
       const int nn = ldv(cn);
-      for (int i = gt; i < nn; i += nt) {
-        const int v = ln[i];
-        const int hv = __ldcg(D.h + v);
-        if (__ldcg(D.e + v) <= 0 || hv >= INF) continue;
-        const int rt = __ldcg(D.rT + v);
-        if (rt > 0 && hv == 1) continue;
-        int mn = rt > 0 ? 0 : INF;
-        bool adm = false;
-        const int a1 = D.row[v + 1];
-        for (int a = D.row[v]; a < a1; ++a) {
-          if (__ldcg(D.res + a) <= 0) continue;
-          const int hu = ldv(D.h + D.to[a]);
-          if (hu == hv - 1) { adm = true; break; }
-          mn = min(mn, hu);
+      for (int i0 = wslot, i = slot; i0 < nn; i0 += slots, i += slots) {
+        int a = 0, a1 = 0, hv = INF, mn = INF;
+        if (i < nn) {
+          if (i != slot) v = __ldcg(ln + i);
+          a = __ldg(D.row + v) + sub;
+          a1 = __ldg(D.row + v + 1);
+          const int ev = __ldcg(D.e + v), rt = __ldcg(D.rT + v);
+          hv = __ldcg(D.h + v);
+          if (ev <= 0 || (rt > 0 && hv == 1)) hv = INF;
+          if (rt > 0) mn = 0;
         }
-        if (!adm) {
-          int hn = mn >= INF ? INF : mn + 1;
-          if (hn >= D.hdead) hn = INF;
+        if (hv >= INF) a1 = 0;
+        for (; __any_sync(FULL, a < a1); a += W) {
+          if (a < a1) {
+            const int r = __ldcg(D.res + a);
+            const int hu = ldv(D.h + __ldg(D.to + a));
+            if (r > 0) mn = min(mn, hu);
+          }
+        }
+#pragma unroll
+        for (int o = 1; o < W; o <<= 1) mn = min(mn, __shfl_xor_sync(FULL, mn, o));
+        if (sub == 0 && hv < INF && mn >= hv) {
+          const int hn = mn >= INF || mn + 1 >= D.hdead ? INF : mn + 1;
           D.h[v] = hn;
         }
       }
@@ -359,19 +438,18 @@ __global__ void __launch_bounds__(CSR_THREADS) k_csr_solve(CsrDev D, CsrParams p
   for (int v = gt; v - lane < n; v += nt) {
     const bool seed = v < n && __ldcg(D.e + v) > 0;
     if (v < n) D.reach[v] = seed ? 1 : 0;
-    csr_append(seed, v, L[0], cb + 0);
+    csr_append(seed, seed ? arcs_of(v) : make_int2(0, 0), D.front, cb + 0);
   }
   if (!sync()) return;
-  const int rrounds = bfs([&](int u, int, int32_t* next, int32_t* cnext) {
-    const int a1 = D.row[u + 1];
-    for (int a = D.row[u]; a < a1; ++a) {
-      const int v = D.to[a];
-      if (__ldcg(D.res + a) > 0 && ldv(D.reach + v) == 0 && atomicCAS(D.reach + v, 0, 1) == 0)
-        next[atomicAdd(cnext, 1)] = v;
-    }
+  const int rrounds = bfs([&](int a, int v, int) {
+    const int r = __ldcg(D.res + a);
+    return ldv(D.reach + v) == 0 && r > 0 && atomicCAS(D.reach + v, 0, 1) == 0;
   });
   if (rrounds < 0) return;
   lap(ns_reach);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) flow += __shfl_down_sync(FULL, flow, o);
+  if (lane == 0 && flow) atomicAdd(D.flow, (unsigned long long)flow);
   if (lead) {
     D.stats[CS_PULSES] = (unsigned long long)pulses;
     D.stats[CS_RELABELS] = (unsigned long long)relabels;
@@ -403,6 +481,7 @@ struct cgc_graph {
   uint8_t* seg = nullptr;
   cgc::CsrDev d{};
   int coop_blocks = 0;
+  int lanes = 8;  // lanes per vertex in the solve
   bool tlinks = false, solved = false;
   cgc_stats st{};
 };
@@ -458,6 +537,7 @@ int graph_create(int32_t n, int64_t m, const int32_t* a, const int32_t* b, const
     const int64_t o_rc = off; off += al((int64_t)n * 4);
     const int64_t o_st = off; off += al((int64_t)n * 4);
     const int64_t o_li = off; off += al(2 * (int64_t)n * 4);
+    const int64_t o_fr = off; off += al(2 * (int64_t)n * 8);
     const int64_t o_cnt = off; off += al(CC_N * 4);
     const int64_t o_fl = off; off += al(8);
     const int64_t o_sta = off; off += al(CS_N * 8);
@@ -484,6 +564,7 @@ int graph_create(int32_t n, int64_t m, const int32_t* a, const int32_t* b, const
     d.reach = (int32_t*)(base + o_rc);
     d.stamp = (uint32_t*)(base + o_st);
     d.list = (int32_t*)(base + o_li);
+    d.front = (int2*)(base + o_fr);
     d.cnt = (int32_t*)(base + o_cnt);
     d.flow = (unsigned long long*)(base + o_fl);
     d.stats = (unsigned long long*)(base + o_sta);
@@ -520,11 +601,11 @@ int graph_create(int32_t n, int64_t m, const int32_t* a, const int32_t* b, const
     }
     cudaDeviceProp prop;
     CGC_CUDA(cudaGetDeviceProperties(&prop, g->device));
-    int occ = 0;
-    CGC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_csr_solve, CSR_THREADS, 0));
-    // enough CTAs to cover the vertices, at most the co-resident count
-    const int want = grid_blocks(n, CSR_THREADS);
-    g->coop_blocks = std::max(1, std::min(std::max(1, occ) * prop.multiProcessorCount, want));
+    // lanes per vertex: about its average number of arcs; enough CTAs to cover
+    // the vertices, at most one per SM
+    const int64_t degree = arcs / n;
+    g->lanes = degree >= 12 ? 16 : degree >= 6 ? 8 : 4;
+    g->coop_blocks = std::max(1, std::min(prop.multiProcessorCount, grid_blocks((int64_t)n * g->lanes, CSR_THREADS)));
     CGC_CUDA(cudaStreamSynchronize(g->stream));
     return CGC_OK;
   }();
@@ -572,7 +653,8 @@ int graph_maxflow(cgc_graph* g, const cgc_options* opts, int64_t* flow) {
     cfg.gridDim = dim3(g->coop_blocks);
     cfg.blockDim = dim3(CSR_THREADS);
     if (int rc2 = coop_launch_ordered(g->device, g->stream, [&]() -> int {
-          CGC_CUDA(cudaLaunchKernelEx(&cfg, k_csr_solve, d, prm));
+          CGC_CUDA(cudaLaunchKernelEx(
+              &cfg, g->lanes == 16 ? k_csr_solve<16> : g->lanes == 8 ? k_csr_solve<8> : k_csr_solve<4>, d, prm));
           return CGC_OK;
         }))
       return rc2;
