@@ -1,8 +1,8 @@
 // Device-resident batch path: many grid instances whose capacities already
 // sit in device memory are uploaded, solved and written back by a fixed
-// sequence of 4 kernels and 6 memory operations with no host synchronisation
-// -- one pointer-table upload kernel for all instances, the preflow kernel,
-// one persistent cooperative solve, one pointer-table output kernel -- which
+// sequence of 3 kernels and 4 memory operations with no host synchronisation
+// -- one pointer-table upload and preflow kernel for all instances, one
+// persistent cooperative solve, one pointer-table output kernel -- which
 // is captured once into a CUDA graph and replayed per batch.
 //
 // The reference solves one graph per Graph object with a host round trip per
@@ -22,9 +22,10 @@ namespace cgc {
 
 // Upload of every instance from its bound device inputs (8 pointers per
 // instance: capS, capT, fwd x/y/z, bwd x/y/z; a null n-link pointer is zero),
-// fused with the preflow initialisation (put_tile4, cgc_kernels.cuh).
-__global__ void __launch_bounds__(128) k_put_all(DevPool P, const int32_t* const* __restrict__ in) {
-  put_tile4(P, blockIdx.x, in + 8 * P.tinst[blockIdx.x]);
+// fused with the preflow initialisation (put_run, cgc_kernels.cuh).
+__global__ void __launch_bounds__(128, 8) k_put_all(DevPool P, const int32_t* const* __restrict__ in) {
+  const int t0 = P.runs[blockIdx.x];
+  put_run(P, t0, in + 8 * (int64_t)P.tinst[t0], true);
 }
 
 // Both cut sets of every instance into its bound device outputs (1/0 bytes),
@@ -34,18 +35,9 @@ __global__ void __launch_bounds__(128) k_put_all(DevPool P, const int32_t* const
 // (seg_gather4 / seg_store4).
 __global__ void __launch_bounds__(256) k_seg_all(DevPool P, uint8_t* const* __restrict__ out) {
   for (int inst = blockIdx.y; inst < P.ninst; inst += gridDim.y) {
-    const InstGeo G = P.geo[inst];
     uint8_t* src = out[2 * inst];
     uint8_t* snk = out[2 * inst + 1];
-    if (!src && !snk) continue;
-    const int64_t N = (int64_t)G.X * G.Y * G.Z;
-    for (int64_t v0 = 4 * ((int64_t)blockIdx.x * blockDim.x + threadIdx.x); v0 < N;
-         v0 += 4 * (int64_t)gridDim.x * blockDim.x) {
-      unsigned a = 0, b = 0;
-      seg_gather4(P, G, v0, N, snk ? &a : nullptr, src ? &b : nullptr);
-      if (src) seg_store4(src, v0, N, b, 1, 0);
-      if (snk) seg_store4(snk, v0, N, a, 1, 0);
-    }
+    if (src || snk) seg_instance(P, inst, src, snk, blockIdx.x, gridDim.x);
   }
 }
 
@@ -101,17 +93,14 @@ int pool_enqueue(Pool& p, const cgc_options* opts, int64_t* flows_dev, cudaStrea
   CGC_CUDA(cudaMemsetAsync(d.flow, 0, (size_t)p.ninst * 8, stream));
   CGC_CUDA(cudaMemsetAsync(d.stats, 0, S_NSTATS * 8, stream));
   CGC_CUDA(cudaMemsetAsync(d.bar, 0, 8, stream));  // and the error word
-  CGC_CUDA(cudaMemsetAsync(d.stamp_bfs, 0, (size_t)d.T * 4, stream));
-  CGC_CUDA(cudaMemsetAsync(d.stamp_sw, 0, 2 * (size_t)d.T * 4, stream));
-  CGC_CUDA(cudaMemsetAsync(d.stamp_inc, 0, (size_t)d.T * 4, stream));
-  k_put_all<<<d.T, 128, 0, stream>>>(d, p.d_in);
+  k_put_all<<<d.nruns, 128, 0, stream>>>(d, p.d_in);
   note_launch();
   const SolveParams prm = solve_params(o);
   if (int rc = launch_solve(d, o, prm, p.device, p.sms, stream)) return rc;
   bool any_out = false;
   for (uint8_t* q : p.out_ptrs) any_out = any_out || q;
   if (any_out) {
-    const unsigned gx = (unsigned)std::min<int64_t>(std::max<int64_t>((p.maxN + 32767) / 32768, 1), 4096);
+    const unsigned gx = (unsigned)std::min<int64_t>(std::max<int64_t>((p.maxN + 8191) / 8192, 1), 4096);
     k_seg_all<<<dim3(gx, (unsigned)std::min(p.ninst, 65535)), 256, 0, stream>>>(d, p.d_out);
     note_launch();
   }

@@ -83,6 +83,8 @@ struct DevPool {
   const int32_t* nbr;   // 6*T: neighbour tile in direction d, -1 outside
   const int32_t* tinst; // T: instance of the tile
   const uint8_t* tpar;  // T: (tx+ty+tz)&1
+  const int32_t* runs;  // first tile of each run of up to 4 tiles along x (pools of several instances)
+  int32_t nruns;        // runs
   uint8_t* act;         // T: tile holds an active voxel (e>0, h<INF)
   uint16_t* tflag;      // T: BFS seed summary (TF_* bits)
   uint32_t* stamp_bfs;  // T: last BFS round the tile was queued for
@@ -126,14 +128,12 @@ struct SolveParams {
 };
 
 // kernels of cgc_engine.cu launched from other translation units
-__global__ void k_put_tlinks(DevPool P, int inst, const int32_t* __restrict__ capS, const int32_t* __restrict__ capT);
-__global__ void k_put_nlinks(DevPool P, int inst, int axis, const int32_t* __restrict__ fwd,
-                             const int32_t* __restrict__ bwd);
-__global__ void k_prepare(DevPool P);
+struct InputPlanes { const int32_t* p[8]; };  // capS, capT, fwd x/y/z, bwd x/y/z (null = zero)
+__global__ void k_put_one(DevPool P, InputPlanes in, bool two_halves);
+__global__ void k_seg_one(DevPool P, uint8_t* src, uint8_t* snk);
 __global__ void k_solve4(DevPool P, SolveParams prm);
 __global__ void k_solve5(DevPool P, SolveParams prm);
 __global__ void k_solve8(DevPool P, SolveParams prm);
-__global__ void k_segments(DevPool P, int inst, int which, uint8_t* out, uint8_t mask, uint8_t bg);
 // kernels of cgc_batch.cu
 __global__ void k_put_all(DevPool P, const int32_t* const* __restrict__ in);
 __global__ void k_seg_all(DevPool P, uint8_t* const* __restrict__ out);

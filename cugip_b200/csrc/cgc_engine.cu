@@ -50,113 +50,15 @@ int ok() {
 // kernels
 // ===========================================================================
 
-// Copies the linear (x-fastest) t-link arrays of one instance into the
-// blocked e (= capS for now) and rT (= capT) planes.
-__global__ void __launch_bounds__(512) k_put_tlinks(DevPool P, int inst, const int32_t* __restrict__ capS,
-                                                    const int32_t* __restrict__ capT) {
-  const InstGeo G = P.geo[inst];
-  const int lt = blockIdx.x;
-  const int tx = lt % G.TX, ty = (lt / G.TX) % G.TY, tz = lt / (G.TX * G.TY);
-  const int l = threadIdx.x;
-  const int x = tx * 8 + (l & 7), y = ty * 8 + ((l >> 3) & 7), z = tz * 8 + (l >> 6);
-  const int64_t g = (int64_t)(G.tile_base + lt) * TV + l;
-  int s = 0, c = 0;
-  if (x < G.X && y < G.Y && z < G.Z) {
-    const int64_t v = x + (int64_t)G.X * (y + (int64_t)G.Y * z);
-    s = capS[v]; c = capT[v];
-    if (s < 0 || c < 0) raise_error(P, CGC_ERR_ARG);
-  }
-  P.e[g] = s;
-  P.rT[g] = c;
+// Fused upload + preflow of a single instance whose 8 input planes are passed
+// by value, so a queued solve reads exactly the planes of its own set_* calls
+// (put_run).
+__global__ void __launch_bounds__(128, 8) k_put_one(DevPool P, InputPlanes in, bool two_halves) {
+  const int TX = P.geo[0].TX, rx = (TX + 3) / 4, row = blockIdx.x / rx;
+  put_run(P, row * TX + 4 * (blockIdx.x - row * rx), in.p, two_halves);
 }
-
-// Copies the n-links of one axis: r[+a][v] = fwd[v], r[-a][v+e_a] = bwd[v].
-__global__ void __launch_bounds__(512) k_put_nlinks(DevPool P, int inst, int axis, const int32_t* __restrict__ fwd,
-                                                    const int32_t* __restrict__ bwd) {
-  const InstGeo G = P.geo[inst];
-  const int lt = blockIdx.x;
-  const int tx = lt % G.TX, ty = (lt / G.TX) % G.TY, tz = lt / (G.TX * G.TY);
-  const int l = threadIdx.x;
-  const int x = tx * 8 + (l & 7), y = ty * 8 + ((l >> 3) & 7), z = tz * 8 + (l >> 6);
-  const int64_t g = (int64_t)(G.tile_base + lt) * TV + l;
-  int f = 0, b = 0;
-  if (x < G.X && y < G.Y && z < G.Z) {
-    const int c = axis == 0 ? x : axis == 1 ? y : z;
-    const int ext = axis == 0 ? G.X : axis == 1 ? G.Y : G.Z;
-    const int64_t stride = axis == 0 ? 1 : axis == 1 ? (int64_t)G.X : (int64_t)G.X * G.Y;
-    const int64_t v = x + (int64_t)G.X * (y + (int64_t)G.Y * z);
-    if (fwd && c + 1 < ext) f = fwd[v];
-    if (bwd && c > 0) b = bwd[v - stride];
-    if (f < 0 || b < 0) raise_error(P, CGC_ERR_ARG);
-  }
-  P.r[(2 * axis) * P.Np + g] = f;
-  P.r[(2 * axis + 1) * P.Np + g] = b;
-}
-
-// Preflow initialisation (replaces initResidualsKernel and
-// pushThroughTLinksFromSourceKernel, graph_cut_implementation.hpp:28-40,
-// graph_cut_push.hpp:11-24): the t-links of a voxel cancel,
-// m = min(capS, capT) goes straight from the source to the sink, the rest of
-// capS becomes excess.  Also checks that no excess or residual can exceed
-// int32 and builds the residual bit mask.  The kernel is bound by load
-// latency: the face neighbours are read first (the same six values for the
-// whole tile), then all fourteen per-voxel loads are issued at once, with the
-// index of a missing neighbour clamped to the voxel itself and the value
-// masked afterwards.
-__global__ void __launch_bounds__(512) k_prepare(DevPool P) {
-  __shared__ long long red[16];
-  const int t = blockIdx.x;
-  const int l = threadIdx.x;
-  const int x = l & 7, y = (l >> 3) & 7, z = l >> 6;
-  const int64_t g = (int64_t)t * TV + l;
-  const int64_t Np = P.Np;
-  int nbt[6];
-#pragma unroll
-  for (int d = 0; d < 6; ++d) nbt[d] = __ldg(P.nbr + d * P.T + t);
-  const int s = P.e[g], c = P.rT[g];
-  int rv[6], bk[6];
-  bool has[6];
-#pragma unroll
-  for (int d = 0; d < 6; ++d) {
-    const bool in = inside(d, x, y, z);
-    has[d] = in || nbt[d] >= 0;
-    const int64_t ng = in ? g + loff(d) : (has[d] ? (int64_t)nbt[d] * TV + l + xoff(d) : g);
-    rv[d] = P.r[d * Np + g];
-    bk[d] = P.r[(d ^ 1) * Np + ng];
-  }
-  const int mcap = min(s, c);
-  const int e = s - mcap, rT = c - mcap;
-  long long inflow = e;
-  unsigned m = (rT > 0 ? 64u : 0u) | (e > 0 ? 128u : 0u);
-  bool bad = false;
-#pragma unroll
-  for (int d = 0; d < 6; ++d) {
-    const long long back = has[d] ? (long long)bk[d] : 0ll;
-    if (!has[d] && rv[d] != 0) bad = true;  // capacity towards the outside of the grid
-    inflow += back;
-    if ((long long)rv[d] + back > 2147483647ll) bad = true;
-    m |= (rv[d] > 0 ? 1u : 0u) << d;
-  }
-  if (inflow > 2147483647ll) bad = true;
-  if (bad) raise_error(P, CGC_ERR_OVERFLOW);
-  P.e[g] = e;
-  P.rT[g] = rT;
-  P.h[g] = 0;  // no label yet (INF would read as "dead" to the first global relabel)
-  P.rmask[g] = (uint8_t)m;
-  P.reach[g] = 0;
-  const long long tot = block_sum64((long long)mcap, red);
-  if (l == 0) {
-    P.act[t] = 0;
-    if (tot) atomicAdd(P.flow + P.tinst[t], (unsigned long long)tot);
-  }
-}
-
-// Fused upload + preflow of a single instance whose 8 input planes (capS,
-// capT, fwd x/y/z, bwd x/y/z; null = zero) are passed by value, so a queued
-// solve reads exactly the planes of its own set_* calls (put_tile4).
-struct InputPlanes { const int32_t* p[8]; };
-__global__ void __launch_bounds__(128) k_put_one(DevPool P, InputPlanes in) {
-  put_tile4(P, blockIdx.x, in.p);
+__global__ void __launch_bounds__(256) k_seg_one(DevPool P, uint8_t* src, uint8_t* snk) {
+  seg_instance(P, 0, src, snk, blockIdx.x, gridDim.x);
 }
 
 // Cut sets as mask / background bytes from the 1/0 bytes of one buffer
@@ -209,9 +111,9 @@ __global__ void k_compact(DevPool P, int parity, int32_t* list, int32_t* cnt) {
   warp_append(P, pred, t, list, cnt);
 }
 
-__global__ void __launch_bounds__(512) k_bfs_init(DevPool P) {
+__global__ void __launch_bounds__(512) k_bfs_init(DevPool P, bool fresh) {
   const int nw = gridDim.x * (blockDim.x >> 5);
-  for (int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < P.T; t += nw) bfs_init_tile_w(P, t);
+  for (int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < P.T; t += nw) bfs_init_tile_w(P, t, fresh);
 }
 
 __global__ void k_bfs_queue(DevPool P, uint32_t id0, int32_t* list0, int32_t* cnt0) {
@@ -427,7 +329,7 @@ __device__ __forceinline__ void solve_body(const DevPool& P, const SolveParams& 
     round_no = 0;
     if (!sync()) return;
     if (!inc) {
-      for (int t = gw; t < P.T; t += nw) bfs_init_tile_w(P, t);  // a warp per tile
+      for (int t = gw; t < P.T; t += nw) bfs_init_tile_w(P, t, relabels == 0);  // a warp per tile
       if (!sync()) return;
       for (int t0 = b * blockDim.x; t0 < P.T; t0 += G * blockDim.x) bfs_queue_tile(P, t0 + tid, bfs_id, list(0), bc + 0);
       if (!sync()) return;
@@ -680,23 +582,8 @@ __global__ void __launch_bounds__(8 * GROUP, 1) k_solve8(DevPool P, SolveParams 
   solve_body(P, prm, reinterpret_cast<TileShared*>(solve_smem));
 }
 
-// Output kernels (linear layout of one instance).  k_segments, a thread per
-// voxel, serves the allocation-free entry point; grids and batches use
-// k_segments_lin / k_seg_all (four voxels per thread).
-__global__ void k_segments(DevPool P, int inst, int which, uint8_t* out, uint8_t mask, uint8_t bg) {
-  const InstGeo G = P.geo[inst];
-  const int64_t N = (int64_t)G.X * G.Y * G.Z;
-  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < N; v += (int64_t)gridDim.x * blockDim.x) {
-    const int x = (int)(v % G.X), y = (int)((v / G.X) % G.Y), z = (int)(v / ((int64_t)G.X * G.Y));
-    const int64_t t = G.tile_base + (x >> 3) + G.TX * ((y >> 3) + G.TY * (z >> 3));
-    const int64_t g = t * TV + (x & 7) + 8 * (y & 7) + 64 * (z & 7);
-    const bool in = which == CGC_SEG_SINK_REACH ? (P.h[g] < INF) : (P.reach[g] != 0);
-    out[v] = in ? mask : bg;
-  }
-}
-
-// The same in linear voxel order, four voxels per thread (seg_gather4 /
-// seg_store4).
+// One cut set of an instance after a device-resident solve, any mask and
+// background (linear layout).
 __global__ void __launch_bounds__(256) k_segments_lin(DevPool P, int inst, int which, uint8_t* out, uint8_t mask,
                                                       uint8_t bg) {
   const InstGeo G = P.geo[inst];
@@ -787,6 +674,7 @@ int pool_create(int32_t count, const int32_t* ext, void* stream, Pool** out) {
   const int64_t o_nbr = off; off += al(6 * T * 4);
   const int64_t o_ti = off; off += al(T * 4);
   const int64_t o_tp = off; off += al(T);
+  const int64_t o_run = off; off += al(T * 4);
   const int64_t o_act = off; off += al(T);
   const int64_t o_tf = off; off += al(T * 2);
   const int64_t o_sb = off; off += al(T * 4);
@@ -814,8 +702,10 @@ int pool_create(int32_t count, const int32_t* ext, void* stream, Pool** out) {
   d.stats = (unsigned long long*)(base + o_st); d.bar = (uint32_t*)(base + o_bar); d.err = (int32_t*)(d.bar + 1);
   d.trace = (unsigned long long*)(base + o_tr);
 
+  d.runs = (int32_t*)(base + o_run);
+
   // tile tables
-  std::vector<int32_t> nbr(6 * (size_t)T, -1), ti((size_t)T);
+  std::vector<int32_t> nbr(6 * (size_t)T, -1), ti((size_t)T), runs;
   std::vector<uint8_t> tp((size_t)T);
   for (int i = 0; i < count; ++i) {
     const InstGeo& G = p->geo[i];
@@ -824,6 +714,7 @@ int pool_create(int32_t count, const int32_t* ext, void* stream, Pool** out) {
         for (int tx = 0; tx < G.TX; ++tx) {
           const int64_t t = G.tile_base + tx + (int64_t)G.TX * (ty + (int64_t)G.TY * tz);
           ti[t] = i;
+          if (tx % 4 == 0) runs.push_back((int32_t)t);
           tp[t] = (uint8_t)((tx + ty + tz) & 1);
           auto id = [&](int a, int b2, int c) -> int32_t {
             if (a < 0 || b2 < 0 || c < 0 || a >= G.TX || b2 >= G.TY || c >= G.TZ) return -1;
@@ -835,6 +726,8 @@ int pool_create(int32_t count, const int32_t* ext, void* stream, Pool** out) {
         }
   }
   CGC_CUDA(cudaMemcpyAsync((void*)d.nbr, nbr.data(), nbr.size() * 4, cudaMemcpyHostToDevice, p->stream));
+  d.nruns = (int32_t)runs.size();
+  CGC_CUDA(cudaMemcpyAsync((void*)d.runs, runs.data(), runs.size() * 4, cudaMemcpyHostToDevice, p->stream));
   CGC_CUDA(cudaMemcpyAsync((void*)d.tinst, ti.data(), ti.size() * 4, cudaMemcpyHostToDevice, p->stream));
   CGC_CUDA(cudaMemcpyAsync((void*)d.tpar, tp.data(), tp.size(), cudaMemcpyHostToDevice, p->stream));
   CGC_CUDA(cudaMemcpyAsync((void*)d.geo, p->geo.data(), p->geo.size() * sizeof(InstGeo), cudaMemcpyHostToDevice, p->stream));
@@ -983,7 +876,7 @@ static int host_bfs(Pool& p, uint32_t& id, int64_t& rounds) {
   const int gi = std::min<int>(d.T, p.sms * 8);
   if (REACH) { k_reach_init<<<gi, 512, 0, p.stream>>>(d, id, bl[0], d.cnt + C_BFS0); note_launch(); }
   else {
-    k_bfs_init<<<gi, 512, 0, p.stream>>>(d); note_launch();
+    k_bfs_init<<<gi, 512, 0, p.stream>>>(d, rounds == 0); note_launch();
     k_bfs_queue<<<(d.T + 255) / 256, 256, 0, p.stream>>>(d, id, bl[0], d.cnt + C_BFS0); note_launch();
   }
   CGC_CUDA(cudaGetLastError());
@@ -1047,15 +940,12 @@ int pool_solve_async(Pool& p, const cgc_options* opts) {
   CGC_CUDA(cudaMemsetAsync(d.flow, 0, (size_t)p.ninst * 8, p.stream));
   CGC_CUDA(cudaMemsetAsync(d.stats, 0, S_NSTATS * 8, p.stream));
   CGC_CUDA(cudaMemsetAsync(d.bar, 0, 8, p.stream));  // and the error word
-  CGC_CUDA(cudaMemsetAsync(d.stamp_bfs, 0, (size_t)d.T * 4, p.stream));
-  CGC_CUDA(cudaMemsetAsync(d.stamp_sw, 0, 2 * (size_t)d.T * 4, p.stream));
-  CGC_CUDA(cudaMemsetAsync(d.stamp_inc, 0, (size_t)d.T * 4, p.stream));
   if (p.ninst == 1) {
     InputPlanes ip;
     for (int k = 0; k < 8; ++k) ip.p[k] = in[k];
-    k_put_one<<<d.T, 128, 0, p.stream>>>(d, ip);
+    k_put_one<<<d.nruns, 128, 0, p.stream>>>(d, ip, true);
   } else {
-    k_put_all<<<d.T, 128, 0, p.stream>>>(d, p.d_host_in);
+    k_put_all<<<d.nruns, 128, 0, p.stream>>>(d, p.d_host_in);
   }
   note_launch();
   CGC_CUDA(cudaGetLastError());
@@ -1109,7 +999,7 @@ int pool_solve_async(Pool& p, const cgc_options* opts) {
     p.host_counts[2] = rounds;
   }
   if (!rc) {
-    const unsigned gx = (unsigned)std::min<int64_t>(std::max<int64_t>((p.maxN + 32767) / 32768, 1), 4096);
+    const unsigned gx = (unsigned)std::min<int64_t>(std::max<int64_t>((p.maxN + 8191) / 8192, 1), 4096);
     k_seg_all<<<dim3(gx, (unsigned)std::min(p.ninst, 65535)), 256, 0, p.stream>>>(d, p.d_segtab);
     note_launch();
     CGC_CUDA(cudaGetLastError());

@@ -847,71 +847,57 @@ __device__ __forceinline__ int sweep_tile_wide(const DevPool& P, const TileGroup
   return pulses;
 }
 
-// Upload of tile t of an instance from its linear (x-fastest) device inputs
-// ip[0..7] = capS, capT, fwd x/y/z, bwd x/y/z (a null n-link pointer is
-// zero), fused with the preflow initialisation: the t-links cancel
-// (m = min(capS, capT) goes straight to the sink, the rest of capS becomes
-// excess), the residual planes and the residual bit mask are written, and
-// capacities that could overflow int32 excess or residuals raise
+// Upload of a run of up to four tiles along x of an instance, from its linear
+// (x-fastest) device inputs ip[0..7] = capS, capT, fwd x/y/z, bwd x/y/z (a null
+// n-link pointer is zero), fused with the preflow initialisation: the t-links
+// cancel (m = min(capS, capT) goes straight to the sink, the rest of capS
+// becomes excess), the residual planes and the residual bit mask are written,
+// and capacities that could overflow int32 excess or residuals raise
 // CGC_ERR_OVERFLOW.  Every value that needs (the capacity into the voxel from
 // each neighbour: bwd[v] from +a, fwd[v - stride] from -a) is an input this
-// thread reads anyway, so the solve starts after one pass over the planes.
+// CTA reads anyway, so the solve starts after one pass over the planes.
+// Heights and reachability are not touched: the first relabel and the final
+// seeding pass write them everywhere.
 // Replaces initResidualsKernel and pushThroughTLinksFromSourceKernel
 // (detail/graph_cut_implementation.hpp:28-40, detail/graph_cut_push.hpp:11-24).
 //
-// One CTA of 128 threads per tile; thread q owns the four voxels 4q..4q+3 of
-// the tile (four consecutive x of one row).  The kernel is bound by load
-// latency, so every load of a thread is issued unconditionally and at once:
-// indices outside the instance are clamped to a valid voxel and missing
-// planes read capS, and the values are masked afterwards.  The outputs are
-// 16-byte stores into the tile-blocked planes.
-__device__ __forceinline__ void put_tile4(const DevPool& P, const int t, const int32_t* const* ip) {
+// 128 threads: thread (xq, y, zh) walks four z planes, four voxels (half a
+// tile row) in each.  Loads in flight bound it, so the step is kept short and
+// small in registers; the run makes every access whole 128-byte lines (a warp
+// reads four rows of 32 voxels and writes four rows of each of the four tiles,
+// which are contiguous there); the neighbour values come from registers (z),
+// the next lane (x) or the L1 (y).
+//   A4: plane rows of four voxels are 16-byte aligned (aligned planes, X a
+//   multiple of 4); otherwise a row is the two aligned vectors that cover it,
+//   or scalars.  SAME: symmetric n-links, one plane per axis.
+//   two_halves: the pool keeps both halves of stamp_sw.
+// 512x512x128: 0.75 -> 0.29 ms, 6.3 TB/s (before: a CTA per tile, eight planes read, 64-bit
+// checks per voxel); 405x377x362, whose rows are not aligned, with both masks: 2.0 -> 1.1 ms.
+template <bool A4, bool SAME>
+__device__ __forceinline__ void put_run_as(const DevPool& P, const int t0, const int32_t* const* ip, const InstGeo& G,
+                                           const int inst, const bool vec, const bool two_halves) {
   __shared__ long long red[4];
-  if (!CGC_IN_BOUNDS(P, t, P.T)) return;  // uniform over the block
-  const int inst = P.tinst[t];
-  const InstGeo G = P.geo[inst];
-  const int lt = t - G.tile_base;
-  const int tx = lt % G.TX, ty = (lt / G.TX) % G.TY, tz = lt / (G.TX * G.TY);
-  const int q = threadIdx.x, l0 = 4 * q;
-  const int x0 = tx * 8 + (l0 & 7), y = ty * 8 + ((l0 >> 3) & 7), z = tz * 8 + (l0 >> 6);
-  const int64_t g0 = (int64_t)t * TV + l0;
-  const int32_t* cs = ip[0];
-  const int32_t* ct = ip[1];
-  const int32_t* fp[3];
-  const int32_t* bp[3];
-  bool hasf[3], hasb[3];
+  const int lt = t0 - G.tile_base;
+  const int rows = lt / G.TX, tx0 = lt - rows * G.TX, tz = rows / G.TY, ty = rows - tz * G.TY;
+  const int q = threadIdx.x, xq = q & 7, yl = (q >> 3) & 7, zh = q >> 6;
+  const bool tile = tx0 + (xq >> 1) < G.TX;
+  const int x0 = tx0 * 8 + 4 * xq, y = ty * 8 + yl;
+  const int64_t N = (int64_t)G.X * G.Y * G.Z, sy = G.X, sz = (int64_t)G.X * G.Y;
+  // the run lies inside the instance with a voxel to spare on every side
+  const bool inner = tx0 > 0 && ty > 0 && tz > 0 && tx0 * 8 + 32 < G.X && ty * 8 + 8 < G.Y && tz * 8 + 8 < G.Z;
+  // o = p[v .. v+3] (0 <= v < N; entries past the plane's end repeat one
+  // inside); a null plane reads as zero
+  auto row4 = [&](int (&o)[4], const int32_t* p, int64_t v) {
+    if (!p) {
 #pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    fp[a] = ip[2 + a]; bp[a] = ip[5 + a];
-    hasf[a] = fp[a] != nullptr; hasb[a] = bp[a] != nullptr;
-    if (!hasf[a]) fp[a] = cs;  // read something valid, then mask
-    if (!hasb[a]) bp[a] = cs;
-  }
-  // vrow: the thread's first voxel, or voxel 0 when that lies outside the instance
-  const bool row = y < G.Y && z < G.Z && x0 < G.X;
-  const int64_t vrow = row ? x0 + (int64_t)G.X * (y + (int64_t)G.Y * z) : 0;
-  const int ex[3] = {G.X, G.Y, G.Z};
-  const int64_t st[3] = {1, (int64_t)G.X, (int64_t)G.X * G.Y};
-  const int co[3] = {0, y, z};  // x is per voxel
-  // loads (all independent).  With 16-byte aligned planes (the choice is
-  // uniform over the block: one instance per tile), each plane row of the
-  // thread's four voxels v..v+3 is read as the one or two aligned int4 that
-  // cover it (load_row4); a row that would reach past the plane's end falls
-  // back to scalar loads.  Otherwise one scalar load per voxel and plane.
-  int s[4], c[4], fv[3][4], bv[3][4], fm[3][4], bm[3][4];
-  bool ok[4];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) ok[k] = row && x0 + k < G.X;
-  uintptr_t align = reinterpret_cast<uintptr_t>(cs) | reinterpret_cast<uintptr_t>(ct);
-#pragma unroll
-  for (int a = 0; a < 3; ++a) align |= reinterpret_cast<uintptr_t>(fp[a]) | reinterpret_cast<uintptr_t>(bp[a]);
-  const int64_t N = (int64_t)G.X * G.Y * G.Z;
-  if ((align & 15) == 0) {
-    // p[v .. v+3] from aligned int4 loads (p 16-byte aligned, 0 <= v < N)
-    auto load_row4 = [N](int (&o)[4], const int32_t* p, int64_t v) {
+      for (int k = 0; k < 4; ++k) o[k] = 0;
+    } else if (A4) {
+      const int4 w = __ldg(reinterpret_cast<const int4*>(p + v));
+      o[0] = w.x; o[1] = w.y; o[2] = w.z; o[3] = w.w;
+    } else {
       const int m = (int)(v & 3);
       const int64_t a = v - m;
-      if (a + (m ? 8 : 4) <= N) {
+      if (vec && a + (m ? 8 : 4) <= N) {
         const int4 A = __ldg(reinterpret_cast<const int4*>(p + a));
         const int4 B = m ? __ldg(reinterpret_cast<const int4*>(p + a + 4)) : A;
         const int w[8] = {A.x, A.y, A.z, A.w, B.x, B.y, B.z, B.w};
@@ -921,115 +907,185 @@ __device__ __forceinline__ void put_tile4(const DevPool& P, const int t, const i
 #pragma unroll
         for (int k = 0; k < 4; ++k) o[k] = p[v + k < N ? v + k : v];
       }
-    };
-    load_row4(s, cs, vrow);
-    load_row4(c, ct, vrow);
+    }
+  };
+  bool neg = false, bad = false;
+  long long tot = 0;
+  int fzm[4], bzm[4];  // fwd / bwd z of the plane below
+#pragma unroll 1
+  for (int i = 0; i < 4; ++i) {
+    const int zl = 4 * zh + i, z = tz * 8 + zl;
+    const bool row = inner || (y < G.Y && z < G.Z && x0 < G.X);
+    const int64_t v = row ? x0 + sy * y + sz * z : 0;
+    const int64_t vy = row && y > 0 ? v - sy : v;
+    const bool left = xq == 0 && row && x0 > 0;
+    // r[2a]: to +a (fwd), r[2a+1]: to -a (bwd of the neighbour); bk: the
+    // capacities back (symmetric n-links: the same numbers)
+    int s[4], c[4], r[6][4], bk[6][4];
+    row4(s, ip[0], v);
+    row4(c, ip[1], v);
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      load_row4(fv[a], fp[a], vrow);
-      load_row4(bv[a], bp[a], vrow);
+      row4(r[2 * a], ip[2 + a], v);
+      if (!SAME) row4(bk[2 * a], ip[5 + a], v);
     }
-    const int64_t vx = row && x0 > 0 ? vrow - 1 : vrow;  // -x neighbour of the first voxel
-    fm[0][0] = __ldg(fp[0] + vx);
-    bm[0][0] = __ldg(bp[0] + vx);
-#pragma unroll
-    for (int k = 1; k < 4; ++k) { fm[0][k] = fv[0][k - 1]; bm[0][k] = bv[0][k - 1]; }
-#pragma unroll
-    for (int a = 1; a < 3; ++a) {
-      const int64_t vm = row && co[a] > 0 ? vrow - st[a] : vrow;
-      load_row4(fm[a], fp[a], vm);
-      load_row4(bm[a], bp[a], vm);
+    int fx = left && ip[2] ? __ldg(ip[2] + v - 1) : 0, bx = 0;
+    row4(SAME ? r[3] : bk[3], ip[3], vy);
+    if (!SAME) {
+      row4(r[3], ip[6], vy);
+      if (left && ip[5]) bx = __ldg(ip[5] + v - 1);
     }
-  } else {
+    if (i == 0) {
+      const int64_t vz = row && z > 0 ? v - sz : v;
+      row4(fzm, ip[4], vz);
+      if (!SAME) row4(bzm, ip[7], vz);
+    }
+    const int fl = __shfl_up_sync(FULL, r[0][3], 1);
+    if (xq > 0) fx = fl;
+    if (!SAME) {
+      const int bl = __shfl_up_sync(FULL, bk[0][3], 1);
+      if (xq > 0) bx = bl;
+    }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const int64_t v = ok[k] ? vrow + k : vrow;
-      s[k] = cs[v];
-      c[k] = ct[v];
-#pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        const int cc = a == 0 ? x0 + k : co[a];
-        const int64_t vm = cc > 0 && ok[k] ? v - st[a] : v;
-        fv[a][k] = fp[a][v];
-        bv[a][k] = bp[a][v];
-        fm[a][k] = fp[a][vm];
-        bm[a][k] = bp[a][vm];
+      (SAME ? r[1] : bk[1])[k] = k > 0 ? r[0][k > 0 ? k - 1 : 0] : fx;
+      (SAME ? r[5] : bk[5])[k] = fzm[k];
+      fzm[k] = r[4][k];
+      if (!SAME) {
+        r[1][k] = k > 0 ? bk[0][k > 0 ? k - 1 : 0] : bx;
+        r[5][k] = bzm[k];
+        bzm[k] = bk[4][k];
       }
     }
-  }
-  int r[6][4];
-  long long inflow[4];
-  bool neg = false, bad = false;
+    if (!inner) {  // nothing outside the instance, no link across its faces
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    inflow[k] = 0;
-    if (!ok[k]) { s[k] = 0; c[k] = 0; }
+      for (int k = 0; k < 4; ++k) {
+        const int x = x0 + k;
+        const bool ok = row && x < G.X;
+        const bool has[6] = {ok && x + 1 < G.X, ok && x > 0, ok && y + 1 < G.Y, ok && y > 0, ok && z + 1 < G.Z, ok && z > 0};
+        if (!ok) s[k] = c[k] = 0;
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      const int cc = a == 0 ? x0 + k : co[a];
-      const bool up = ok[k] && cc + 1 < ex[a], dn = ok[k] && cc > 0;
-      r[2 * a][k] = up && hasf[a] ? fv[a][k] : 0;        // v -> v + e_a
-      const int back_p = up && hasb[a] ? bv[a][k] : 0;   // v + e_a -> v
-      r[2 * a + 1][k] = dn && hasb[a] ? bm[a][k] : 0;    // v -> v - e_a
-      const int back_m = dn && hasf[a] ? fm[a][k] : 0;   // v - e_a -> v
-      inflow[k] += (long long)back_p + back_m;
-      bad = bad || (long long)r[2 * a][k] + back_p > 2147483647ll || (long long)r[2 * a + 1][k] + back_m > 2147483647ll;
+        for (int d = 0; d < 6; ++d) {
+          if (!has[d]) r[d][k] = 0;
+          if (!SAME && !has[d]) bk[d][k] = 0;
+        }
+      }
     }
-    neg = neg || s[k] < 0 || c[k] < 0;
+    // Checks.  Values below 2^28 are not negative and cannot overflow: a voxel
+    // sums seven of them, a link two.
+    unsigned any = 0;
 #pragma unroll
-    for (int d = 0; d < 6; ++d) neg = neg || r[d][k] < 0;
+    for (int k = 0; k < 4; ++k) {
+      any |= (unsigned)(s[k] | c[k]);
+#pragma unroll
+      for (int d = 0; d < 6; ++d) any |= (unsigned)(SAME ? r[d][k] : r[d][k] | bk[d][k]);
+    }
+    if (any >> 28) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        neg = neg || s[k] < 0 || c[k] < 0;
+        long long inflow = (long long)s[k] - min(s[k], c[k]);
+#pragma unroll
+        for (int d = 0; d < 6; ++d) {
+          const long long back = SAME ? r[d][k] : bk[d][k];
+          neg = neg || r[d][k] < 0;
+          inflow += back;
+          bad = bad || (long long)r[d][k] + back > 2147483647ll;
+        }
+        bad = bad || inflow > 2147483647ll;
+      }
+    }
+    // t-link cancellation: min(capS, capT) flows straight through
+    unsigned m4 = 0;
+    int through = 0;  // below 2^30 where no value reaches 2^28
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int mcap = min(s[k], c[k]);
+      s[k] -= mcap;
+      c[k] -= mcap;
+      if (any >> 28) tot += mcap; else through += mcap;
+#pragma unroll
+      for (int d = 0; d < 6; ++d) m4 |= (r[d][k] > 0 ? 1u : 0u) << (8 * k + d);
+      m4 |= (c[k] > 0 ? 64u : 0u) << (8 * k) | (s[k] > 0 ? 128u : 0u) << (8 * k);
+    }
+    tot += through;
+    if (tile) {
+      const int64_t g = (int64_t)(t0 + (xq >> 1)) * TV + 64 * zl + 8 * yl + 4 * (xq & 1);
+      st4(P.e + g, s);
+      st4(P.rT + g, c);
+#pragma unroll
+      for (int d = 0; d < 6; ++d) st4(P.r + d * P.Np + g, r[d]);
+      *reinterpret_cast<uint32_t*>(P.rmask + g) = m4;
+    }
   }
   if (neg) raise_error(P, CGC_ERR_ARG);
-  // t-link cancellation: min(capS, capT) flows straight through
-  int e[4], rT[4];
-  unsigned m4 = 0;
-  long long tot = 0;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int mcap = min(s[k], c[k]);
-    e[k] = s[k] - mcap;
-    rT[k] = c[k] - mcap;
-    tot += mcap;
-    unsigned m = (rT[k] > 0 ? 64u : 0u) | (e[k] > 0 ? 128u : 0u);
-#pragma unroll
-    for (int d = 0; d < 6; ++d) m |= (r[d][k] > 0 ? 1u : 0u) << d;
-    m4 |= m << (8 * k);
-    bad = bad || inflow[k] + e[k] > 2147483647ll;
-  }
   if (bad) raise_error(P, CGC_ERR_OVERFLOW);
-  *reinterpret_cast<int4*>(P.e + g0) = make_int4(e[0], e[1], e[2], e[3]);
-  *reinterpret_cast<int4*>(P.rT + g0) = make_int4(rT[0], rT[1], rT[2], rT[3]);
+  if (tile && (q & ~6) == 0) {  // one thread per tile
+    const int t = t0 + (xq >> 1);
+    P.act[t] = 0;
+    P.stamp_bfs[t] = P.stamp_sw[t] = P.stamp_inc[t] = 0u;
+    if (two_halves) P.stamp_sw[P.T + t] = 0u;
+  }
 #pragma unroll
-  for (int d = 0; d < 6; ++d)
-    *reinterpret_cast<int4*>(P.r + d * P.Np + g0) = make_int4(r[d][0], r[d][1], r[d][2], r[d][3]);
-  // no label yet (INF would read as "dead" to the first global relabel)
-  *reinterpret_cast<int4*>(P.h + g0) = make_int4(0, 0, 0, 0);
-  *reinterpret_cast<uint32_t*>(P.rmask + g0) = m4;
-  *reinterpret_cast<uint32_t*>(P.reach + g0) = 0u;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) tot += __shfl_down_sync(0xffffffffu, tot, o);
+  for (int o = 16; o > 0; o >>= 1) tot += __shfl_down_sync(FULL, tot, o);
   if ((q & 31) == 0) red[q >> 5] = tot;
   __syncthreads();
   if (q == 0) {
     const long long sum = red[0] + red[1] + red[2] + red[3];
-    P.act[t] = 0;
     if (sum) atomicAdd(P.flow + inst, (unsigned long long)sum);
   }
 }
 
+__device__ __forceinline__ void put_run(const DevPool& P, const int t0, const int32_t* const* ip, const bool two_halves) {
+  if (!CGC_IN_BOUNDS(P, t0, P.T)) return;  // uniform over the block, as is all below
+  const int inst = P.tinst[t0];
+  const InstGeo G = P.geo[inst];
+  uintptr_t align = 0;
+  bool same = true;
+#pragma unroll
+  for (int a = 0; a < 8; ++a) align |= reinterpret_cast<uintptr_t>(ip[a]);
+#pragma unroll
+  for (int a = 0; a < 3; ++a) same = same && ip[2 + a] == ip[5 + a];
+  const bool vec = (align & 15) == 0, a4 = vec && (G.X & 3) == 0;
+  if (a4 && same) put_run_as<true, true>(P, t0, ip, G, inst, vec, two_halves);
+  else if (a4) put_run_as<true, false>(P, t0, ip, G, inst, vec, two_halves);
+  else if (same) put_run_as<false, true>(P, t0, ip, G, inst, vec, two_halves);
+  else put_run_as<false, false>(P, t0, ip, G, inst, vec, two_halves);
+}
+
 // ---------------------------------------------------------------------------
 // Cut sets in linear voxel order, four voxels per thread: voxels v0..v0+3 of
-// an instance (v0 a multiple of 4) are gathered from the tile layout (one
-// 64-bit division per four voxels, all loads issued at once from clamped
-// indices), and the four output bytes go out as one 32-bit store when the
-// destination is aligned, so a warp writes whole 128-byte lines.
+// an instance (v0 a multiple of 4), one 32-bit store per output when the
+// destination is aligned, so a warp writes whole 128-byte lines.  Where X is a
+// multiple of 4 they are half a tile row, read with one 16-byte and one 4-byte
+// load; else each is gathered (all loads issued at once from clamped indices).
 // Bit 0 of each byte of *sink: height < INF; of *source: in the minimal
 // source set.
 __device__ __forceinline__ void seg_gather4(const DevPool& P, const InstGeo& G, int64_t v0, int64_t N,
                                             unsigned* sink, unsigned* source) {
-  int64_t rest = v0 / G.X;
-  int x = (int)(v0 - rest * G.X);
-  int y = (int)(rest % G.Y), z = (int)(rest / G.Y);
+  int x, y, z;
+  if (N <= 0xffffffffll) {
+    const unsigned v = (unsigned)v0, rest = v / (unsigned)G.X;
+    x = (int)(v - rest * (unsigned)G.X);
+    z = (int)(rest / (unsigned)G.Y);
+    y = (int)(rest - (unsigned)z * (unsigned)G.Y);
+  } else {
+    const int64_t rest = v0 / G.X;
+    x = (int)(v0 - rest * G.X);
+    y = (int)(rest % G.Y);
+    z = (int)(rest / G.Y);
+  }
+  if ((G.X & 3) == 0) {
+    const int64_t t = G.tile_base + (x >> 3) + (int64_t)G.TX * ((y >> 3) + (int64_t)G.TY * (z >> 3));
+    const int64_t g = t * TV + (x & 7) + 8 * (y & 7) + 64 * (z & 7);
+    int h[4];
+    unsigned b = 0;
+    if (sink) ldcg4(P.h + g, h);
+    if (source) b = __ldcg(reinterpret_cast<const unsigned*>(P.reach + g));
+    if (sink) *sink = (h[0] < INF ? 1u : 0u) | (h[1] < INF ? 256u : 0u) | (h[2] < INF ? 65536u : 0u) | (h[3] < INF ? 1u << 24 : 0u);
+    if (source) *source = b;  // bytes of 0 or 1
+    return;
+  }
   int64_t gk[4];
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
@@ -1066,6 +1122,20 @@ __device__ __forceinline__ void seg_store4(uint8_t* out, int64_t v0, int64_t N, 
     *reinterpret_cast<unsigned*>(p) = w;
   } else {
     for (int k = 0; k < 4 && v0 + k < N; ++k) p[k] = (uint8_t)(w >> (8 * k));
+  }
+}
+
+// Both cut sets of an instance into src / snk (1/0 bytes, each may be null);
+// CTA `cta` of `ctas`.
+__device__ __forceinline__ void seg_instance(const DevPool& P, int inst, uint8_t* src, uint8_t* snk, int cta, int ctas) {
+  const InstGeo G = P.geo[inst];
+  const int64_t N = (int64_t)G.X * G.Y * G.Z;
+#pragma unroll 4
+  for (int64_t v0 = 4 * ((int64_t)cta * blockDim.x + threadIdx.x); v0 < N; v0 += 4 * (int64_t)ctas * blockDim.x) {
+    unsigned a = 0, b = 0;
+    seg_gather4(P, G, v0, N, snk ? &a : nullptr, src ? &b : nullptr);
+    if (src) seg_store4(src, v0, N, b, 1, 0);
+    if (snk) seg_store4(snk, v0, N, a, 1, 0);
   }
 }
 

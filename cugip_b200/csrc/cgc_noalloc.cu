@@ -177,18 +177,18 @@ extern "C" int cgc_grid_maxflow_noalloc(int32_t X, int32_t Y, int32_t Z, const i
   G.hdead = (int32_t)((int64_t)X * Y * Z + 1);  // distances to the sink are at most X*Y*Z
 
   // everything that must start at zero: counters, flow, statistics, error
-  // word, barrier, queue stamps
+  // word, barrier (the upload kernel clears the queue stamps)
   NA_CUDA(cudaMemsetAsync(base + kOffCnt, 0, kOffBar + 8 - kOffCnt, st));
-  NA_CUDA(cudaMemsetAsync(base + kOffStampB, 0, kOffLists - kOffStampB, st));
   k_noalloc_tables<<<(unsigned)((T + 255) / 256), 256, 0, st>>>(P, G);
   NA_CUDA(cudaGetLastError());
-  k_put_tlinks<<<(unsigned)T, 512, 0, st>>>(P, 0, capS, capT);
-  NA_CUDA(cudaGetLastError());
+  InputPlanes in{};
+  in.p[0] = capS;
+  in.p[1] = capT;
   for (int a = 0; a < 3; ++a) {
-    k_put_nlinks<<<(unsigned)T, 512, 0, st>>>(P, 0, a, fwd ? fwd[a] : nullptr, bwd ? bwd[a] : nullptr);
-    NA_CUDA(cudaGetLastError());
+    in.p[2 + a] = fwd ? fwd[a] : nullptr;
+    in.p[5 + a] = bwd ? bwd[a] : nullptr;
   }
-  k_prepare<<<(unsigned)T, 512, 0, st>>>(P);
+  k_put_one<<<(unsigned)((TX + 3) / 4 * TY * TZ), 128, 0, st>>>(P, in, false);
   NA_CUDA(cudaGetLastError());
 
   cgc_options o = resolve_options(opts);
@@ -199,14 +199,8 @@ extern "C" int cgc_grid_maxflow_noalloc(int32_t X, int32_t Y, int32_t Z, const i
   // a preparation error (overflowing capacities) makes every CTA leave at its
   // first barrier
   if ((rc = launch_solve(P, o, prm, dev, su->sms, st))) return rc;
-  if (source_side) {
-    k_segments<<<(unsigned)((G.hdead + 254) / 256 < 65535 ? (G.hdead + 254) / 256 : 65535), 256, 0, st>>>(
-        P, 0, CGC_SEG_SOURCE_MIN, source_side, 1, 0);
-    NA_CUDA(cudaGetLastError());
-  }
-  if (sink_side) {
-    k_segments<<<(unsigned)((G.hdead + 254) / 256 < 65535 ? (G.hdead + 254) / 256 : 65535), 256, 0, st>>>(
-        P, 0, CGC_SEG_SINK_REACH, sink_side, 1, 0);
+  if (source_side || sink_side) {
+    k_seg_one<<<(unsigned)((G.hdead + 4094) / 4096), 256, 0, st>>>(P, source_side, sink_side);
     NA_CUDA(cudaGetLastError());
   }
   struct { unsigned long long flow; int32_t err; } res;

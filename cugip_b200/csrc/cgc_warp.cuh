@@ -20,21 +20,21 @@ __device__ __forceinline__ int wv_z(int k) { return k >> 1; }
 // tflag for the second seeding step (bfs_seed_tile / bfs_queue_tile).
 // A tile whose voxels were all found unable to reach the sink stays so (dead
 // vertices neither receive nor send flow, and all their residual neighbours
-// are dead), so it keeps INF and is never visited again; heights are 0 before
-// the first relabel of a solve.  A tile whose voxels are all seeds is final
+// are dead), so it keeps INF and is never visited again.  fresh: the first
+// relabel of a solve, when the heights are not set yet.  A tile whose voxels are all seeds is final
 // at h = 1 and is never visited.
-__device__ inline void bfs_init_tile_w(const DevPool& P, const int t) {
+__device__ inline void bfs_init_tile_w(const DevPool& P, const int t, const bool fresh) {
   if (!CGC_IN_BOUNDS(P, t, P.T)) return;  // uniform over the warp
   const int lane = threadIdx.x & 31;
   const int64_t base = (int64_t)t * TV;
-  bool dead = true, all_seed = true, any_excess = false;
+  bool dead = !fresh, all_seed = true, any_excess = false;
   unsigned flags = 0;
   unsigned rms[16];
 #pragma unroll
   for (int k = 0; k < 16; ++k) {
     const int i = wv_index(lane, k);
     rms[k] = __ldcg(P.rmask + base + i);
-    dead = dead && __ldcg(P.h + base + i) == INF;
+    if (!fresh) dead = dead && __ldcg(P.h + base + i) == INF;
   }
   // a tile whose voxels were all found unable to reach the sink stays so
   dead = __all_sync(FULL, dead);
