@@ -1,6 +1,6 @@
 // Device-resident batch path: many grid instances whose capacities already
 // sit in device memory are uploaded, solved and written back by a fixed
-// sequence of 3 kernels and 4 memory operations with no host synchronisation
+// sequence of 3 kernels and 2 memory operations with no host synchronisation
 // -- one pointer-table upload and preflow kernel for all instances, one
 // persistent cooperative solve, one pointer-table output kernel -- which
 // is captured once into a CUDA graph and replayed per batch.
@@ -43,8 +43,8 @@ __global__ void __launch_bounds__(256) k_seg_all(DevPool P, uint8_t* const* __re
 
 static int ensure_tables(Pool& p) {
   if (!p.d_in) {
-    CGC_CUDA(cudaMalloc(&p.d_in, sizeof(int32_t*) * 8 * p.ninst));
-    CGC_CUDA(cudaMalloc(&p.d_out, sizeof(uint8_t*) * 2 * p.ninst));
+    if (int rc = dev_alloc(p.device, &p.d_in, sizeof(int32_t*) * 8 * p.ninst)) return rc;
+    if (int rc = dev_alloc(p.device, &p.d_out, sizeof(uint8_t*) * 2 * p.ninst)) return rc;
     p.in_ptrs.assign(8 * (size_t)p.ninst, nullptr);
     p.out_ptrs.assign(2 * (size_t)p.ninst, nullptr);
   }
@@ -90,9 +90,7 @@ int pool_enqueue(Pool& p, const cgc_options* opts, int64_t* flows_dev, cudaStrea
     if (rc) return rc;
   }
   DevPool& d = p.dp;
-  CGC_CUDA(cudaMemsetAsync(d.flow, 0, (size_t)p.ninst * 8, stream));
-  CGC_CUDA(cudaMemsetAsync(d.stats, 0, S_NSTATS * 8, stream));
-  CGC_CUDA(cudaMemsetAsync(d.bar, 0, 8, stream));  // and the error word
+  CGC_CUDA(cudaMemsetAsync(p.back_dev, 0, p.back_bytes, stream));  // statistics, barrier, error word, flows
   k_put_all<<<d.nruns, 128, 0, stream>>>(d, p.d_in);
   note_launch();
   const SolveParams prm = solve_params(o);
@@ -115,26 +113,9 @@ int pool_enqueue(Pool& p, const cgc_options* opts, int64_t* flows_dev, cudaStrea
 // Waits for the last enqueued or replayed batch; reports device errors and
 // refreshes flows and statistics.
 int pool_wait(Pool& p, cudaStream_t stream) {
+  if (int rc = queue_back(p, stream)) return rc;
   CGC_CUDA(cudaStreamSynchronize(stream));
-  int rc = check_device_error(p, "batch");
-  if (rc) return rc;
-  unsigned long long stats[S_NSTATS];
-  CGC_CUDA(cudaMemcpyAsync(stats, p.dp.stats, sizeof(stats), cudaMemcpyDeviceToHost, stream));
-  CGC_CUDA(cudaMemcpyAsync(p.flows.data(), p.dp.flow, (size_t)p.ninst * 8, cudaMemcpyDeviceToHost, stream));
-  CGC_CUDA(cudaStreamSynchronize(stream));
-  std::memset(&p.st, 0, sizeof(p.st));
-  for (int64_t f : p.flows) p.st.flow += f;
-  p.st.sweeps = (int64_t)stats[S_SWEEPS];
-  p.st.global_relabels = (int64_t)stats[S_RELABELS];
-  p.st.bfs_rounds = (int64_t)stats[S_ROUNDS];
-  p.st.tiles_swept = (int64_t)stats[S_TILES_SWEPT];
-  p.st.tiles_relabelled = (int64_t)stats[S_TILES_BFS];
-  p.st.tiles_checked = (int64_t)stats[S_TILES_CHECK];
-  p.st.pulses = (int64_t)stats[S_PULSES];
-  p.st.bfs_ms = 1e-6 * (double)stats[S_NS_BFS];
-  p.st.sweep_ms = 1e-6 * (double)stats[S_NS_SWEEP];
-  p.st.reach_ms = 1e-6 * (double)stats[S_NS_REACH];
-  p.st.sched_ms = 1e-6 * (double)stats[S_NS_SCHED];
+  if (int rc = read_back(p, "batch")) return rc;
   return ok();
 }
 

@@ -493,7 +493,13 @@ using cgc::ok;
 
 void graph_free(cgc_graph* g) {
   if (!g) return;
-  if (g->dbuf) cudaFree(g->dbuf);
+  if (g->dbuf) {  // the block may be handed out again: nothing may be using it
+    int cur = 0;
+    const bool other = cudaGetDevice(&cur) == cudaSuccess && cur != g->device && cudaSetDevice(g->device) == cudaSuccess;
+    cudaDeviceSynchronize();
+    if (other) cudaSetDevice(cur);
+    cgc::dev_free(g->dbuf);
+  }
   delete g;
 }
 
@@ -544,7 +550,7 @@ int graph_create(int32_t n, int64_t m, const int32_t* a, const int32_t* b, const
     const int64_t o_bar = off; off += al(8);
     const int64_t o_seg = off; off += al(n);
     const int64_t o_bs = off; off += al((int64_t)nb * 4);
-    CGC_CUDA(cudaMalloc(&g->dbuf, off));
+    if (int rc2 = dev_alloc(g->device, &g->dbuf, off)) return rc2;
     CGC_CUDA(cudaMemsetAsync(g->dbuf, 0, off, g->stream));
     char* base = (char*)g->dbuf;
     CsrDev& d = g->d;
@@ -575,7 +581,7 @@ int graph_create(int32_t n, int64_t m, const int32_t* a, const int32_t* b, const
     if (m > 0) {
       // edges to the device, then degrees -> row offsets -> arcs
       int32_t* stage = nullptr;
-      CGC_CUDA(cudaMalloc(&stage, 4 * m * 4));
+      if (int rc2 = dev_alloc(g->device, &stage, 4 * m * 4)) return rc2;
       int rc2 = [&]() -> int {
         CGC_CUDA(cudaMemcpyAsync(stage, a, m * 4, cudaMemcpyHostToDevice, g->stream));
         CGC_CUDA(cudaMemcpyAsync(stage + m, b, m * 4, cudaMemcpyHostToDevice, g->stream));
@@ -596,16 +602,17 @@ int graph_create(int32_t n, int64_t m, const int32_t* a, const int32_t* b, const
         CGC_CUDA(cudaStreamSynchronize(g->stream));
         return CGC_OK;
       }();
-      cudaFree(stage);
+      if (rc2) cudaStreamSynchronize(g->stream);
+      dev_free(stage);
       if (rc2) return rc2;
     }
-    cudaDeviceProp prop;
-    CGC_CUDA(cudaGetDeviceProperties(&prop, g->device));
+    int sms = 0;
+    CGC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, g->device));
     // lanes per vertex: about its average number of arcs; enough CTAs to cover
     // the vertices, at most one per SM
     const int64_t degree = arcs / n;
     g->lanes = degree >= 12 ? 16 : degree >= 6 ? 8 : 4;
-    g->coop_blocks = std::max(1, std::min(prop.multiProcessorCount, grid_blocks((int64_t)n * g->lanes, CSR_THREADS)));
+    g->coop_blocks = std::max(1, std::min(sms, grid_blocks((int64_t)n * g->lanes, CSR_THREADS)));
     CGC_CUDA(cudaStreamSynchronize(g->stream));
     return CGC_OK;
   }();

@@ -61,6 +61,14 @@ __global__ void __launch_bounds__(256) k_seg_one(DevPool P, uint8_t* src, uint8_
   seg_instance(P, 0, src, snk, blockIdx.x, gridDim.x);
 }
 
+__global__ void __launch_bounds__(256) k_copy_two(int32_t* __restrict__ d0, const int32_t* __restrict__ s0,
+                                                  int32_t* __restrict__ d1, const int32_t* __restrict__ s1, int64_t n) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    d0[i] = s0[i];
+    d1[i] = s1[i];
+  }
+}
+
 // Cut sets as mask / background bytes from the 1/0 bytes of one buffer
 // (16 bytes per thread where src and dst allow it).
 __global__ void k_mask_remap(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, int64_t n, uint8_t mask,
@@ -559,7 +567,12 @@ int launch_solve(const DevPool& d, const cgc_options& o, const SolveParams& prm,
   cfg.blockDim = dim3(groups * GROUP);
   cfg.dynamicSmemBytes = groups * sizeof(TileShared);
   // a property of the function on the current device, set before its first launch there
-  CGC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes));
+  static std::atomic<bool> done[64][3] = {};
+  const int which = groups == 8 ? 2 : groups == 5 ? 1 : 0;
+  if (device < 0 || device >= 64 || !done[device][which].load(std::memory_order_acquire)) {
+    CGC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes));
+    if (device >= 0 && device < 64) done[device][which].store(true, std::memory_order_release);
+  }
   int rc = coop_launch_ordered(device, stream, [&]() -> int {
     CGC_CUDA(cudaLaunchKernelEx(&cfg, kernel, d, prm));
     return CGC_OK;
@@ -611,26 +624,124 @@ __global__ void k_unpermute(DevPool P, int inst, const int32_t* plane, int32_t* 
 // host side
 // ===========================================================================
 
-int check_device_error(Pool& p, const char* where) {
-  int32_t err = 0;
-  CGC_CUDA(cudaMemcpyAsync(&err, p.dp.err, sizeof(int32_t), cudaMemcpyDeviceToHost, p.stream));
-  CGC_CUDA(cudaStreamSynchronize(p.stream));
+static std::mutex g_mem_mu;
+static cudaMemPool_t g_mem_pool[64] = {};
+static cudaStream_t g_mem_stream[64] = {};
+static bool g_mem_tried[64] = {};
+
+int dev_alloc(int device, void** p, size_t bytes) {
+  constexpr size_t kLargest = (size_t)128 << 20;
+  constexpr unsigned long long kKept = 256ull << 20;
+  if (bytes <= kLargest && device >= 0 && device < 64) {
+    std::lock_guard<std::mutex> lock(g_mem_mu);
+    if (!g_mem_tried[device]) {
+      g_mem_tried[device] = true;
+      int has = 0;
+      cudaMemPoolProps props = {};
+      props.allocType = cudaMemAllocationTypePinned;
+      props.location.type = cudaMemLocationTypeDevice;
+      props.location.id = device;
+      unsigned long long kept = kKept;
+      if (cudaDeviceGetAttribute(&has, cudaDevAttrMemoryPoolsSupported, device) == cudaSuccess && has &&
+          cudaMemPoolCreate(&g_mem_pool[device], &props) == cudaSuccess) {
+        if (cudaMemPoolSetAttribute(g_mem_pool[device], cudaMemPoolAttrReleaseThreshold, &kept) != cudaSuccess ||
+            cudaStreamCreateWithFlags(&g_mem_stream[device], cudaStreamNonBlocking) != cudaSuccess) {
+          cudaMemPoolDestroy(g_mem_pool[device]);
+          g_mem_pool[device] = nullptr;
+        }
+      }
+      cudaGetLastError();
+    }
+    if (g_mem_pool[device]) {
+      // allocated on a stream of its own and waited for, so any stream may use it
+      if (cudaMallocFromPoolAsync(p, bytes, g_mem_pool[device], g_mem_stream[device]) == cudaSuccess) {
+        CGC_CUDA(cudaStreamSynchronize(g_mem_stream[device]));
+        return CGC_OK;
+      }
+      cudaGetLastError();
+    }
+  }
+  CGC_CUDA(cudaMalloc(p, bytes));
+  return CGC_OK;
+}
+
+static std::mutex g_pin_mu;
+static char* g_pin = nullptr;
+static uint64_t g_pin_used = 0;
+constexpr size_t kPinSlot = 1024, kPinSlots = 64;
+
+void* pinned_take(size_t bytes) {
+  void* p = nullptr;
+  if (bytes <= kPinSlot) {
+    std::lock_guard<std::mutex> lock(g_pin_mu);
+    if (!g_pin && cudaMallocHost(&p, kPinSlot * kPinSlots) == cudaSuccess) g_pin = (char*)p;
+    if (g_pin && ~g_pin_used) {
+      const int i = __builtin_ctzll(~g_pin_used);
+      g_pin_used |= 1ull << i;
+      return g_pin + i * kPinSlot;
+    }
+  }
+  return cudaMallocHost(&p, bytes) == cudaSuccess ? p : nullptr;
+}
+
+void pinned_give(void* p) {
+  if (!p) return;
+  {
+    std::lock_guard<std::mutex> lock(g_pin_mu);
+    const char* c = (const char*)p;
+    if (g_pin && c >= g_pin && c < g_pin + kPinSlot * kPinSlots) {
+      g_pin_used &= ~(1ull << ((c - g_pin) / kPinSlot));
+      return;
+    }
+  }
+  cudaFreeHost(p);
+}
+
+static int device_error(int err, long long bound_at, const char* where) {
   if (err == 0) return CGC_OK;
 #ifdef CGC_BOUNDS_CHECK
-  if (err == CGC_ERR_ARG) {
-    unsigned long long at = 0;
-    CGC_CUDA(cudaMemcpyAsync(&at, p.dp.stats + S_BOUND_AT, 8, cudaMemcpyDeviceToHost, p.stream));
-    CGC_CUDA(cudaStreamSynchronize(p.stream));
-    return fail(err, std::string(where) + ": index out of range (bounds-checked build): " +
-                         std::to_string((long long)at) + ", or a negative capacity");
-  }
+  if (err == CGC_ERR_ARG)
+    return fail(err, std::string(where) + ": index out of range (bounds-checked build): " + std::to_string(bound_at) +
+                         ", or a negative capacity");
 #endif
+  (void)bound_at;
   const char* what = err == CGC_ERR_OVERFLOW ? "capacities may overflow int32 excess/residuals (or a capacity points outside the grid)"
                    : err == CGC_ERR_ARG ? "negative capacity"
                    : err == CGC_ERR_TIMEOUT ? "a device-side wait timed out"
                    : err == CGC_ERR_NOT_CONVERGED ? "max_sweeps reached before convergence"
                    : "device error";
   return fail(err, std::string(where) + ": " + what);
+}
+
+int queue_back(Pool& p, cudaStream_t stream) {
+  CGC_CUDA(cudaMemcpyAsync(p.pinned_cnt + 64, p.back_dev, p.back_bytes, cudaMemcpyDeviceToHost, stream));
+  return CGC_OK;
+}
+
+int check_device_error(Pool& p, const char* where) {
+  if (int rc = queue_back(p, p.stream)) return rc;
+  CGC_CUDA(cudaStreamSynchronize(p.stream));
+  return device_error((int)(p.back()[S_NSTATS] >> 32), (long long)p.back()[S_BOUND_AT], where);
+}
+
+int read_back(Pool& p, const char* where) {
+  const unsigned long long* stats = p.back();
+  if (int rc = device_error((int)(stats[S_NSTATS] >> 32), (long long)stats[S_BOUND_AT], where)) return rc;
+  std::memcpy(p.flows.data(), stats + S_NSTATS + 1, (size_t)p.ninst * 8);
+  std::memset(&p.st, 0, sizeof(p.st));
+  for (int64_t f : p.flows) p.st.flow += f;
+  p.st.sweeps = (int64_t)stats[S_SWEEPS];
+  p.st.global_relabels = (int64_t)stats[S_RELABELS];
+  p.st.bfs_rounds = (int64_t)stats[S_ROUNDS];
+  p.st.tiles_swept = (int64_t)stats[S_TILES_SWEPT];
+  p.st.tiles_relabelled = (int64_t)stats[S_TILES_BFS];
+  p.st.tiles_checked = (int64_t)stats[S_TILES_CHECK];
+  p.st.pulses = (int64_t)stats[S_PULSES];
+  p.st.bfs_ms = 1e-6 * (double)stats[S_NS_BFS];
+  p.st.sweep_ms = 1e-6 * (double)stats[S_NS_SWEEP];
+  p.st.reach_ms = 1e-6 * (double)stats[S_NS_REACH];
+  p.st.sched_ms = 1e-6 * (double)stats[S_NS_SCHED];
+  return CGC_OK;
 }
 
 int pool_create(int32_t count, const int32_t* ext, void* stream, Pool** out) {
@@ -682,12 +793,14 @@ int pool_create(int32_t count, const int32_t* ext, void* stream, Pool** out) {
   const int64_t o_si = off; off += al(T * 4);
   const int64_t o_li = off; off += al(7 * T * 4);
   const int64_t o_cnt = off; off += al(C_NCOUNTERS * 4);
-  const int64_t o_fl = off; off += al((int64_t)count * 8);
   const int64_t o_geo = off; off += al((int64_t)count * sizeof(InstGeo));
-  const int64_t o_st = off; off += al(S_NSTATS * 8);
-  const int64_t o_bar = off; off += al(8);
+  // read back together: statistics, barrier count and error word, flows
+  const int64_t o_st = off, o_bar = off + S_NSTATS * 8, o_fl = o_bar + 8;
+  p->back_bytes = (size_t)(o_fl + (int64_t)count * 8 - o_st);
+  off += al((int64_t)p->back_bytes);
   const int64_t o_tr = off; off += al(2 * TRACE_CAP * 8);
-  CGC_CUDA(cudaMalloc(&p->dbuf, off));
+  if (int rc = dev_alloc(p->device, &p->dbuf, off)) return rc;
+  p->back_dev = (char*)p->dbuf + o_st;
   CGC_CUDA(cudaMemsetAsync(p->dbuf, 0, off, p->stream));
   char* base = (char*)p->dbuf;
   DevPool& d = p->dp;
@@ -737,13 +850,12 @@ int pool_create(int32_t count, const int32_t* ext, void* stream, Pool** out) {
     p->sumN += ((int64_t)p->geo[i].X * p->geo[i].Y * p->geo[i].Z + 3) & ~(int64_t)3;
   }
   p->host_in.assign(8 * (size_t)count, nullptr);
-  CGC_CUDA(cudaMallocHost(&p->pinned_cnt, 64 * 4));
+  p->pinned_cnt = (int32_t*)pinned_take(64 * 4 + p->back_bytes);
+  if (!p->pinned_cnt) return fail(CGC_ERR_OOM, "create: pinned host memory");
   CGC_CUDA(cudaEventCreateWithFlags(&p->inputs_read, cudaEventDisableTiming));
   for (auto& e : p->ev) CGC_CUDA(cudaEventCreate(&e));
 
-  cudaDeviceProp prop;
-  CGC_CUDA(cudaGetDeviceProperties(&prop, p->device));
-  p->sms = prop.multiProcessorCount;
+  CGC_CUDA(cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, p->device));
   int occ2 = 0;
   CGC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ2, k_sweep_list, WIDE, 0));
   p->sweep_blocks = std::max(1, occ2) * p->sms;
@@ -759,12 +871,26 @@ int pool_create(int32_t count, const int32_t* ext, void* stream, Pool** out) {
 // setter returns once the host array has been read: the reference's setters
 // copy at call time too (graph_cut.hpp:284-285, 298-299).  Device-pointer
 // setters copy device to device on the solve stream.
-static int ensure_lin(Pool& p, bool bwd) {
+// The same allocation holds the cut sets of the solve that will read them and
+// the device table of their addresses.
+static int ensure_lin(Pool& p, bool bwd, bool host) {
   if (!p.lin) {
-    CGC_CUDA(cudaMalloc(&p.lin, 5 * (size_t)p.sumN * 4));
-    CGC_CUDA(cudaStreamCreateWithFlags(&p.copy_stream, cudaStreamNonBlocking));
+    const size_t in = 5 * (size_t)p.sumN * 4, seg = (2 * (size_t)p.sumN + 255) & ~(size_t)255;
+    const size_t tab = 2 * (size_t)p.ninst * sizeof(uint8_t*);
+    if (int rc = dev_alloc(p.device, &p.lin, ((in + 255) & ~(size_t)255) + seg + tab)) return rc;
+    p.segbuf = (uint8_t*)p.lin + ((in + 255) & ~(size_t)255);
+    p.d_segtab = (uint8_t**)(p.segbuf + seg);
+    std::vector<uint8_t*> addr(2 * (size_t)p.ninst);
+    for (int i = 0; i < p.ninst; ++i) {
+      addr[2 * i] = p.segbuf + p.voff[i];               // source side
+      addr[2 * i + 1] = p.segbuf + p.sumN + p.voff[i];  // sink side
+    }
+    // pageable source: staged before the call returns
+    CGC_CUDA(cudaMemcpyAsync(p.d_segtab, addr.data(), tab, cudaMemcpyHostToDevice, p.stream));
   }
-  if (bwd && !p.lin_bwd) CGC_CUDA(cudaMalloc(&p.lin_bwd, 3 * (size_t)p.sumN * 4));
+  if (bwd && !p.lin_bwd)
+    if (int rc = dev_alloc(p.device, &p.lin_bwd, 3 * (size_t)p.sumN * 4)) return rc;
+  if (host && !p.copy_stream) CGC_CUDA(cudaStreamCreateWithFlags(&p.copy_stream, cudaStreamNonBlocking));
   return CGC_OK;
 }
 
@@ -778,15 +904,27 @@ static int copy_plane(Pool& p, int32_t* dst, const int32_t* src, int64_t N, bool
   return CGC_OK;
 }
 
+// Two planes device to device on the solve stream: small ones by one kernel (a
+// copy command each costs more than the copy), large ones by the copy commands.
+static int copy_two(Pool& p, int32_t* d0, const int32_t* s0, int32_t* d1, const int32_t* s1, int64_t N, bool host) {
+  if (!host && N <= (1 << 18)) {
+    k_copy_two<<<(unsigned)((N + 1023) / 1024), 256, 0, p.stream>>>(d0, s0, d1, s1, N);
+    note_launch();
+    CGC_CUDA(cudaGetLastError());
+    return CGC_OK;
+  }
+  if (int rc = copy_plane(p, d0, s0, N, host)) return rc;
+  return copy_plane(p, d1, s1, N, host);
+}
+
 int pool_put_tlinks(Pool& p, int inst, const int32_t* capS, const int32_t* capT, bool host) {
   if (inst < 0 || inst >= p.ninst || !capS || !capT) return fail(CGC_ERR_ARG, "set_tlinks: bad arguments");
   const InstGeo& G = p.geo[inst];
   const int64_t N = (int64_t)G.X * G.Y * G.Z;
-  if (int rc = ensure_lin(p, false)) return rc;
+  if (int rc = ensure_lin(p, false, host)) return rc;
   int32_t* s = p.lin + p.voff[inst];
   int32_t* c = p.lin + p.sumN + p.voff[inst];
-  if (int rc = copy_plane(p, s, capS, N, host)) return rc;
-  if (int rc = copy_plane(p, c, capT, N, host)) return rc;
+  if (int rc = copy_two(p, s, capS, c, capT, N, host)) return rc;
   if (host) CGC_CUDA(cudaStreamSynchronize(p.copy_stream));
   p.host_in[8 * (size_t)inst] = s;
   p.host_in[8 * (size_t)inst + 1] = c;
@@ -802,12 +940,10 @@ int pool_put_nlinks(Pool& p, int inst, int axis, const int32_t* fwd, const int32
   const InstGeo& G = p.geo[inst];
   const int64_t N = (int64_t)G.X * G.Y * G.Z;
   const bool same = bwd == fwd;  // symmetric weights: one plane
-  if (int rc = ensure_lin(p, !same)) return rc;
+  if (int rc = ensure_lin(p, !same, host)) return rc;
   int32_t* f = p.lin + (2 + axis) * p.sumN + p.voff[inst];
   int32_t* b = same ? f : p.lin_bwd + axis * p.sumN + p.voff[inst];
-  if (int rc = copy_plane(p, f, fwd, N, host)) return rc;
-  if (!same)
-    if (int rc = copy_plane(p, b, bwd, N, host)) return rc;
+  if (int rc = same ? copy_plane(p, f, fwd, N, host) : copy_two(p, f, fwd, b, bwd, N, host)) return rc;
   if (host) CGC_CUDA(cudaStreamSynchronize(p.copy_stream));
   p.host_in[8 * (size_t)inst + 2 + axis] = f;
   p.host_in[8 * (size_t)inst + 5 + axis] = b;
@@ -895,21 +1031,6 @@ static int host_bfs(Pool& p, uint32_t& id, int64_t& rounds) {
   return CGC_OK;
 }
 
-// Buffers of the host-path outputs: both cut sets of every instance (1/0
-// bytes, linear order) and the device table of their addresses.
-static int ensure_segbuf(Pool& p) {
-  if (p.segbuf) return CGC_OK;
-  CGC_CUDA(cudaMalloc(&p.segbuf, 2 * (size_t)p.sumN));
-  CGC_CUDA(cudaMalloc(&p.d_segtab, 2 * (size_t)p.ninst * sizeof(uint8_t*)));
-  std::vector<uint8_t*> tab(2 * (size_t)p.ninst);
-  for (int i = 0; i < p.ninst; ++i) {
-    tab[2 * i] = p.segbuf + p.voff[i];               // source side
-    tab[2 * i + 1] = p.segbuf + p.sumN + p.voff[i];  // sink side
-  }
-  CGC_CUDA(cudaMemcpy(p.d_segtab, tab.data(), tab.size() * sizeof(uint8_t*), cudaMemcpyHostToDevice));
-  return CGC_OK;
-}
-
 // Enqueues one solve of the set_* inputs on p.stream: fused upload and
 // preflow, the solve, and both cut sets of every instance into segbuf.  With
 // the persistent solve (the default) nothing synchronises the host, so the
@@ -929,17 +1050,15 @@ int pool_solve_async(Pool& p, const cgc_options* opts) {
   const SolveParams prm = solve_params(o);
   if (o.persistent > 0 && (prm.learned || prm.trace_cycles))  // buffers and weights before anything is queued
     if (int rc = ensure_sched(p, prm.learned != 0, prm.trace_cycles)) return rc;
-  if (int rc = ensure_segbuf(p)) return rc;
   if (p.ninst > 1) {
-    if (!p.d_host_in) CGC_CUDA(cudaMalloc(&p.d_host_in, 8 * (size_t)p.ninst * sizeof(int32_t*)));
+    if (!p.d_host_in)
+      if (int rc = dev_alloc(p.device, &p.d_host_in, 8 * (size_t)p.ninst * sizeof(int32_t*))) return rc;
     // pageable source: the table is staged before the call returns
     CGC_CUDA(cudaMemcpyAsync(p.d_host_in, in.data(), in.size() * sizeof(int32_t*), cudaMemcpyHostToDevice, p.stream));
   }
   p.launches0 = g_launches.load();
   CGC_CUDA(cudaEventRecord(p.ev[0], p.stream));
-  CGC_CUDA(cudaMemsetAsync(d.flow, 0, (size_t)p.ninst * 8, p.stream));
-  CGC_CUDA(cudaMemsetAsync(d.stats, 0, S_NSTATS * 8, p.stream));
-  CGC_CUDA(cudaMemsetAsync(d.bar, 0, 8, p.stream));  // and the error word
+  CGC_CUDA(cudaMemsetAsync(p.back_dev, 0, p.back_bytes, p.stream));  // statistics, barrier, error word, flows
   if (p.ninst == 1) {
     InputPlanes ip;
     for (int k = 0; k < 8; ++k) ip.p[k] = in[k];
@@ -1004,6 +1123,7 @@ int pool_solve_async(Pool& p, const cgc_options* opts) {
     note_launch();
     CGC_CUDA(cudaGetLastError());
   }
+  if (!rc) rc = queue_back(p, p.stream);
   CGC_CUDA(cudaEventRecord(p.ev[1], p.stream));
   if (rc) {
     // nothing to wait for: leave the stream idle and report now
@@ -1020,36 +1140,18 @@ int pool_solve_wait(Pool& p) {
   if (!p.pending) return fail(CGC_ERR_STATE, "wait: no solve was enqueued");
   p.pending = false;
   CGC_CUDA(cudaEventSynchronize(p.ev[1]));
-  if (int rc = check_device_error(p, "maxflow")) return rc;
+  if (int rc = read_back(p, "maxflow")) return rc;
   float ms = 0.f, kms = 0.f;
   cudaEventElapsedTime(&ms, p.ev[0], p.ev[1]);
   cudaEventElapsedTime(&kms, p.ev[2], p.ev[3]);
-  unsigned long long stats[S_NSTATS];
-  CGC_CUDA(cudaMemcpyAsync(stats, p.dp.stats, sizeof(stats), cudaMemcpyDeviceToHost, p.stream));
-  CGC_CUDA(cudaMemcpyAsync(p.flows.data(), p.dp.flow, (size_t)p.ninst * 8, cudaMemcpyDeviceToHost, p.stream));
-  CGC_CUDA(cudaStreamSynchronize(p.stream));
-  std::memset(&p.st, 0, sizeof(p.st));
-  for (int64_t f : p.flows) p.st.flow += f;
-  if (p.pending_persistent > 0) {
-    p.st.sweeps = (int64_t)stats[S_SWEEPS];
-    p.st.global_relabels = (int64_t)stats[S_RELABELS];
-    p.st.bfs_rounds = (int64_t)stats[S_ROUNDS];
-  } else {
+  if (p.pending_persistent <= 0) {
     p.st.sweeps = p.host_counts[0];
     p.st.global_relabels = p.host_counts[1];
     p.st.bfs_rounds = p.host_counts[2];
   }
-  p.st.tiles_swept = (int64_t)stats[S_TILES_SWEPT];
-  p.st.tiles_relabelled = (int64_t)stats[S_TILES_BFS];
-  p.st.tiles_checked = (int64_t)stats[S_TILES_CHECK];
-  p.st.pulses = (int64_t)stats[S_PULSES];
   p.st.solve_ms = ms;
   p.st.kernel_ms = kms;
   p.st.launches = g_launches.load() - p.launches0;
-  p.st.bfs_ms = 1e-6 * (double)stats[S_NS_BFS];
-  p.st.sweep_ms = 1e-6 * (double)stats[S_NS_SWEEP];
-  p.st.reach_ms = 1e-6 * (double)stats[S_NS_REACH];
-  p.st.sched_ms = 1e-6 * (double)stats[S_NS_SCHED];
   p.solved = true;
   p.seg_valid = true;
   return ok();
@@ -1067,7 +1169,8 @@ int pool_segments(Pool& p, int inst, int which, uint8_t* out, uint8_t mask, uint
   if (!p.solved) return fail(CGC_ERR_STATE, "get_segments: call maxflow first");
   const InstGeo& G = p.geo[inst];
   const int64_t N = (int64_t)G.X * G.Y * G.Z;
-  if ((host || !p.seg_valid || mask != 1 || bg != 0) && !p.segtmp) CGC_CUDA(cudaMalloc(&p.segtmp, p.maxN));
+  if ((host || !p.seg_valid || mask != 1 || bg != 0) && !p.segtmp)
+    if (int rc = dev_alloc(p.device, &p.segtmp, p.maxN)) return rc;
   const unsigned blocks = (unsigned)std::min<int64_t>(std::max<int64_t>((N + 4095) / 4096, 1), 8 * (int64_t)p.sms);
   const uint8_t* src = nullptr;  // device bytes to copy to `out` as they are
   if (p.seg_valid) {
@@ -1098,7 +1201,8 @@ int pool_residuals(Pool& p, int inst, int32_t* const res[6], int32_t* resT, int3
   if (!p.solved) return fail(CGC_ERR_STATE, "get_residuals: call maxflow first");
   const InstGeo& G = p.geo[inst];
   const int64_t N = (int64_t)G.X * G.Y * G.Z;
-  if (!p.resid) CGC_CUDA(cudaMalloc(&p.resid, (size_t)p.maxN * 4));
+  if (!p.resid)
+    if (int rc = dev_alloc(p.device, &p.resid, (size_t)p.maxN * 4)) return rc;
   const int blocks = (int)std::min<int64_t>((N + 255) / 256, 65535);
   auto one = [&](const int32_t* plane, int32_t* out) -> int {
     if (!out) return CGC_OK;
@@ -1125,7 +1229,8 @@ int pool_labels(Pool& p, int inst, int32_t* labels) {
   if (!p.solved) return fail(CGC_ERR_STATE, "get_labels: call maxflow first");
   const InstGeo& G = p.geo[inst];
   const int64_t N = (int64_t)G.X * G.Y * G.Z;
-  if (!p.resid) CGC_CUDA(cudaMalloc(&p.resid, (size_t)p.maxN * 4));
+  if (!p.resid)
+    if (int rc = dev_alloc(p.device, &p.resid, (size_t)p.maxN * 4)) return rc;
   k_unpermute<<<(int)std::min<int64_t>((N + 255) / 256, 65535), 256, 0, p.stream>>>(p.dp, inst, p.dp.h, p.resid);
   note_launch();
   CGC_CUDA(cudaGetLastError());

@@ -63,10 +63,10 @@ constexpr int64_t kOffStampS = kOffStampB + al256(kMaxTiles * 4);
 constexpr int64_t kOffStampI = kOffStampS + al256(kMaxTiles * 4);
 constexpr int64_t kOffLists = kOffStampI + al256(kMaxTiles * 4);
 constexpr int64_t kOffCnt = kOffLists + al256(7 * kMaxTiles * 4);
-constexpr int64_t kOffFlow = kOffCnt + al256(C_NCOUNTERS * 4);
-constexpr int64_t kOffGeo = kOffFlow + al256(8);
+constexpr int64_t kOffGeo = kOffCnt + al256(C_NCOUNTERS * 4);
 constexpr int64_t kOffStats = kOffGeo + al256(sizeof(InstGeo));
-constexpr int64_t kOffBar = kOffStats + al256(S_NSTATS * 8);  // barrier count, error word
+constexpr int64_t kOffFlow = kOffStats + al256(S_NSTATS * 8);  // read back together: flow, barrier count, error word
+constexpr int64_t kOffBar = kOffFlow + 8;
 constexpr int64_t kScratchBytes = kOffBar + al256(8);
 
 }  // namespace
@@ -203,9 +203,9 @@ extern "C" int cgc_grid_maxflow_noalloc(int32_t X, int32_t Y, int32_t Z, const i
     k_seg_one<<<(unsigned)((G.hdead + 4094) / 4096), 256, 0, st>>>(P, source_side, sink_side);
     NA_CUDA(cudaGetLastError());
   }
-  struct { unsigned long long flow; int32_t err; } res;
-  NA_CUDA(cudaMemcpyAsync(&res.flow, base + kOffFlow, 8, cudaMemcpyDeviceToHost, st));
-  NA_CUDA(cudaMemcpyAsync(&res.err, base + kOffBar + 4, 4, cudaMemcpyDeviceToHost, st));
+  struct { unsigned long long flow; uint32_t bar; int32_t err; } res;
+  static_assert(sizeof(res) == 16, "layout of the scratch array's flow, barrier count and error word");
+  NA_CUDA(cudaMemcpyAsync(&res, base + kOffFlow, sizeof(res), cudaMemcpyDeviceToHost, st));
   NA_CUDA(cudaStreamSynchronize(st));
   if (res.err) {
     const char* what = res.err == CGC_ERR_OVERFLOW ? "capacities may overflow int32 excess/residuals"

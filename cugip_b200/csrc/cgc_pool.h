@@ -25,6 +25,20 @@ namespace cgc {
 extern std::atomic<long long> g_launches;
 void note_launch();
 
+// Device memory of handles.  Blocks of at most 128 MB come from a CUDA memory
+// pool of the device that keeps up to 256 MB of freed blocks mapped (anything
+// above goes back to the driver): mapping and unmapping a block costs about
+// 0.35 ms each, more than a small solve.  dev_free may be called once no work
+// uses the block.
+int dev_alloc(int device, void** p, size_t bytes);
+template <typename T>
+int dev_alloc(int device, T** p, size_t bytes) { return dev_alloc(device, reinterpret_cast<void**>(p), bytes); }
+inline void dev_free(void* p) { if (p) cudaFree(p); }
+// Pinned host memory of a handle: a slot of one 64 KB block the process keeps,
+// or a block of its own (null: no memory).
+void* pinned_take(size_t bytes);
+void pinned_give(void* p);
+
 struct Pool {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -40,7 +54,7 @@ struct Pool {
   // to back at voff[i]; read by the fused upload kernel of the next solve.
   int64_t sumN = 0;
   std::vector<int64_t> voff;
-  int32_t* lin = nullptr;        // 5 planes of sumN: capS, capT, fwd x/y/z (first set_* call)
+  int32_t* lin = nullptr;        // 5 planes of sumN: capS, capT, fwd x/y/z (first set_* call), then segbuf and d_segtab
   int32_t* lin_bwd = nullptr;    // 3 planes of sumN: bwd x/y/z (first asymmetric n-link upload)
   std::vector<const int32_t*> host_in;  // 8 per instance: planes the next solve reads (null = zero)
   const int32_t** d_host_in = nullptr;  // device copy of host_in (batches of more than one instance)
@@ -58,7 +72,10 @@ struct Pool {
   int pending_persistent = 1;    // its options' persistent field
   long long launches0 = 0;       // launch counter when it was enqueued
   int64_t host_counts[3] = {0, 0, 0};  // host-driven schedule: sweeps, relabels, BFS rounds
-  int32_t* pinned_cnt = nullptr; // host-pinned counters
+  int32_t* pinned_cnt = nullptr; // host-pinned: 64 counters, then the read-back of back_dev
+  void* back_dev = nullptr;      // device: statistics, barrier and error word, flows (contiguous)
+  size_t back_bytes = 0;
+  const unsigned long long* back() const { return reinterpret_cast<const unsigned long long*>(pinned_cnt + 64); }
   bool solved = false;
   int sms = 148;
   int sweep_blocks = 0;
@@ -80,31 +97,39 @@ struct Pool {
   int trace_cap = 0;
   uint64_t sched_wver = 0;
   ~Pool() {
+    if (dbuf) {  // the blocks may be handed out again: nothing may be using them
+      int cur = 0;
+      const bool other = cudaGetDevice(&cur) == cudaSuccess && cur != device && cudaSetDevice(device) == cudaSuccess;
+      cudaDeviceSynchronize();
+      if (other) cudaSetDevice(cur);
+    }
     if (sbuf) cudaFree(sbuf);
     if (tbuf) cudaFree(tbuf);
     if (graph_exec) cudaGraphExecDestroy(graph_exec);
     if (graph) cudaGraphDestroy(graph);
     if (cap_stream) cudaStreamDestroy(cap_stream);
-    if (d_in) cudaFree(d_in);
-    if (d_out) cudaFree(d_out);
-    if (dbuf) cudaFree(dbuf);
-    if (lin) cudaFree(lin);
-    if (lin_bwd) cudaFree(lin_bwd);
-    if (d_host_in) cudaFree(d_host_in);
-    if (segbuf) cudaFree(segbuf);
-    if (d_segtab) cudaFree(d_segtab);
-    if (segtmp) cudaFree(segtmp);
-    if (resid) cudaFree(resid);
+    dev_free(d_in);
+    dev_free(d_out);
+    dev_free(dbuf);
+    dev_free(lin);
+    dev_free(lin_bwd);
+    dev_free(d_host_in);
+    dev_free(segtmp);
+    dev_free(resid);
     if (inputs_read) cudaEventDestroy(inputs_read);
     for (auto e : ev)
       if (e) cudaEventDestroy(e);
     if (copy_stream) cudaStreamDestroy(copy_stream);
-    if (pinned_cnt) cudaFreeHost(pinned_cnt);
+    pinned_give(pinned_cnt);
   }
 };
 
 
 int check_device_error(Pool& p, const char* where);
+// device statistics, error word and flows to the host, behind the work on stream
+int queue_back(Pool& p, cudaStream_t stream);
+// once that copy is done: the device error, or the flows and statistics
+int read_back(Pool& p, const char* where);
 int pool_create(int32_t count, const int32_t* ext, void* stream, Pool** out);
 int pool_put_tlinks(Pool& p, int inst, const int32_t* capS, const int32_t* capT, bool host);
 int pool_put_nlinks(Pool& p, int inst, int axis, const int32_t* fwd, const int32_t* bwd, bool host);
