@@ -90,7 +90,7 @@ def learned_report(workloads=(1, 2, 3)) -> dict:
     import torch
     from cugip_b200 import volume
     from cugip_b200.graph_cut import SINK, SOURCE, GridGraph, Policy
-    base = dict(local_pulses=4, region_relabels=2, sweeps_per_relabel=8, ctas_per_sm=3)
+    base = dict(local_pulses=4, region_relabels=2, sweeps_per_relabel=8)
     keep = ("kernel_ms", "sched_ms", "sweeps", "global_relabels", "tiles_swept", "pulses")
     out = {}
     for w in workloads:
@@ -158,7 +158,7 @@ def generic_layered() -> dict:
 
 def solve_kernel_name(pol) -> str:
     """The persistent solve kernel a policy launches (cgc_engine.cu launch_solve)."""
-    return {2: "k_solve4", 3: "k_solve5", 4: "k_solve8"}[pol.ctas_per_sm or 2]  # by tile groups per SM
+    return "k_solve"
 
 
 def profiled_traffic(workload: int):
@@ -173,12 +173,11 @@ def profiled_traffic(workload: int):
     return None
 
 
-# autotune candidates: pulses, region relabels and sweep pairs per cycle, tiles per SM and exclusive sweeps
-# (which only the kernel with the most tiles per SM is measured to gain from)
-BATCH_CANDIDATES = [dict(local_pulses=L, region_relabels=R, sweeps_per_relabel=K, ctas_per_sm=c, exclusive=ex)
+# autotune candidates: pulses, region relabels and sweep pairs per cycle, and exclusive sweeps
+BATCH_CANDIDATES = [dict(local_pulses=L, region_relabels=R, sweeps_per_relabel=K, exclusive=ex)
                     for (L, R, K) in ((4, 2, 8), (2, 4, 4), (2, 4, 8), (4, 2, 4), (4, 4, 8), (8, 2, 8), (2, 4, 6),
                                       (4, 2, 6))
-                    for c in (2, 3, 4) for ex in ((0, 1) if c == 4 else (0,))]
+                    for ex in (0, 1)]
 GRID_SCHEDULES = ((4, 2, 8), (2, 4, 4), (8, 2, 8), (4, 2, 16), (2, 4, 8), (4, 4, 8), (4, 2, 6), (2, 4, 6))
 
 
@@ -438,13 +437,12 @@ def main():
     B = Batch([(v.X, v.Y, v.Z)])
     B.bind_inputs(0, d_in[0].data_ptr(), d_in[1].data_ptr(), [t.data_ptr() for t in d_in[2:]])
     B.bind_outputs(0, d_seg[0].data_ptr(), d_seg[1].data_ptr())
-    cands = [Policy(local_pulses=L, region_relabels=R, sweeps_per_relabel=K, ctas_per_sm=c, learned=lr, exclusive=ex)
+    cands = [Policy(local_pulses=L, region_relabels=R, sweeps_per_relabel=K, learned=lr, exclusive=ex)
              for (L, R, K) in GRID_SCHEDULES
-             for c in (2, 3, 4) for lr in ((0, 1, 3) if have_learned else (0,))
-             for ex in ((0, 1) if c == 4 else (0,))]
+             for lr in ((0, 1, 3) if have_learned else (0,)) for ex in (0, 1)]
     if args.schedule:
         L, R, K, c, lr = (int(x) for x in args.schedule.split(","))
-        best, best_ms = Policy(local_pulses=L, region_relabels=R, sweeps_per_relabel=K, ctas_per_sm=c, learned=lr), None
+        best, best_ms = Policy(local_pulses=L, region_relabels=R, sweeps_per_relabel=K, learned=lr), None
     else:
         best, best_ms = B.autotune(cands, repeats=2)
     B.graph_create(best, d_flow.data_ptr())

@@ -84,15 +84,14 @@ void store(std::pair<int, int> key, const cgc_options& o, double ms) {
 
 std::vector<cgc_options> default_candidates() {
   std::vector<cgc_options> c;
-  for (int cta : {2, 3, 4})
-    for (int R : {1, 2, 4})
-      for (int L : {2, 4, 8})
-        for (int K : {4, 8, 16}) {
-          cgc_options o{};
-          o.struct_size = sizeof(cgc_options);
-          o.local_pulses = L; o.region_relabels = R; o.sweeps_per_relabel = K; o.ctas_per_sm = cta;
-          c.push_back(o);
-        }
+  for (int R : {1, 2, 4})
+    for (int L : {2, 4, 8})
+      for (int K : {4, 8, 16}) {
+        cgc_options o{};
+        o.struct_size = sizeof(cgc_options);
+        o.local_pulses = L; o.region_relabels = R; o.sweeps_per_relabel = K;
+        c.push_back(o);
+      }
   return c;
 }
 

@@ -27,7 +27,7 @@ namespace cgc {
 constexpr int TILE = 8;
 constexpr int TV = 512;            // voxels per tile
 constexpr int INF = 0x3fffffff;    // height of vertices that cannot reach the sink
-constexpr int MAX_GROUPS = 8;      // tile groups per CTA of the persistent solve
+constexpr int GROUPS = 4;          // tile groups per CTA of the persistent solve
 
 enum Dir { PX = 0, MX = 1, PY = 2, MY = 3, PZ = 4, MZ = 5 };
 
@@ -131,9 +131,7 @@ struct SolveParams {
 struct InputPlanes { const int32_t* p[8]; };  // capS, capT, fwd x/y/z, bwd x/y/z (null = zero)
 __global__ void k_put_one(DevPool P, InputPlanes in, bool two_halves);
 __global__ void k_seg_one(DevPool P, uint8_t* src, uint8_t* snk);
-__global__ void k_solve4(DevPool P, SolveParams prm);
-__global__ void k_solve5(DevPool P, SolveParams prm);
-__global__ void k_solve8(DevPool P, SolveParams prm);
+__global__ void k_solve(DevPool P, SolveParams prm);
 // kernels of cgc_batch.cu
 __global__ void k_put_all(DevPool P, const int32_t* const* __restrict__ in);
 __global__ void k_seg_all(DevPool P, uint8_t* const* __restrict__ out);

@@ -207,8 +207,8 @@ union TileShared {  // size a multiple of 16: the members are aligned
 struct SolveBook {
   unsigned long long tmark, t_launch, ns_bfs, ns_sweep, ns_reach, ns_sched;  // CTA 0
   int ntrace;                                                               // CTA 0
-  unsigned visits_sw[MAX_GROUPS], pulses[MAX_GROUPS], visits_bfs[MAX_GROUPS], visits_chk[MAX_GROUPS];
-  int next[2 * MAX_GROUPS];  // for_entries
+  unsigned visits_sw[GROUPS], pulses[GROUPS], visits_bfs[GROUPS], visits_chk[GROUPS];
+  int next[2 * GROUPS];  // for_entries
 };
 
 // a list entry, loaded ahead of the test that may discard it
@@ -231,7 +231,7 @@ __device__ __forceinline__ void solve_body(const DevPool& P, const SolveParams& 
   const int gw = b * (int)(blockDim.x >> 5) + (tid >> 5), nw = G * (int)(blockDim.x >> 5);
   uint32_t bar_target = 0;
   auto sync = [&]() { return grid_barrier(P.bar, bar_target, prm.limit_ns); };
-  if (tid < MAX_GROUPS) book.visits_sw[tid] = book.pulses[tid] = book.visits_bfs[tid] = book.visits_chk[tid] = 0;
+  if (tid < GROUPS) book.visits_sw[tid] = book.pulses[tid] = book.visits_bfs[tid] = book.visits_chk[tid] = 0;
   if (tid == 0) {
     book.tmark = book.t_launch = globaltimer_ns();
     book.ns_bfs = book.ns_sweep = book.ns_reach = book.ns_sched = 0;
@@ -255,7 +255,7 @@ __device__ __forceinline__ void solve_body(const DevPool& P, const SolveParams& 
     int32_t* take = P.cnt + C_TAKE0 + round_no % 3;
     if (b == 0 && tid == 0) P.cnt[C_TAKE0 + (round_no + 1) % 3] = 0;
     ++round_no;
-    const int first = G * (int)(blockDim.x / GROUP);
+    const int first = G * GROUPS;
     int i = grp * G + b, j = 2 * grp;
     while (i < n) {
       int nx = 0;
@@ -301,7 +301,29 @@ __device__ __forceinline__ void solve_body(const DevPool& P, const SolveParams& 
       const int n = ld_cnt(k == 0 ? cnt0 : bc + k % 3);
       if (n == 0) break;
       if (b == 0 && tid == 0) bc[(k + 2) % 3] = 0;
-      if (inval) {
+      // More than a tile per SM: a warp per tile; else the group's shorter
+      // chains win (all relabels, 405x377x362: 2.48 ms with groups alone, 1.63;
+      // 150x140x96 segmentation: 4.2, 3.0; thresholds of 2, 4, 8 tiles: 3.0,
+      // 3.1, 3.4; of 0, 64^3 balls: 0.112 -> 0.118 ms).
+      if (n > G) {
+        const int nn = CGC_IN_BOUNDS(P, n, P.T + 1) ? n : P.T;
+        int32_t* take = P.cnt + C_TAKE0 + round_no % 3;  // handed out as in for_entries
+        if (b == 0 && tid == 0) P.cnt[C_TAKE0 + (round_no + 1) % 3] = 0;
+        ++round_no;
+        unsigned short* const g = reinterpret_cast<unsigned short*>(groups) + (tid >> 5) * WREL_SMEM;
+        int32_t* const ln = list((k + 1) % 3);
+        int32_t* const cn = bc + (k + 1) % 3;
+        int visits = 0;
+        for (int i = (tid >> 5) * G + b; i < nn;) {
+          int nx = 0;
+          if ((tid & 31) == 0) nx = atomicAdd(take, 1);
+          const int t = __ldcg(lst + i);
+          visits += inval ? relabel_tile_w<true>(P, t, g, bfs_id + k + 1, ln, cn, (uint32_t)(relabels + 1), list(3), P.cnt + C_INC)
+                          : relabel_tile_w<false>(P, t, g, bfs_id + k + 1, ln, cn, 0u, nullptr, nullptr);
+          i = nw + __shfl_sync(FULL, nx, 0);
+        }
+        if ((tid & 31) == 0) atomicAdd(inval ? &book.visits_chk[grp] : &book.visits_bfs[grp], (unsigned)visits);
+      } else if (inval) {
         for_entries(lst, t0, n, [&](int t) {
           const int v = inval_tile(P, tg, t, S.bfs, bfs_id + k + 1, list((k + 1) % 3), bc + (k + 1) % 3,
                                    (uint32_t)(relabels + 1), list(3), P.cnt + C_INC);
@@ -396,7 +418,7 @@ __device__ __forceinline__ void solve_body(const DevPool& P, const SolveParams& 
     // order.  Budgets can still shorten that visit, so learned = 3 runs the
     // stage in every cycle, with each tile's budget capped at the schedule's L
     // (a budget may only end a visit early).
-    const bool throughput = nact > 2 * G * (int)(blockDim.x / GROUP);
+    const bool throughput = nact > 2 * G * GROUPS;
     const bool learned = prm.learned && (throughput || prm.learned == 3);
     if (learned || tracing) {
       if (!sched_stage(P, prm, cycle, learned, tracing, list(3 + (s & 3)), ld_cnt(sc + (s & 3)), list(3 + ((s + 1) & 3)),
@@ -543,19 +565,16 @@ int coop_launch_ordered(int device, cudaStream_t stream, const std::function<int
   return CGC_OK;
 }
 
-// Tile groups per SM.  More groups hide more latency while tiles are plenty
-// (512x512x128 tubes, sweeps: 4.2 ms at 4 groups, 3.8 at 5, 3.7 at 8); fewer
-// leave each visit more registers and issue slots, which the tail of a solve
-// wants (256^3 balls, kernel: 5.1, 5.2, 5.8 ms).
-static int solve_groups(const cgc_options& o) { return o.ctas_per_sm == 4 ? 8 : o.ctas_per_sm == 3 ? 5 : 4; }
-
-static void (*solve_kernel(int groups))(DevPool, SolveParams) {
-  return groups == 8 ? k_solve8 : groups == 5 ? k_solve5 : k_solve4;
+// One CTA of GROUPS tile groups per SM, 128 registers per thread.  Five groups
+// (96 registers) and eight (64) spill in the sweep: 256^3 balls 3.9 -> 4.2 and
+// 4.8 ms, 48-instance batch 5.9 -> 6.4 and 7.2 ms; only the tubes, all short
+// visits, gain 3 % (5.06 -> 4.90 ms at L = 4, R = 2).
+extern __shared__ __align__(16) unsigned char solve_smem[];
+__global__ void __launch_bounds__(GROUPS * GROUP, 1) k_solve(DevPool P, SolveParams prm) {
+  solve_body(P, prm, reinterpret_cast<TileShared*>(solve_smem));
 }
 
-int launch_solve(const DevPool& d, const cgc_options& o, const SolveParams& prm, int device, int sms, cudaStream_t stream) {
-  const int groups = solve_groups(o);
-  auto* kernel = solve_kernel(groups);
+int launch_solve(const DevPool& d, const SolveParams& prm, int device, int sms, cudaStream_t stream) {
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
@@ -564,35 +583,21 @@ int launch_solve(const DevPool& d, const cgc_options& o, const SolveParams& prm,
   cfg.numAttrs = 1;
   cfg.stream = stream;
   cfg.gridDim = dim3(sms);
-  cfg.blockDim = dim3(groups * GROUP);
-  cfg.dynamicSmemBytes = groups * sizeof(TileShared);
+  cfg.blockDim = dim3(GROUPS * GROUP);
+  cfg.dynamicSmemBytes = GROUPS * sizeof(TileShared);
   // a property of the function on the current device, set before its first launch there
-  static std::atomic<bool> done[64][3] = {};
-  const int which = groups == 8 ? 2 : groups == 5 ? 1 : 0;
-  if (device < 0 || device >= 64 || !done[device][which].load(std::memory_order_acquire)) {
-    CGC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes));
-    if (device >= 0 && device < 64) done[device][which].store(true, std::memory_order_release);
+  static std::atomic<bool> done[64] = {};
+  if (device < 0 || device >= 64 || !done[device].load(std::memory_order_acquire)) {
+    CGC_CUDA(cudaFuncSetAttribute(k_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes));
+    if (device >= 0 && device < 64) done[device].store(true, std::memory_order_release);
   }
   int rc = coop_launch_ordered(device, stream, [&]() -> int {
-    CGC_CUDA(cudaLaunchKernelEx(&cfg, kernel, d, prm));
+    CGC_CUDA(cudaLaunchKernelEx(&cfg, k_solve, d, prm));
     return CGC_OK;
   });
   if (rc) return rc;
   note_launch();
   return ok();
-}
-
-// The solve kernel with 4, 5 or 8 tile groups per SM (128, 96 and 64 registers
-// per thread).
-extern __shared__ __align__(16) unsigned char solve_smem[];
-__global__ void __launch_bounds__(4 * GROUP, 1) k_solve4(DevPool P, SolveParams prm) {
-  solve_body(P, prm, reinterpret_cast<TileShared*>(solve_smem));
-}
-__global__ void __launch_bounds__(5 * GROUP, 1) k_solve5(DevPool P, SolveParams prm) {
-  solve_body(P, prm, reinterpret_cast<TileShared*>(solve_smem));
-}
-__global__ void __launch_bounds__(8 * GROUP, 1) k_solve8(DevPool P, SolveParams prm) {
-  solve_body(P, prm, reinterpret_cast<TileShared*>(solve_smem));
 }
 
 // One cut set of an instance after a device-resident solve, any mask and
@@ -1079,7 +1084,7 @@ int pool_solve_async(Pool& p, const cgc_options* opts) {
   int rc = CGC_OK;
   if (o.persistent > 0) {
     CGC_CUDA(cudaEventRecord(p.ev[2], p.stream));
-    rc = launch_solve(d, o, prm, p.device, p.sms, p.stream);
+    rc = launch_solve(d, prm, p.device, p.sms, p.stream);
     CGC_CUDA(cudaEventRecord(p.ev[3], p.stream));
   } else {
     // the host loop reads counters back every round; a preparation error

@@ -127,9 +127,28 @@ __device__ __forceinline__ void ldcg4(const int32_t* p, int (&v)[4]) {
 }
 __device__ __forceinline__ int at(const int4& v, int k) { return k == 0 ? v.x : k == 1 ? v.y : k == 2 ? v.z : v.w; }
 
+// Heights as 16-bit numbers, two to a register, for the relaxations: a step
+// then issues half the instructions (they are bound by the integer pipe).  A
+// tile with a finite height above FAR16 around it uses 32-bit steps instead;
+// below, no path in the tile reaches INF16.
+constexpr int INF16 = 0x3fff, CLOSED16 = 0x4000, FAR16 = 15000;
+__device__ __forceinline__ unsigned pack16(int lo, int hi) {
+  return (unsigned)min(lo, INF16) | (unsigned)min(hi, INF16) << 16;
+}
+__device__ __forceinline__ void unpack16(unsigned v, int& lo, int& hi) {
+  lo = (int)(v & 0xffffu);
+  hi = (int)(v >> 16);
+  if (lo == INF16) lo = INF;
+  if (hi == INF16) hi = INF;
+}
+__device__ __forceinline__ bool far16(int h) { return h > FAR16 && h < INF; }
+
 // Halo of tile t: 64 threads each load half a y or z halo row into sh0 (and
-// sh1 if given), every thread returns its x halo height (INF outside the grid).
-__device__ __forceinline__ int load_halo_heights(const DevPool& P, const int t, const int q, int* sh0, int* sh1) {
+// sh1 if given) and, as 16-bit heights, into s16 (if given); every thread
+// returns its x halo height (INF outside the grid).  far: set if a height the
+// thread loaded does not fit 16 bits.
+__device__ __forceinline__ int load_halo_heights(const DevPool& P, const int t, const int q, int* sh0, int* sh1,
+                                                 unsigned short* s16, bool& far) {
   const int half = q & 1, k = (q >> 1) & 7;
   const int nx = __ldcg(P.nbr + (half ? PX : MX) * P.T + t);
   if (q < 64) {
@@ -141,8 +160,12 @@ __device__ __forceinline__ int load_halo_heights(const DevPool& P, const int t, 
     if (nt >= 0 && CGC_IN_BOUNDS(P, nt, P.T)) v = __ldcg(reinterpret_cast<const int4*>(P.h + (int64_t)nt * TV + src));
     *reinterpret_cast<int4*>(sh0 + dst) = v;
     if (sh1) *reinterpret_cast<int4*>(sh1 + dst) = v;
+    if (s16) *reinterpret_cast<uint2*>(s16 + dst) = make_uint2(pack16(v.x, v.y), pack16(v.z, v.w));
+    far = far || far16(v.x) || far16(v.y) || far16(v.z) || far16(v.w);
   }
-  return (nx >= 0 && CGC_IN_BOUNDS(P, nx, P.T)) ? __ldcg(P.h + (int64_t)nx * TV + 8 * (q >> 1) + (half ? 0 : 7)) : INF;
+  const int hx = (nx >= 0 && CGC_IN_BOUNDS(P, nx, P.T)) ? __ldcg(P.h + (int64_t)nx * TV + 8 * (q >> 1) + (half ? 0 : 7)) : INF;
+  far = far || far16(hx);
+  return hx;
 }
 
 // Cost of a closed edge in the relaxation: INF + CLOSED does not overflow, and
@@ -175,6 +198,32 @@ __device__ __forceinline__ bool relax_row(int* S, const int row, const int half,
 #pragma unroll
   for (int k = 0; k < 4; ++k) d[k] = n[k];
   if (ch) st4(S + row, d);
+  return ch;
+}
+
+// The same step on 16-bit heights: d[0] holds the row's first two voxels, d[1]
+// the others; c[dir][0..1] is 1 or CLOSED16 per half.
+__device__ __forceinline__ bool relax_row16(unsigned short* S, const int row, const int half, const unsigned hx,
+                                            unsigned (&d)[2], const unsigned (&c)[6][2]) {
+  const uint2 yp = *reinterpret_cast<const uint2*>(S + row + 8), ym = *reinterpret_cast<const uint2*>(S + row - 8);
+  const uint2 zp = *reinterpret_cast<const uint2*>(S + row + 80), zm = *reinterpret_cast<const uint2*>(S + row - 80);
+  const unsigned xo = __shfl_xor_sync(FULL, half ? d[0] : d[1], 1);  // the row's other half
+  const unsigned l = __byte_perm(half ? xo : hx, d[0], half ? 0x5432 : 0x5410);  // left neighbours of d[0]
+  unsigned n0 = __viaddmin_s16x2(yp.x, c[PY][0], d[0]), n1 = __viaddmin_s16x2(yp.y, c[PY][1], d[1]);
+  n0 = __viaddmin_s16x2(ym.x, c[MY][0], n0);
+  n1 = __viaddmin_s16x2(ym.y, c[MY][1], n1);
+  n0 = __viaddmin_s16x2(zp.x, c[PZ][0], n0);
+  n1 = __viaddmin_s16x2(zp.y, c[PZ][1], n1);
+  n0 = __viaddmin_s16x2(zm.x, c[MZ][0], n0);
+  n1 = __viaddmin_s16x2(zm.y, c[MZ][1], n1);
+  n0 = __viaddmin_s16x2(l, c[MX][0], n0);
+  n1 = __viaddmin_s16x2(__byte_perm(n0, n1, 0x5432), c[MX][1], n1);
+  n1 = __viaddmin_s16x2(__byte_perm(n1, half ? hx : xo, 0x5432), c[PX][1], n1);
+  n0 = __viaddmin_s16x2(__byte_perm(n0, n1, 0x5432), c[PX][0], n0);
+  const bool ch = ((n0 ^ d[0]) | (n1 ^ d[1])) != 0;
+  d[0] = n0;
+  d[1] = n1;
+  if (ch) *reinterpret_cast<uint2*>(S + row) = make_uint2(n0, n1);
   return ch;
 }
 
@@ -221,6 +270,7 @@ __device__ __forceinline__ long long block_sum64(long long v, long long* red) {
 // Shared state of one tile group.
 struct alignas(16) SweepShared {
   int h[2][HROWS * 8];  // heights, double buffered by pulse
+  unsigned short g[HROWS * 8];  // 16-bit heights of the region relabel
   int out[2][TV];       // flow pushed along +z / -z in this pulse; zero between pulses
   int facc[6][64];      // flow pushed out of the tile per face entry
   unsigned char face[8];  // faces that flow left through
@@ -229,6 +279,7 @@ struct alignas(16) SweepShared {
 
 struct alignas(16) BfsShared {
   int h[HROWS * 8];
+  unsigned short g[HROWS * 8];  // 16-bit heights
   unsigned char face[8];  // BFS / invalidation: faces whose heights changed
   unsigned char act;      // an excess voxel that reaches the sink
   unsigned char any;      // a voxel was dropped
@@ -271,7 +322,8 @@ __device__ __forceinline__ int sweep_tile(const DevPool& P, const TileGroup<GROU
 #pragma unroll
   for (int d = 0; d < 6; ++d) ldcg4(P.r + d * Np + g, r[d]);
   st4(S.h[0] + row, h);
-  const int hx = load_halo_heights(P, t, q, S.h[0], S.h[1]);
+  bool far = false;
+  const int hx = load_halo_heights(P, t, q, S.h[0], S.h[1], S.g, far);
   const int inst = __ldcg(P.tinst + t);
   const int hdead = P.geo[inst].hdead;
   {
@@ -282,7 +334,7 @@ __device__ __forceinline__ int sweep_tile(const DevPool& P, const TileGroup<GROU
   }
   if (q < 8) S.face[q] = 0;
   if (q == 0) S.lastout = 0;
-  if (R <= 0 || exact) tg.sync();  // the region relabel has its own
+  far = tg.any(far);
 
   // some voxel of the thread holds excess and may still reach the sink
   auto active = [&]() {
@@ -303,16 +355,35 @@ __device__ __forceinline__ int sweep_tile(const DevPool& P, const TileGroup<GROU
       int dd[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) dd[k] = rT[k] > 0 ? 1 : INF;
-      st4(S.h[cur] + row, dd);
-      int c[6][4];
+      // Bellman-Ford: < 512 steps in a tile
+      if (!far) {
+        unsigned d2[2] = {pack16(dd[0], dd[1]), pack16(dd[2], dd[3])}, c[6][2];
+        *reinterpret_cast<uint2*>(S.g + row) = make_uint2(d2[0], d2[1]);
 #pragma unroll
-      for (int d = 0; d < 6; ++d)
+        for (int d = 0; d < 6; ++d)
 #pragma unroll
-        for (int k = 0; k < 4; ++k) c[d][k] = r[d][k] > 0 ? 1 : CLOSED;
-      tg.sync();
-      for (int it = 0; it < 600; ++it) {  // Bellman-Ford: < 512 steps in a tile
-        const bool ch = relax_row(S.h[cur], row, half, hx, dd, c);
-        if (!tg.any(ch)) break;
+          for (int j = 0; j < 2; ++j)
+            c[d][j] = (r[d][2 * j] > 0 ? 1u : (unsigned)CLOSED16) | (r[d][2 * j + 1] > 0 ? 1u << 16 : (unsigned)CLOSED16 << 16);
+        const unsigned hx2 = pack16(hx, 0);
+        tg.sync();
+        for (int it = 0; it < 600; ++it) {
+          const bool ch = relax_row16(S.g, row, half, hx2, d2, c);
+          if (!tg.any(ch)) break;
+        }
+        unpack16(d2[0], dd[0], dd[1]);
+        unpack16(d2[1], dd[2], dd[3]);
+      } else {
+        st4(S.h[cur] + row, dd);
+        int c[6][4];
+#pragma unroll
+        for (int d = 0; d < 6; ++d)
+#pragma unroll
+          for (int k = 0; k < 4; ++k) c[d][k] = r[d][k] > 0 ? 1 : CLOSED;
+        tg.sync();
+        for (int it = 0; it < 600; ++it) {
+          const bool ch = relax_row(S.h[cur], row, half, hx, dd, c);
+          if (!tg.any(ch)) break;
+        }
       }
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
@@ -1182,39 +1253,64 @@ __device__ __forceinline__ int bfs_tile(const DevPool& P, const TileGroup<GROUP>
   int h[4];
   ldcg4(P.h + g, h);
   const unsigned m = __ldcg(reinterpret_cast<const unsigned*>(P.rmask + g));
-  const int hx = load_halo_heights(P, t, q, S.h, nullptr);
+  bool far = far16(h[0]) || far16(h[1]) || far16(h[2]) || far16(h[3]);
+  const int hx = load_halo_heights(P, t, q, S.h, nullptr, S.g, far);
   if (dead) return 0;  // uniform over the group; nothing can change
   const int nb = q >= 32 && q < 38 ? __ldcg(P.nbr + (q - 32) * P.T + t) : -1;  // face neighbour, for the re-queue
+  unsigned d2[2] = {pack16(h[0], h[1]), pack16(h[2], h[3])};
+  *reinterpret_cast<uint2*>(S.g + row) = make_uint2(d2[0], d2[1]);
   st4(S.h + row, h);
   if (q < 8) S.face[q] = 0;
   if (q == 8) S.act = 0;
-  tg.sync();
-  // faces the thread's voxels lie on: its own row end, y and z
-  const int fx = half ? PX : MX, kx = half ? 3 : 0;
+  far = tg.any(far);
+  // after a step that lowered the thread's row: the faces it lies on (the row
+  // end that moved, y and z)
   bool changed = false;
-  int c[6][4];
+  auto lowered = [&](bool end) {
+    changed = true;
+    if (end) S.face[half ? PX : MX] = 1;
+    if (y == 7) S.face[PY] = 1;
+    if (y == 0) S.face[MY] = 1;
+    if (z == 7) S.face[PZ] = 1;
+    if (z == 0) S.face[MZ] = 1;
+  };
+  // a voxel with excess that reaches the sink (heights never rise here)
+  const unsigned ex = (m >> 7) & 0x01010101u;
+  auto note_active = [&](bool a0, bool a1, bool a2, bool a3) {
+    if ((a0 && (ex & 1u)) || (a1 && (ex & 0x100u)) || (a2 && (ex & 0x10000u)) || (a3 && (ex & 0x1000000u))) S.act = 1;
+  };
+  if (!far) {
+    unsigned c[6][2];
 #pragma unroll
-  for (int d = 0; d < 6; ++d)
+    for (int d = 0; d < 6; ++d)
 #pragma unroll
-    for (int k = 0; k < 4; ++k) c[d][k] = ((m >> (8 * k + d)) & 1u) ? 1 : CLOSED;
-  for (int it = 0; it < 1024; ++it) {  // converges in < 512 steps (path length in a tile)
-    const int hxe = kx ? h[3] : h[0];
-    const bool ch = relax_row(S.h, row, half, hx, h, c);
-    if (ch) {
-      changed = true;
-      if ((kx ? h[3] : h[0]) < hxe) S.face[fx] = 1;
-      if (y == 7) S.face[PY] = 1;
-      if (y == 0) S.face[MY] = 1;
-      if (z == 7) S.face[PZ] = 1;
-      if (z == 0) S.face[MZ] = 1;
+      for (int j = 0; j < 2; ++j)
+        c[d][j] = (((m >> (16 * j + d)) & 1u) ? 1u : (unsigned)CLOSED16) |
+                  (((m >> (16 * j + 8 + d)) & 1u) ? 1u << 16 : (unsigned)CLOSED16 << 16);
+    const unsigned hx2 = pack16(hx, 0);
+    for (int it = 0; it < 1024; ++it) {  // converges in < 512 steps (path length in a tile)
+      const unsigned e0 = half ? d2[1] >> 16 : d2[0] & 0xffffu;
+      const bool ch = relax_row16(S.g, row, half, hx2, d2, c);
+      if (ch) lowered((half ? d2[1] >> 16 : d2[0] & 0xffffu) != e0);
+      if ((it == 0 || ch) && ex)
+        note_active((d2[0] & 0xffffu) < INF16, (d2[0] >> 16) < INF16, (d2[1] & 0xffffu) < INF16, (d2[1] >> 16) < INF16);
+      if (!tg.any(ch)) break;
     }
-    if (it == 0 || ch) {
-      bool act = false;
+    unpack16(d2[0], h[0], h[1]);
+    unpack16(d2[1], h[2], h[3]);
+  } else {
+    int c[6][4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) act = act || (((m >> (8 * k + 7)) & 1u) && h[k] < INF);
-      if (act) S.act = 1;
+    for (int d = 0; d < 6; ++d)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) c[d][k] = ((m >> (8 * k + d)) & 1u) ? 1 : CLOSED;
+    for (int it = 0; it < 1024; ++it) {
+      const int e0 = half ? h[3] : h[0];
+      const bool ch = relax_row(S.h, row, half, hx, h, c);
+      if (ch) lowered((half ? h[3] : h[0]) < e0);
+      if ((it == 0 || ch) && ex) note_active(h[0] < INF, h[1] < INF, h[2] < INF, h[3] < INF);
+      if (!tg.any(ch)) break;
     }
-    if (!tg.any(ch)) break;
   }
   if (q >= 32 && q < 38 && S.face[q - 32] && nb >= 0) queue_tile(P, P.stamp_bfs, nb, id_next, list_next, cnt_next);
   if (changed) st4(P.h + g, h);
@@ -1279,7 +1375,8 @@ __device__ __forceinline__ int inval_tile(const DevPool& P, const TileGroup<GROU
   int h[4];
   ldcg4(P.h + g, h);
   const unsigned m = __ldcg(reinterpret_cast<const unsigned*>(P.rmask + g));
-  const int hx = load_halo_heights(P, t, q, S.h, nullptr);
+  bool far = false;
+  const int hx = load_halo_heights(P, t, q, S.h, nullptr, nullptr, far);
   const int nb = q >= 32 && q < 38 ? __ldcg(P.nbr + (q - 32) * P.T + t) : -1;  // face neighbour, for the re-queue
   st4(S.h + row, h);
   if (q < 8) S.face[q] = 0;

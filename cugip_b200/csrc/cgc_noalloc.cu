@@ -198,7 +198,7 @@ extern "C" int cgc_grid_maxflow_noalloc(int32_t X, int32_t Y, int32_t Z, const i
   const SolveParams prm = solve_params(o);
   // a preparation error (overflowing capacities) makes every CTA leave at its
   // first barrier
-  if ((rc = launch_solve(P, o, prm, dev, su->sms, st))) return rc;
+  if ((rc = launch_solve(P, prm, dev, su->sms, st))) return rc;
   if (source_side || sink_side) {
     k_seg_one<<<(unsigned)((G.hdead + 4094) / 4096), 256, 0, st>>>(P, source_side, sink_side);
     NA_CUDA(cudaGetLastError());

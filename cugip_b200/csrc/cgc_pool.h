@@ -144,8 +144,8 @@ int pool_solve_wait(Pool& p);
 // runs `launch` (a cooperative launch into `stream`) after every earlier
 // cooperative launch of this library on the device has ended
 int coop_launch_ordered(int device, cudaStream_t stream, const std::function<int()>& launch);
-// cooperative launch of the persistent solve kernel selected by the options
-int launch_solve(const DevPool& d, const cgc_options& o, const SolveParams& prm, int device, int sms, cudaStream_t stream);
+// cooperative launch of the persistent solve kernel
+int launch_solve(const DevPool& d, const SolveParams& prm, int device, int sms, cudaStream_t stream);
 int pool_segments(Pool& p, int inst, int which, uint8_t* out, uint8_t mask, uint8_t bg, bool host);
 int pool_residuals(Pool& p, int inst, int32_t* const res[6], int32_t* resT, int32_t* excess);
 int pool_trace(Pool& p, int64_t* out, int32_t cap, int32_t* count);

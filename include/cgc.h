@@ -73,14 +73,14 @@ typedef struct cgc_options {
   int32_t persistent;         /* 1 = one cooperative launch per solve (default), -1 = host loop */
   int32_t region_relabels;    /* region-relabel rounds per tile visit (default 2, -1 = none) */
   int32_t stall_sweeps;       /* persistent: relabel early after this many sweep pairs without sink flow (0 = never) */
-  int32_t ctas_per_sm;        /* persistent: 2 (default), 3 or 4: tiles an SM works on at a time, in 128-thread
-                                 groups (4, 5 or 8 of them at 128, 96 or 64 registers per thread) */
+  int32_t ctas_per_sm;        /* accepted and without effect: the solve runs one CTA of four 128-thread tile groups
+                                 per SM, which is the fastest shape for every workload this selected between */
   int32_t learned;            /* persistent: learned scheduler, 1 = budgets + priorities, 2 = budgets only
                                  (both only in cycles with more active tiles than twice the CTAs), 3 = budgets
                                  capped at local_pulses in every cycle + priorities where 1 uses them */
   int32_t trace_cycles;       /* persistent: record scheduling traces of the first trace_cycles relabel cycles */
   int32_t bfs_warp_min;       /* accepted and without effect: BFS rounds visit a tile with a 128-thread group,
-                                 which is faster at every round size than the warp per tile this selected */
+                                 or, where tiles outnumber the SMs, with a warp */
   int32_t exclusive;          /* persistent: 1 = every sweep visits each queued tile, except a tile that has a
                                  face neighbour of the sweep's parity queued for the same sweep (which waits one
                                  sweep); 0 = checkerboard sweeps, one parity at a time (the default) */

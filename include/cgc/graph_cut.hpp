@@ -57,7 +57,7 @@ struct GraphCutPolicy {
   int wait_limit_us = 0;       // bound of every device-side wait in microseconds (0: 20 s)
   int max_sweeps = 0;          // safety cap (0: default)
   int stall_sweeps = 0;        // relabel early after this many idle sweep pairs (0: never)
-  int ctas_per_sm = 0;         // 2 (default), 3 or 4: tiles per SM (cgc.h)
+  int ctas_per_sm = 0;         // accepted, without effect (cgc.h)
   int learned = 0;             // learned scheduler: 1 budgets + priorities, 2 budgets only
   int bfs_warp_min = 0;        // accepted, without effect (cgc.h)
   int exclusive = 0;           // 1: sweeps visit every queued tile without a queued face neighbour of the sweep's parity
