@@ -405,6 +405,18 @@ __device__ __forceinline__ void solve_body(const DevPool& P, const SolveParams& 
       P.trace[2 * i + 1] = f;
     }
     if (nact == 0) break;
+    // Sweep pairs of this cycle.  Where a sweep costs more than a relabel -- more
+    // than 16 active tiles per SM -- a cycle ends after 4 pairs at the latest,
+    // since by then most tiles hold excess that a relabel finds cut off from the
+    // sink: 405x377x362 8.9 -> 8.0 ms, 512x512x128 tubes 3.6 -> 3.3, 256^3 3.13
+    // -> 3.05, segmentation of 150x140x96 9.1 -> 8.9 (K = 8).  2 pairs are better
+    // on balls (7.6 ms) and worse on the segmentation (10.0 ms), whose relabels
+    // take long; lower limits on the tiles cost small grids 10 %.
+    // A cycle in which the limit on sweeps may be met is a full one, so that a
+    // small limit allows the sweeps that it always did.
+    const bool cut = nact > 16 * G && prm.K > 4 &&
+                     sweeps + 2 * prm.K < (int64_t)prm.max_sweeps;
+    const int K = cut ? 4 : prm.K;
     if (sweeps >= prm.max_sweeps) {
       if (b == 0 && tid == 0) raise_error(P, CGC_ERR_NOT_CONVERGED);
       break;
@@ -428,7 +440,7 @@ __device__ __forceinline__ void solve_body(const DevPool& P, const SolveParams& 
     }
     // ------------------------------------------------ sweeps
     int idle = 0;  // consecutive sweeps in which no tile delivered flow to the sink
-    for (int j = 0; j < 2 * prm.K; ++j, ++s) {
+    for (int j = 0; j < 2 * K; ++j, ++s) {
       const int32_t* const lst = list(3 + (s & 3));
       const int t0 = first_entry(lst), tw = b < P.T ? ld_ahead(lst + b) : 0;
       const int n = ld_cnt(sc + (s & 3));
@@ -451,7 +463,7 @@ __device__ __forceinline__ void solve_body(const DevPool& P, const SolveParams& 
         const int sn = s + 1, ss = prm.exclusive ? s + 1 : s + 2;  // the sweeps the neighbours and the tile queue for
         // the learned scheduler defers low-priority tiles during the first half
         // of the cycle; every active tile is swept in the second half
-        if (learned && throughput && prm.learned != 2 && j < prm.K && !__ldcg(P.sprio + t)) {
+        if (learned && throughput && prm.learned != 2 && j < K && !__ldcg(P.sprio + t)) {
           if (vg.q == 0) queue_tile(P, stamp_q, t, (uint32_t)(ss + 1), list(3 + (ss & 3)), sc + (ss & 3));
           return;
         }
