@@ -301,11 +301,12 @@ __device__ __forceinline__ void solve_body(const DevPool& P, const SolveParams& 
       const int n = ld_cnt(k == 0 ? cnt0 : bc + k % 3);
       if (n == 0) break;
       if (b == 0 && tid == 0) bc[(k + 2) % 3] = 0;
-      // More than a tile per SM: a warp per tile; else the group's shorter
-      // chains win (all relabels, 405x377x362: 2.48 ms with groups alone, 1.63;
-      // 150x140x96 segmentation: 4.2, 3.0; thresholds of 2, 4, 8 tiles: 3.0,
-      // 3.1, 3.4; of 0, 64^3 balls: 0.112 -> 0.118 ms).
-      if (n > G) {
+      // More tiles than groups: a warp per tile; else the groups' shorter steps
+      // win (relabels of a 150x140x96 segmentation with a warp from more than 1,
+      // 2, 3, 4 tiles per SM on: 4.19, 4.09, 4.03, 3.89 ms; of a batch of 160^3:
+      // 1.69, 1.68, 1.67, 1.61.  Without warp visits the segmentation's solve
+      // took 10.3 ms, with them 9.1).
+      if (n > GROUPS * G) {
         const int nn = CGC_IN_BOUNDS(P, n, P.T + 1) ? n : P.T;
         int32_t* take = P.cnt + C_TAKE0 + round_no % 3;  // handed out as in for_entries
         if (b == 0 && tid == 0) P.cnt[C_TAKE0 + (round_no + 1) % 3] = 0;

@@ -280,9 +280,7 @@ struct alignas(16) SweepShared {
 struct alignas(16) BfsShared {
   int h[HROWS * 8];
   unsigned short g[HROWS * 8];  // 16-bit heights
-  unsigned char face[8];  // BFS / invalidation: faces whose heights changed
-  unsigned char act;      // an excess voxel that reaches the sink
-  unsigned char any;      // a voxel was dropped
+  unsigned flags;  // of the visit: faces whose heights changed (bits 0..5), and bit 6 (bfs_tile, inval_tile)
 };
 
 // optional per-visit bookkeeping of the persistent schedule
@@ -1238,11 +1236,21 @@ __device__ __forceinline__ void bfs_queue_tile(const DevPool& P, const int t, co
   warp_append(P, q, t, list0, cnt0);
 }
 
+// faces that a changed half row lies on, as bits (end: its voxel on the x face changed)
+__device__ __forceinline__ unsigned row_faces(int half, int y, int z, bool end) {
+  return (end ? 1u << (half ? PX : MX) : 0u) | (y == 7 ? 1u << PY : 0u) | (y == 0 ? 1u << MY : 0u) |
+         (z == 7 ? 1u << PZ : 0u) | (z == 0 ? 1u << MZ : 0u);
+}
+
 // One BFS visit: relax h(v) = min(h(v), 1 + h(u)) over residual edges v->u
-// until the tile is stable; re-queue face neighbours whose halo changed.  The
-// face and activity flags are set as heights drop (they never rise again), so
-// the barrier that ends the relaxation also publishes them.  The caller
-// synchronises the group before S is used again; returns 1 for a visited tile.
+// until the tile is stable; re-queue face neighbours whose halo changed.  What
+// changed, and whether an excess voxel reaches the sink, is read off the heights
+// once the relaxation has ended, and two steps share a barrier: a step is bound
+// by its own chain of latencies, and a round by the visit with the most steps
+// (about 20 where the mean is 5).  All relabels of a 256^3 solve: 0.83 -> 0.69
+// ms, of a 150x140x96 segmentation 4.4 -> 3.8 (flags set as heights drop, a
+// barrier per step).  The caller synchronises the group before S is used again;
+// returns 1 for a visited tile.
 __device__ __forceinline__ int bfs_tile(const DevPool& P, const TileGroup<GROUP> tg, const int t, BfsShared& S,
                                         const uint32_t id_next, int32_t* list_next, int32_t* cnt_next) {
   if (!CGC_IN_BOUNDS(P, t, P.T)) return 0;  // uniform over the group
@@ -1260,26 +1268,11 @@ __device__ __forceinline__ int bfs_tile(const DevPool& P, const TileGroup<GROUP>
   unsigned d2[2] = {pack16(h[0], h[1]), pack16(h[2], h[3])};
   *reinterpret_cast<uint2*>(S.g + row) = make_uint2(d2[0], d2[1]);
   st4(S.h + row, h);
-  if (q < 8) S.face[q] = 0;
-  if (q == 8) S.act = 0;
+  if (q == 0) S.flags = 0;
   far = tg.any(far);
-  // after a step that lowered the thread's row: the faces it lies on (the row
-  // end that moved, y and z)
-  bool changed = false;
-  auto lowered = [&](bool end) {
-    changed = true;
-    if (end) S.face[half ? PX : MX] = 1;
-    if (y == 7) S.face[PY] = 1;
-    if (y == 0) S.face[MY] = 1;
-    if (z == 7) S.face[PZ] = 1;
-    if (z == 0) S.face[MZ] = 1;
-  };
-  // a voxel with excess that reaches the sink (heights never rise here)
-  const unsigned ex = (m >> 7) & 0x01010101u;
-  auto note_active = [&](bool a0, bool a1, bool a2, bool a3) {
-    if ((a0 && (ex & 1u)) || (a1 && (ex & 0x100u)) || (a2 && (ex & 0x10000u)) || (a3 && (ex & 0x1000000u))) S.act = 1;
-  };
+  bool changed, end;  // a voxel of the row dropped, and the one on the tile's x face
   if (!far) {
+    const unsigned w0 = d2[0], w1 = d2[1];
     unsigned c[6][2];
 #pragma unroll
     for (int d = 0; d < 6; ++d)
@@ -1289,32 +1282,44 @@ __device__ __forceinline__ int bfs_tile(const DevPool& P, const TileGroup<GROUP>
                   (((m >> (16 * j + 8 + d)) & 1u) ? 1u << 16 : (unsigned)CLOSED16 << 16);
     const unsigned hx2 = pack16(hx, 0);
     for (int it = 0; it < 1024; ++it) {  // converges in < 512 steps (path length in a tile)
-      const unsigned e0 = half ? d2[1] >> 16 : d2[0] & 0xffffu;
-      const bool ch = relax_row16(S.g, row, half, hx2, d2, c);
-      if (ch) lowered((half ? d2[1] >> 16 : d2[0] & 0xffffu) != e0);
-      if ((it == 0 || ch) && ex)
-        note_active((d2[0] & 0xffffu) < INF16, (d2[0] >> 16) < INF16, (d2[1] & 0xffffu) < INF16, (d2[1] >> 16) < INF16);
+      bool ch = relax_row16(S.g, row, half, hx2, d2, c);
+      __syncwarp();
+      ch = relax_row16(S.g, row, half, hx2, d2, c) || ch;
       if (!tg.any(ch)) break;
     }
+    changed = d2[0] != w0 || d2[1] != w1;
+    end = half ? ((d2[1] ^ w1) >> 16) != 0 : ((d2[0] ^ w0) & 0xffffu) != 0;
     unpack16(d2[0], h[0], h[1]);
     unpack16(d2[1], h[2], h[3]);
   } else {
+    const int4 was = make_int4(h[0], h[1], h[2], h[3]);
     int c[6][4];
 #pragma unroll
     for (int d = 0; d < 6; ++d)
 #pragma unroll
       for (int k = 0; k < 4; ++k) c[d][k] = ((m >> (8 * k + d)) & 1u) ? 1 : CLOSED;
     for (int it = 0; it < 1024; ++it) {
-      const int e0 = half ? h[3] : h[0];
       const bool ch = relax_row(S.h, row, half, hx, h, c);
-      if (ch) lowered((half ? h[3] : h[0]) < e0);
-      if ((it == 0 || ch) && ex) note_active(h[0] < INF, h[1] < INF, h[2] < INF, h[3] < INF);
       if (!tg.any(ch)) break;
     }
+    changed = h[0] != was.x || h[1] != was.y || h[2] != was.z || h[3] != was.w;
+    end = half ? h[3] != was.w : h[0] != was.x;
   }
-  if (q >= 32 && q < 38 && S.face[q - 32] && nb >= 0) queue_tile(P, P.stamp_bfs, nb, id_next, list_next, cnt_next);
+  // faces whose voxels changed (bits 0..5) and, in bit 6, an excess voxel that
+  // reaches the sink
+  unsigned flags = 0;
+  if (changed) flags = row_faces(half, y, z, end);
+  if (((m & 0x80u) && h[0] < INF) || ((m & 0x8000u) && h[1] < INF) || ((m & 0x800000u) && h[2] < INF) ||
+      ((m & 0x80000000u) && h[3] < INF))
+    flags |= 64u;
+  flags = __reduce_or_sync(FULL, flags);
+  if ((q & 31) == 0 && flags) atomicOr(&S.flags, flags);
+  tg.sync();
+  flags = S.flags;
+  if (q >= 32 && q < 38 && ((flags >> (q - 32)) & 1u) && nb >= 0)
+    queue_tile(P, P.stamp_bfs, nb, id_next, list_next, cnt_next);
   if (changed) st4(P.h + g, h);
-  if (q == 0) P.act[t] = S.act;  // heights only drop in later visits: the last visit's value is final
+  if (q == 0) P.act[t] = (uint8_t)((flags >> 6) & 1u);  // heights only drop in later visits: the last visit's value is final
   return 1;
 }
 
@@ -1379,10 +1384,9 @@ __device__ __forceinline__ int inval_tile(const DevPool& P, const TileGroup<GROU
   const int hx = load_halo_heights(P, t, q, S.h, nullptr, nullptr, far);
   const int nb = q >= 32 && q < 38 ? __ldcg(P.nbr + (q - 32) * P.T + t) : -1;  // face neighbour, for the re-queue
   st4(S.h + row, h);
-  if (q < 8) S.face[q] = 0;
-  if (q == 8) S.any = 0;
+  if (q == 0) S.flags = 0;
   tg.sync();
-  bool dropped = false;
+  unsigned drop = 0;  // bit k: voxel k was dropped
   for (int it = 0; it < 1024; ++it) {  // a drop per step climbs one height: < 512 steps in a tile
     const int4 yp = ld4(S.h + row + 8), ym = ld4(S.h + row - 8), zp = ld4(S.h + row + 80), zm = ld4(S.h + row - 80);
     const int xo = __shfl_xor_sync(FULL, half ? h[0] : h[3], 1);
@@ -1399,23 +1403,22 @@ __device__ __forceinline__ int inval_tile(const DevPool& P, const TileGroup<GROU
       if (h[k] < INF && !sup) {
         h[k] = INF;
         ch = true;
-        if (k == (half ? 3 : 0)) S.face[half ? PX : MX] = 1;
+        drop |= 1u << k;
       }
     }
-    if (ch) {
-      st4(S.h + row, h);
-      dropped = true;
-      S.any = 1;
-      if (y == 7) S.face[PY] = 1;
-      if (y == 0) S.face[MY] = 1;
-      if (z == 7) S.face[PZ] = 1;
-      if (z == 0) S.face[MZ] = 1;
-    }
+    if (ch) st4(S.h + row, h);
     if (!tg.any(ch)) break;
   }
-  if (q == 0 && S.any) queue_tile(P, P.stamp_inc, t, id_bfs, list_bfs, cnt_bfs);
-  if (q >= 32 && q < 38 && S.face[q - 32] && nb >= 0) queue_tile(P, P.stamp_bfs, nb, id_next, list_next, cnt_next);
-  if (dropped) st4(P.h + g, h);
+  unsigned flags = 0;  // faces that voxels were dropped on (bits 0..5), any drop (bit 6)
+  if (drop) flags = 64u | row_faces(half, y, z, (drop >> (half ? 3 : 0)) & 1u);
+  flags = __reduce_or_sync(FULL, flags);
+  if ((q & 31) == 0 && flags) atomicOr(&S.flags, flags);
+  tg.sync();
+  flags = S.flags;
+  if (q == 0 && (flags & 64u)) queue_tile(P, P.stamp_inc, t, id_bfs, list_bfs, cnt_bfs);
+  if (q >= 32 && q < 38 && ((flags >> (q - 32)) & 1u) && nb >= 0)
+    queue_tile(P, P.stamp_bfs, nb, id_next, list_next, cnt_next);
+  if (drop) st4(P.h + g, h);
   return 1;
 }
 

@@ -1,6 +1,7 @@
-"""Tile visits of the persistent solve where the dispatch changes: sweeps and
-relabel rounds of at most / more than one tile per SM (512-thread, 128-thread
-and warp visits), several rounds per group, and heights on both sides of the
+"""Tile visits of the persistent solve where the dispatch changes: sweeps of at
+most / more than one tile per SM (512-thread and 128-thread visits), relabel
+rounds of at most / more than one tile per group (128-thread and warp visits),
+several rounds per group, and heights on both sides of the
 16-bit relaxations' range.  Flow and both cut sets against the oracle."""
 import numpy as np
 import pytest
