@@ -499,9 +499,11 @@ __device__ __forceinline__ void solve_body(const DevPool& P, const SolveParams& 
           book.pulses[grp] += (unsigned)np;
         }
       };
-      // At most one tile per SM: 512 threads per visit.  A visit then lasts
-      // about 12k cycles instead of 18k (256^3 tail); with two tiles per SM one
-      // after the other it gains nothing over two groups side by side.
+      // At most one tile per SM: 512 threads per visit, which shortens a visit's
+      // own chain (kernel times with groups alone and so: 128^3 1.03 and 0.94 ms,
+      // 640x480 0.47 and 0.44, segmentation 8.45 and 8.34; the 160^3 batch 5.64
+      // and 5.86).  With two tiles per SM, one after the other, it gains nothing
+      // over two groups side by side (128^3 0.97, 256^3 2.94 -> 3.07, batch 6.16).
       if (n <= G) {
         const auto wide = TileGroup<WIDE>::of_thread();
         if (tid < WIDE && b < n) sweep_visit(wide, *reinterpret_cast<WideShared*>(groups), tw);

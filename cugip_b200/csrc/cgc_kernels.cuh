@@ -937,14 +937,16 @@ __device__ __forceinline__ int sweep_tile_wide(const DevPool& P, const TileGroup
 // which are contiguous there); the neighbour values come from registers (z),
 // the next lane (x) or the L1 (y).
 //   A4: plane rows of four voxels are 16-byte aligned (aligned planes, X a
-//   multiple of 4); otherwise a row is the two aligned vectors that cover it,
-//   or scalars.  SAME: symmetric n-links, one plane per axis.
+//   multiple of 4); otherwise a row is four scalars, all of a step's loads in
+//   flight at once (the two aligned vectors that cover it, with a branch at the
+//   plane's end, took 405x377x362 1.13 ms with both masks, scalars 0.81; without
+//   the branch 0.90).  SAME: symmetric n-links, one plane per axis.
 //   two_halves: the pool keeps both halves of stamp_sw.
 // 512x512x128: 0.75 -> 0.29 ms, 6.3 TB/s (before: a CTA per tile, eight planes read, 64-bit
-// checks per voxel); 405x377x362, whose rows are not aligned, with both masks: 2.0 -> 1.1 ms.
+// checks per voxel); 405x377x362, whose rows are not aligned, with both masks: 2.0 -> 0.81 ms.
 template <bool A4, bool SAME>
 __device__ __forceinline__ void put_run_as(const DevPool& P, const int t0, const int32_t* const* ip, const InstGeo& G,
-                                           const int inst, const bool vec, const bool two_halves) {
+                                           const int inst, const bool two_halves) {
   __shared__ long long red[4];
   const int lt = t0 - G.tile_base;
   const int rows = lt / G.TX, tx0 = lt - rows * G.TX, tz = rows / G.TY, ty = rows - tz * G.TY;
@@ -964,18 +966,9 @@ __device__ __forceinline__ void put_run_as(const DevPool& P, const int t0, const
       const int4 w = __ldg(reinterpret_cast<const int4*>(p + v));
       o[0] = w.x; o[1] = w.y; o[2] = w.z; o[3] = w.w;
     } else {
-      const int m = (int)(v & 3);
-      const int64_t a = v - m;
-      if (vec && a + (m ? 8 : 4) <= N) {
-        const int4 A = __ldg(reinterpret_cast<const int4*>(p + a));
-        const int4 B = m ? __ldg(reinterpret_cast<const int4*>(p + a + 4)) : A;
-        const int w[8] = {A.x, A.y, A.z, A.w, B.x, B.y, B.z, B.w};
+      const int lim = (int)min((int64_t)3, N - 1 - v);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) o[k] = m == 0 ? w[k] : m == 1 ? w[k + 1] : m == 2 ? w[k + 2] : w[k + 3];
-      } else {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) o[k] = p[v + k < N ? v + k : v];
-      }
+      for (int k = 0; k < 4; ++k) o[k] = __ldg(p + v + min(k, lim));
     }
   };
   bool neg = false, bad = false;
@@ -1115,11 +1108,11 @@ __device__ __forceinline__ void put_run(const DevPool& P, const int t0, const in
   for (int a = 0; a < 8; ++a) align |= reinterpret_cast<uintptr_t>(ip[a]);
 #pragma unroll
   for (int a = 0; a < 3; ++a) same = same && ip[2 + a] == ip[5 + a];
-  const bool vec = (align & 15) == 0, a4 = vec && (G.X & 3) == 0;
-  if (a4 && same) put_run_as<true, true>(P, t0, ip, G, inst, vec, two_halves);
-  else if (a4) put_run_as<true, false>(P, t0, ip, G, inst, vec, two_halves);
-  else if (same) put_run_as<false, true>(P, t0, ip, G, inst, vec, two_halves);
-  else put_run_as<false, false>(P, t0, ip, G, inst, vec, two_halves);
+  const bool a4 = (align & 15) == 0 && (G.X & 3) == 0;
+  if (a4 && same) put_run_as<true, true>(P, t0, ip, G, inst, two_halves);
+  else if (a4) put_run_as<true, false>(P, t0, ip, G, inst, two_halves);
+  else if (same) put_run_as<false, true>(P, t0, ip, G, inst, two_halves);
+  else put_run_as<false, false>(P, t0, ip, G, inst, two_halves);
 }
 
 // ---------------------------------------------------------------------------
