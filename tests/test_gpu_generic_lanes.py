@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 from cugip_b200.graph_cut import SINK, SOURCE, GenericGraph
-from oracle import oracle  # the checker
+from oracle import oracle
 
 pytestmark = pytest.mark.gpu
 

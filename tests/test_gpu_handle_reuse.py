@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 from cugip_b200.graph_cut import SINK, SOURCE, Batch, GenericGraph, GridGraph
-from oracle import oracle  # the checker
+from oracle import oracle
 from tests import graphs
 
 pytestmark = pytest.mark.gpu

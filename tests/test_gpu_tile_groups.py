@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 from cugip_b200.graph_cut import SINK, SOURCE, Batch, Policy
-from oracle import oracle  # the checker
+from oracle import oracle
 from tests import graphs
 from tests.gpu_helpers import solve
 

@@ -7,7 +7,7 @@ import pytest
 
 from cugip_b200 import _lib
 from cugip_b200.graph_cut import SINK, SOURCE, Batch, GridGraph
-from oracle import oracle  # the checker
+from oracle import oracle
 from tests import graphs
 
 pytestmark = pytest.mark.gpu
