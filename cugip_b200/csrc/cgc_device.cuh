@@ -35,7 +35,7 @@ enum Dir { PX = 0, MX = 1, PY = 2, MY = 3, PZ = 4, MZ = 5 };
 enum Counter {
   C_BFS0 = 0,      // 3 BFS worklists
   C_SW0 = 3,       // 4 sweep worklists
-  C_ACT = 7,       // active tiles after the last global relabel
+  C_ACT = 7,       // active tiles after the last global relabel (fixed until the next)
   C_ROUNDS = 8,    // BFS rounds executed
   C_SINKT0 = 9,    // 3 slots: tiles that delivered flow to the sink in a sweep
   C_TAKE0 = 12,    // 3 slots: next list entry to hand out in a round (persistent solve)

@@ -355,7 +355,7 @@ __device__ __forceinline__ void solve_body(const DevPool& P, const SolveParams& 
       sc[0] = sc[1] = sc[2] = sc[3] = 0;
       P.cnt[C_SINKT0] = P.cnt[C_SINKT0 + 1] = P.cnt[C_SINKT0 + 2] = 0;
       P.cnt[C_TAKE0] = P.cnt[C_TAKE0 + 1] = P.cnt[C_TAKE0 + 2] = 0;
-      P.cnt[C_INC] = 0;
+      P.cnt[C_INC] = P.cnt[C_ACT] = 0;
     }
     round_no = 0;
     if (!sync()) return;
@@ -386,6 +386,8 @@ __device__ __forceinline__ void solve_body(const DevPool& P, const SolveParams& 
       const int t = t0 + (tid & 31);
       const bool a = t < P.T && __ldcg(P.act + t);
       const int par = a ? __ldcg(P.tpar + t) : 0;
+      const unsigned acts = __ballot_sync(FULL, a);
+      if ((tid & 31) == 0 && acts) atomicAdd(P.cnt + C_ACT, __popc(acts));
       if (prm.exclusive) {  // one list: the whole active set is queued for sweep s
         if (a) P.stamp_sw[(int64_t)(s & 1) * P.T + t] = (uint32_t)(s + 1);
         warp_append(P, a, t, list(3 + (s & 3)), sc + (s & 3));
@@ -396,7 +398,10 @@ __device__ __forceinline__ void solve_body(const DevPool& P, const SolveParams& 
       }
     }
     if (!sync()) return;
-    const int nact = ld_cnt(sc + (s & 3)) + ld_cnt(sc + ((s + 1) & 3));
+    // From a counter of its own: the lists' counters grow as soon as the first
+    // CTA sweeps, and a CTA that read them late would choose another cycle length
+    // or scheduler stage than the others, and meet other grid barriers.
+    const int nact = ld_cnt(P.cnt + C_ACT);
     record(TR_RELABEL_DONE, relabels, nact);
     if (b == 0 && tid == 0 && P.trace && book.ntrace < TRACE_CAP) {  // flow at this relabel (after the barrier)
       unsigned long long f = 0;
