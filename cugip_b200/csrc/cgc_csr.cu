@@ -348,10 +348,16 @@ __global__ void __launch_bounds__(CSR_THREADS, 1) k_csr_solve(CsrDev D, CsrParam
           if (i != slot) v = __ldcg(lc + i);
           a = __ldg(D.row + v) + sub;
           a1 = __ldg(D.row + v + 1);
-          ev = __ldcg(D.e + v);
           hv = __ldcg(D.h + v);
-          rt = __ldcg(D.rT + v);
+          if (sub == 0) {
+            ev = __ldcg(D.e + v);
+            rt = __ldcg(D.rT + v);
+          }
         }
+        // One read for all lanes: neighbours add to the excess meanwhile, and the
+        // lanes share out what is subtracted from it below.
+        ev = __shfl_sync(FULL, ev, 0, W);
+        rt = __shfl_sync(FULL, rt, 0, W);
         if (ev <= 0 || hv >= INF) { ev = 0; a1 = 0; }
         const int e0 = ev;
         if (rt > 0 && hv == 1 && ev > 0) {
