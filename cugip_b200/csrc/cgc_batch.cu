@@ -43,11 +43,22 @@ __global__ void __launch_bounds__(256) k_seg_all(DevPool P, uint8_t* const* __re
 
 static int ensure_tables(Pool& p) {
   if (!p.d_in) {
+    if (!p.bound) CGC_CUDA(cudaEventCreateWithFlags(&p.bound, cudaEventDisableTiming));
     if (int rc = dev_alloc(p.device, &p.d_in, sizeof(int32_t*) * 8 * p.ninst)) return rc;
     if (int rc = dev_alloc(p.device, &p.d_out, sizeof(uint8_t*) * 2 * p.ninst)) return rc;
     p.in_ptrs.assign(8 * (size_t)p.ninst, nullptr);
     p.out_ptrs.assign(2 * (size_t)p.ninst, nullptr);
   }
+  return CGC_OK;
+}
+
+// `bytes` of a table to the device; the copy of pageable memory may end after
+// the call returns, so its end is marked.
+static int copy_table(Pool& p, void* dst, const void* src, size_t bytes) {
+  cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaEventRecord(p.bound, cudaStreamLegacy);
+  if (e != cudaSuccess) p.untracked = true;
+  CGC_CUDA(e);
   return CGC_OK;
 }
 
@@ -63,7 +74,7 @@ int pool_bind_inputs(Pool& p, int inst, const int32_t* capS, const int32_t* capT
     ip[2 + a] = fwd ? fwd[a] : nullptr;
     ip[5 + a] = bwd ? bwd[a] : (fwd ? fwd[a] : nullptr);
   }
-  CGC_CUDA(cudaMemcpy(p.d_in + 8 * (size_t)inst, ip, 8 * sizeof(int32_t*), cudaMemcpyHostToDevice));
+  if ((rc = copy_table(p, p.d_in + 8 * (size_t)inst, ip, 8 * sizeof(int32_t*)))) return rc;
   return ok();
 }
 
@@ -73,8 +84,8 @@ int pool_bind_outputs(Pool& p, int inst, uint8_t* source_side, uint8_t* sink_sid
   if (rc) return rc;
   p.out_ptrs[2 * (size_t)inst] = source_side;
   p.out_ptrs[2 * (size_t)inst + 1] = sink_side;
-  CGC_CUDA(cudaMemcpy(p.d_out + 2 * (size_t)inst, p.out_ptrs.data() + 2 * (size_t)inst, 2 * sizeof(uint8_t*),
-                      cudaMemcpyHostToDevice));
+  if ((rc = copy_table(p, p.d_out + 2 * (size_t)inst, p.out_ptrs.data() + 2 * (size_t)inst, 2 * sizeof(uint8_t*))))
+    return rc;
   return ok();
 }
 
@@ -90,6 +101,8 @@ int pool_enqueue(Pool& p, const cgc_options* opts, int64_t* flows_dev, cudaStrea
     if (rc) return rc;
   }
   DevPool& d = p.dp;
+  NoteUse note(p);
+  note.waited = stream != p.stream;  // the handle's own capture queues nothing
   CGC_CUDA(cudaMemsetAsync(p.back_dev, 0, p.back_bytes, stream));  // statistics, barrier, error word, flows
   k_put_all<<<d.nruns, 128, 0, stream>>>(d, p.d_in);
   note_launch();
@@ -113,8 +126,10 @@ int pool_enqueue(Pool& p, const cgc_options* opts, int64_t* flows_dev, cudaStrea
 // Waits for the last enqueued or replayed batch; reports device errors and
 // refreshes flows and statistics.
 int pool_wait(Pool& p, cudaStream_t stream) {
+  NoteUse note(p);
   if (int rc = queue_back(p, stream)) return rc;
   CGC_CUDA(cudaStreamSynchronize(stream));
+  note.waited = true;
   if (int rc = read_back(p, "batch")) return rc;
   return ok();
 }
@@ -156,6 +171,7 @@ int pool_graph_create(Pool& p, const cgc_options* opts, int64_t* flows_dev) {
 int pool_graph_launch(Pool& p) {
   if (!p.graph_exec) return fail(CGC_ERR_STATE, "graph_launch: no graph (call cgc_batch_graph_create)");
   if (p.pending) return fail(CGC_ERR_STATE, "graph_launch: a host-path solve of this handle was not waited for");
+  NoteUse note(p);
   CGC_CUDA(cudaGraphLaunch(p.graph_exec, p.stream));
   for (int i = 0; i < p.graph_kernels; ++i) note_launch();
   for (auto& u : p.uploaded) u = 0;

@@ -489,6 +489,7 @@ struct cgc_graph {
   int coop_blocks = 0;
   int lanes = 8;  // lanes per vertex in the solve
   bool tlinks = false, solved = false;
+  bool untracked = false;  // a call failed before it had waited for what it queued
   cgc_stats st{};
 };
 
@@ -497,15 +498,21 @@ namespace {
 using cgc::fail;
 using cgc::ok;
 
+// Around calls that queue work: marks the graph where one returns before it
+// has waited.
+struct Queued {
+  cgc_graph* g;
+  bool waited = false;
+  explicit Queued(cgc_graph* graph) : g(graph) {}
+  Queued(const Queued&) = delete;
+  ~Queued() { if (!waited) g->untracked = true; }
+};
+
 void graph_free(cgc_graph* g) {
   if (!g) return;
-  if (g->dbuf) {  // the block may be handed out again: nothing may be using it
-    int cur = 0;
-    const bool other = cudaGetDevice(&cur) == cudaSuccess && cur != g->device && cudaSetDevice(g->device) == cudaSuccess;
-    cudaDeviceSynchronize();
-    if (other) cudaSetDevice(cur);
-    cgc::dev_free(g->dbuf);
-  }
+  // every call that succeeded has waited for its work; a block that something
+  // may still be using is not handed out again
+  if (g->dbuf && (!g->untracked || cgc::wait_for_device(g->device))) cgc::dev_free(g->dbuf);
   delete g;
 }
 
@@ -557,6 +564,7 @@ int graph_create(int32_t n, int64_t m, const int32_t* a, const int32_t* b, const
     const int64_t o_seg = off; off += al(n);
     const int64_t o_bs = off; off += al((int64_t)nb * 4);
     if (int rc2 = dev_alloc(g->device, &g->dbuf, off)) return rc2;
+    Queued queued(g);
     CGC_CUDA(cudaMemsetAsync(g->dbuf, 0, off, g->stream));
     char* base = (char*)g->dbuf;
     CsrDev& d = g->d;
@@ -608,8 +616,7 @@ int graph_create(int32_t n, int64_t m, const int32_t* a, const int32_t* b, const
         CGC_CUDA(cudaStreamSynchronize(g->stream));
         return CGC_OK;
       }();
-      if (rc2) cudaStreamSynchronize(g->stream);
-      dev_free(stage);
+      if (!rc2 || wait_for_device(g->device)) dev_free(stage);
       if (rc2) return rc2;
     }
     int sms = 0;
@@ -620,6 +627,7 @@ int graph_create(int32_t n, int64_t m, const int32_t* a, const int32_t* b, const
     g->lanes = degree >= 12 ? 16 : degree >= 6 ? 8 : 4;
     g->coop_blocks = std::max(1, std::min(sms, grid_blocks((int64_t)n * g->lanes, CSR_THREADS)));
     CGC_CUDA(cudaStreamSynchronize(g->stream));
+    queued.waited = true;
     return CGC_OK;
   }();
   if (rc) {
@@ -647,6 +655,7 @@ int graph_maxflow(cgc_graph* g, const cgc_options* opts, int64_t* flow) {
     for (auto& e : ev)
       if (e) cudaEventDestroy(e);
   };
+  Queued queued(g);
   int rc = [&]() -> int {
     CGC_CUDA(cudaEventRecord(ev[0], g->stream));
     CGC_CUDA(cudaMemsetAsync(d.flow, 0, 8, g->stream));
@@ -675,6 +684,7 @@ int graph_maxflow(cgc_graph* g, const cgc_options* opts, int64_t* flow) {
     CGC_CUDA(cudaEventRecord(ev[2], g->stream));
     CGC_CUDA(cudaEventRecord(ev[3], g->stream));
     CGC_CUDA(cudaEventSynchronize(ev[3]));
+    queued.waited = true;
     int32_t err = 0;
     CGC_CUDA(cudaMemcpy(&err, d.err, 4, cudaMemcpyDeviceToHost));
     if (err == CGC_ERR_TIMEOUT) return fail(CGC_ERR_TIMEOUT, "cgc_graph_maxflow: a grid barrier timed out");
@@ -728,9 +738,11 @@ int cgc_graph_set_tlinks(cgc_graph* g, const int32_t* capS, const int32_t* capT)
   for (int32_t v = 0; v < g->n; ++v)
     if (capS[v] < 0 || capT[v] < 0)
       return cgc::fail(CGC_ERR_ARG, "cgc_graph_set_tlinks: negative capacity at vertex " + std::to_string(v));
+  Queued queued(g);
   CGC_CUDA(cudaMemcpyAsync((void*)g->d.capS, capS, (size_t)g->n * 4, cudaMemcpyHostToDevice, g->stream));
   CGC_CUDA(cudaMemcpyAsync((void*)g->d.capT, capT, (size_t)g->n * 4, cudaMemcpyHostToDevice, g->stream));
   CGC_CUDA(cudaStreamSynchronize(g->stream));
+  queued.waited = true;
   g->tlinks = true;
   return cgc::ok();
 }
@@ -741,20 +753,24 @@ int cgc_graph_get_segments(cgc_graph* g, int which, uint8_t* out, uint8_t mask, 
   if (!g || !out || (which != CGC_SEG_SINK_REACH && which != CGC_SEG_SOURCE_MIN))
     return cgc::fail(CGC_ERR_ARG, "cgc_graph_get_segments: bad arguments");
   if (!g->solved) return cgc::fail(CGC_ERR_STATE, "cgc_graph_get_segments: call maxflow first");
+  Queued queued(g);
   cgc::k_csr_segments<<<cgc::grid_blocks(g->n, 256), 256, 0, g->stream>>>(g->d, which, g->seg, mask, background);
   cgc::note_launch();
   CGC_CUDA(cudaGetLastError());
   CGC_CUDA(cudaMemcpyAsync(out, g->seg, (size_t)g->n, cudaMemcpyDeviceToHost, g->stream));
   CGC_CUDA(cudaStreamSynchronize(g->stream));
+  queued.waited = true;
   return cgc::ok();
 }
 
 int cgc_graph_get_state(cgc_graph* g, int32_t* labels, int32_t* excess) {
   if (!g) return cgc::fail(CGC_ERR_ARG, "cgc_graph_get_state: null graph");
   if (!g->solved) return cgc::fail(CGC_ERR_STATE, "cgc_graph_get_state: call maxflow first");
+  Queued queued(g);
   if (labels) CGC_CUDA(cudaMemcpyAsync(labels, g->d.h, (size_t)g->n * 4, cudaMemcpyDeviceToHost, g->stream));
   if (excess) CGC_CUDA(cudaMemcpyAsync(excess, g->d.e, (size_t)g->n * 4, cudaMemcpyDeviceToHost, g->stream));
   CGC_CUDA(cudaStreamSynchronize(g->stream));
+  queued.waited = true;
   if (labels)
     for (int32_t v = 0; v < g->n; ++v)
       if (labels[v] >= cgc::INF) labels[v] = INT32_MIN;

@@ -690,6 +690,35 @@ int dev_alloc(int device, void** p, size_t bytes) {
   return CGC_OK;
 }
 
+bool wait_for_device(int device) {
+  int cur = 0;
+  const bool other = cudaGetDevice(&cur) == cudaSuccess && cur != device && cudaSetDevice(device) == cudaSuccess;
+  void* q = nullptr;
+  const bool done = cudaMalloc(&q, 1) == cudaSuccess && cudaFree(q) == cudaSuccess;
+  if (other) cudaSetDevice(cur);
+  cudaGetLastError();
+  return done;
+}
+
+bool Pool::idle() {
+  bool told = !untracked;
+  for (cudaEvent_t e : {used, bound, ev[1]})  // no wait for one that was never recorded
+    if (e && cudaEventSynchronize(e) != cudaSuccess) {
+      cudaGetLastError();
+      told = false;
+    }
+  return told || wait_for_device(device);
+}
+
+void Pool::note_use() {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (!used || cudaStreamIsCapturing(stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone ||
+      cudaEventRecord(used, stream) != cudaSuccess) {
+    cudaGetLastError();
+    untracked = true;
+  }
+}
+
 static std::mutex g_pin_mu;
 static char* g_pin = nullptr;
 static uint64_t g_pin_used = 0;
@@ -825,6 +854,7 @@ int pool_create(int32_t count, const int32_t* ext, void* stream, Pool** out) {
   off += al((int64_t)p->back_bytes);
   const int64_t o_tr = off; off += al(2 * TRACE_CAP * 8);
   if (int rc = dev_alloc(p->device, &p->dbuf, off)) return rc;
+  p->untracked = true;  // until the wait below
   p->back_dev = (char*)p->dbuf + o_st;
   CGC_CUDA(cudaMemsetAsync(p->dbuf, 0, off, p->stream));
   char* base = (char*)p->dbuf;
@@ -877,7 +907,7 @@ int pool_create(int32_t count, const int32_t* ext, void* stream, Pool** out) {
   p->host_in.assign(8 * (size_t)count, nullptr);
   p->pinned_cnt = (int32_t*)pinned_take(64 * 4 + p->back_bytes);
   if (!p->pinned_cnt) return fail(CGC_ERR_OOM, "create: pinned host memory");
-  CGC_CUDA(cudaEventCreateWithFlags(&p->inputs_read, cudaEventDisableTiming));
+  for (cudaEvent_t* e : {&p->inputs_read, &p->used}) CGC_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
   for (auto& e : p->ev) CGC_CUDA(cudaEventCreate(&e));
 
   CGC_CUDA(cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, p->device));
@@ -885,6 +915,7 @@ int pool_create(int32_t count, const int32_t* ext, void* stream, Pool** out) {
   CGC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ2, k_sweep_list, WIDE, 0));
   p->sweep_blocks = std::max(1, occ2) * p->sms;
   CGC_CUDA(cudaStreamSynchronize(p->stream));
+  p->untracked = false;
   *out = p.release();
   return ok();
 }
@@ -946,6 +977,8 @@ int pool_put_tlinks(Pool& p, int inst, const int32_t* capS, const int32_t* capT,
   if (inst < 0 || inst >= p.ninst || !capS || !capT) return fail(CGC_ERR_ARG, "set_tlinks: bad arguments");
   const InstGeo& G = p.geo[inst];
   const int64_t N = (int64_t)G.X * G.Y * G.Z;
+  NoteUse note(p);
+  note.waited = host && p.lin;  // host planes are waited for, the table that comes with `lin` is not
   if (int rc = ensure_lin(p, false, host)) return rc;
   int32_t* s = p.lin + p.voff[inst];
   int32_t* c = p.lin + p.sumN + p.voff[inst];
@@ -965,6 +998,8 @@ int pool_put_nlinks(Pool& p, int inst, int axis, const int32_t* fwd, const int32
   const InstGeo& G = p.geo[inst];
   const int64_t N = (int64_t)G.X * G.Y * G.Z;
   const bool same = bwd == fwd;  // symmetric weights: one plane
+  NoteUse note(p);
+  note.waited = host && p.lin;
   if (int rc = ensure_lin(p, !same, host)) return rc;
   int32_t* f = p.lin + (2 + axis) * p.sumN + p.voff[inst];
   int32_t* b = same ? f : p.lin_bwd + axis * p.sumN + p.voff[inst];
@@ -1073,6 +1108,7 @@ int pool_solve_async(Pool& p, const cgc_options* opts) {
     for (int a = 0; a < 3; ++a)
       if (!(p.uploaded[i] & (2u << a))) in[8 * (size_t)i + 2 + a] = in[8 * (size_t)i + 5 + a] = nullptr;
   const SolveParams prm = solve_params(o);
+  NoteUse note(p);
   if (o.persistent > 0 && (prm.learned || prm.trace_cycles))  // buffers and weights before anything is queued
     if (int rc = ensure_sched(p, prm.learned != 0, prm.trace_cycles)) return rc;
   if (p.ninst > 1) {
@@ -1156,6 +1192,7 @@ int pool_solve_async(Pool& p, const cgc_options* opts) {
     p.pending = false;
     return rc;
   }
+  note.waited = true;  // ev[1] marks the end
   return ok();
 }
 
@@ -1194,6 +1231,7 @@ int pool_segments(Pool& p, int inst, int which, uint8_t* out, uint8_t mask, uint
   if (!p.solved) return fail(CGC_ERR_STATE, "get_segments: call maxflow first");
   const InstGeo& G = p.geo[inst];
   const int64_t N = (int64_t)G.X * G.Y * G.Z;
+  NoteUse note(p);
   if ((host || !p.seg_valid || mask != 1 || bg != 0) && !p.segtmp)
     if (int rc = dev_alloc(p.device, &p.segtmp, p.maxN)) return rc;
   const unsigned blocks = (unsigned)std::min<int64_t>(std::max<int64_t>((N + 4095) / 4096, 1), 8 * (int64_t)p.sms);
@@ -1217,6 +1255,7 @@ int pool_segments(Pool& p, int inst, int which, uint8_t* out, uint8_t mask, uint
   CGC_CUDA(cudaGetLastError());
   if (src) CGC_CUDA(cudaMemcpyAsync(out, src, N, host ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice, p.stream));
   CGC_CUDA(cudaStreamSynchronize(p.stream));
+  note.waited = true;
   return ok();
 }
 
@@ -1226,6 +1265,7 @@ int pool_residuals(Pool& p, int inst, int32_t* const res[6], int32_t* resT, int3
   if (!p.solved) return fail(CGC_ERR_STATE, "get_residuals: call maxflow first");
   const InstGeo& G = p.geo[inst];
   const int64_t N = (int64_t)G.X * G.Y * G.Z;
+  NoteUse note(p);
   if (!p.resid)
     if (int rc = dev_alloc(p.device, &p.resid, (size_t)p.maxN * 4)) return rc;
   const int blocks = (int)std::min<int64_t>((N + 255) / 256, 65535);
@@ -1243,6 +1283,7 @@ int pool_residuals(Pool& p, int inst, int32_t* const res[6], int32_t* resT, int3
       if ((rc = one(p.dp.r + d * p.Np, res[d]))) return rc;
   if ((rc = one(p.dp.rT, resT))) return rc;
   if ((rc = one(p.dp.e, excess))) return rc;
+  note.waited = true;
   return ok();
 }
 
@@ -1254,6 +1295,7 @@ int pool_labels(Pool& p, int inst, int32_t* labels) {
   if (!p.solved) return fail(CGC_ERR_STATE, "get_labels: call maxflow first");
   const InstGeo& G = p.geo[inst];
   const int64_t N = (int64_t)G.X * G.Y * G.Z;
+  NoteUse note(p);
   if (!p.resid)
     if (int rc = dev_alloc(p.device, &p.resid, (size_t)p.maxN * 4)) return rc;
   k_unpermute<<<(int)std::min<int64_t>((N + 255) / 256, 65535), 256, 0, p.stream>>>(p.dp, inst, p.dp.h, p.resid);
@@ -1261,6 +1303,7 @@ int pool_labels(Pool& p, int inst, int32_t* labels) {
   CGC_CUDA(cudaGetLastError());
   CGC_CUDA(cudaMemcpyAsync(labels, p.resid, N * 4, cudaMemcpyDeviceToHost, p.stream));
   CGC_CUDA(cudaStreamSynchronize(p.stream));
+  note.waited = true;
   for (int64_t v = 0; v < N; ++v)
     if (labels[v] >= INF) labels[v] = INT32_MIN;
   return ok();

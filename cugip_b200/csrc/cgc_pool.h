@@ -34,6 +34,11 @@ int dev_alloc(int device, void** p, size_t bytes);
 template <typename T>
 int dev_alloc(int device, T** p, size_t bytes) { return dev_alloc(device, reinterpret_cast<void**>(p), bytes); }
 inline void dev_free(void* p) { if (p) cudaFree(p); }
+// Waits until the device has finished all its work: for memory whose last use
+// no event tells.  Freeing an ordinary allocation waits for every stream and,
+// unlike cudaDeviceSynchronize, neither fails beside another thread's stream
+// capture nor ends that capture.  False if it failed.
+bool wait_for_device(int device);
 // Pinned host memory of a handle: a slot of one 64 KB block the process keeps,
 // or a block of its own (null: no memory).
 void* pinned_take(size_t bytes);
@@ -68,6 +73,10 @@ struct Pool {
   uint8_t* segtmp = nullptr;     // maxN bytes for remapped masks (mask / background values)
   int32_t* resid = nullptr;      // maxN int32 for cgc_grid_get_residuals
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};  // solve and kernel timing
+  // the end of what the handle queued besides solves (whose end is ev[1])
+  cudaEvent_t used = nullptr;    // on the handle's stream (note_use)
+  cudaEvent_t bound = nullptr;   // on the legacy stream: the copies of the bound pointers
+  bool untracked = false;        // something was queued behind no event (a stream under capture, a failed record)
   bool pending = false;          // a host-path solve was enqueued and not yet waited for
   int pending_persistent = 1;    // its options' persistent field
   long long launches0 = 0;       // launch counter when it was enqueued
@@ -97,33 +106,41 @@ struct Pool {
   int trace_cap = 0;
   uint64_t sched_wver = 0;
   ~Pool() {
-    if (dbuf) {  // the blocks may be handed out again: nothing may be using them
-      int cur = 0;
-      const bool other = cudaGetDevice(&cur) == cudaSuccess && cur != device && cudaSetDevice(device) == cudaSuccess;
-      cudaDeviceSynchronize();
-      if (other) cudaSetDevice(cur);
-    }
+    const bool ended = idle();
     if (sbuf) cudaFree(sbuf);
     if (tbuf) cudaFree(tbuf);
     if (graph_exec) cudaGraphExecDestroy(graph_exec);
     if (graph) cudaGraphDestroy(graph);
     if (cap_stream) cudaStreamDestroy(cap_stream);
-    dev_free(d_in);
-    dev_free(d_out);
-    dev_free(dbuf);
-    dev_free(lin);
-    dev_free(lin_bwd);
-    dev_free(d_host_in);
-    dev_free(segtmp);
-    dev_free(resid);
+    if (ended) {  // the blocks may be handed out again at once; else they are kept back
+      for (void* q : {(void*)d_in, (void*)d_out, dbuf, (void*)lin, (void*)lin_bwd, (void*)d_host_in, (void*)segtmp,
+                      (void*)resid})
+        dev_free(q);
+      pinned_give(pinned_cnt);
+    }
+    for (auto e : {used, bound})
+      if (e) cudaEventDestroy(e);
     if (inputs_read) cudaEventDestroy(inputs_read);
     for (auto e : ev)
       if (e) cudaEventDestroy(e);
     if (copy_stream) cudaStreamDestroy(copy_stream);
-    pinned_give(pinned_cnt);
   }
+  // Waits for the handle's own work, on whichever stream it is (the streams
+  // themselves may be gone by now); false if that cannot be told.
+  bool idle();
+  // Marks the end of what was queued so far on the handle's stream.
+  void note_use();
 };
 
+// Notes a function's use of the handle's stream when it returns, by whichever
+// path; not where it has waited for the stream.
+struct NoteUse {
+  Pool& p;
+  bool waited = false;
+  explicit NoteUse(Pool& pool) : p(pool) {}
+  NoteUse(const NoteUse&) = delete;
+  ~NoteUse() { if (!waited) p.note_use(); }
+};
 
 int check_device_error(Pool& p, const char* where);
 // device statistics, error word and flows to the host, behind the work on stream
