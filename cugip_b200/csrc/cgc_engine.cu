@@ -9,6 +9,7 @@
 // no host round trip happens per BFS level or push level (the reference
 // synchronises and copies a counter back for every level,
 // detail/graph_cut_relabeling.hpp:962-984, detail/graph_cut_push.hpp:395-459).
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -960,10 +961,42 @@ static int copy_plane(Pool& p, int32_t* dst, const int32_t* src, int64_t N, bool
   return CGC_OK;
 }
 
-// Two planes device to device on the solve stream: small ones by one kernel (a
-// copy command each costs more than the copy), large ones by the copy commands.
+// Whether a kernel on `device` may read `bytes` at p where a copy command would:
+// ordinary memory of that device, aligned, and all of it inside one allocation.
+// Copy commands also take other devices' memory, managed and pinned memory and
+// any alignment, and they answer an invalid range with an error.
+static bool kernel_may_read(const void* p, size_t bytes, int device) {
+  using Query = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+  static const Query query = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    const bool ok = cudaGetDriverEntryPoint("cuPointerGetAttributes", &f, cudaEnableDefault, &found) == cudaSuccess &&
+                    found == cudaDriverEntryPointSuccess;
+    if (!ok) cudaGetLastError();
+    return ok ? reinterpret_cast<Query>(f) : nullptr;
+  }();
+  if (!query || (reinterpret_cast<uintptr_t>(p) & 3)) return false;
+  CUmemorytype type = (CUmemorytype)0;
+  unsigned managed = 1;
+  int ordinal = -1;
+  CUdeviceptr start = 0;
+  size_t size = 0;
+  CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+  void* to[] = {&type, &managed, &ordinal, &start, &size};
+  const CUdeviceptr at = reinterpret_cast<CUdeviceptr>(p);
+  return query(5, what, to, at) == CUDA_SUCCESS && type == CU_MEMORYTYPE_DEVICE && !managed && ordinal == device &&
+         start != 0 && at - start <= size && size - (at - start) >= bytes;
+}
+
+// Two planes device to device on the solve stream, by one kernel where it may
+// read them and they are small: the eight planes of directed n-links take 25 us
+// at 64^3 by kernels and 47 by copy commands (whole solve of 24x20x12: 287 and
+// 309 us).  At 128^3 (33 and 50 us) that is 2 % of the solve and at 200^3 (93 and
+// 133) less, so above 2^18 voxels the copy commands, which take any memory, stay.
 static int copy_two(Pool& p, int32_t* d0, const int32_t* s0, int32_t* d1, const int32_t* s1, int64_t N, bool host) {
-  if (!host && N <= (1 << 18)) {
+  if (!host && N <= (1 << 18) && kernel_may_read(s0, (size_t)N * 4, p.device) && kernel_may_read(s1, (size_t)N * 4, p.device)) {
     k_copy_two<<<(unsigned)((N + 1023) / 1024), 256, 0, p.stream>>>(d0, s0, d1, s1, N);
     note_launch();
     CGC_CUDA(cudaGetLastError());
