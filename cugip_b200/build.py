@@ -23,7 +23,7 @@ VOL_SOURCES = ["cgc_volume.cpp"]
 SOURCES = ["cgc_engine.cu", "cgc_batch.cu", "cgc_autotune.cu", "cgc_sched_train.cu", "cgc_noalloc.cu",
            "cgc_build.cu", "cgc_csr.cu", "cgc_graph.cpp"]
 HEADERS = ["cgc_device.cuh", "cgc_kernels.cuh", "cgc_internal.h", "cgc_pool.h", "cgc_sched.cuh",
-           "cgc_sync.cuh", "cgc_warp.cuh"]
+           "cgc_sync.cuh", "cgc_warp.cuh", "cgc_arcs.h"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

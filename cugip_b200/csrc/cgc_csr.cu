@@ -31,6 +31,7 @@
 #include <vector>
 
 #include "cgc.h"
+#include "cgc_arcs.h"
 #include "cgc_internal.h"
 #include "cgc_pool.h"
 #include "cgc_sync.cuh"
@@ -277,15 +278,15 @@ __global__ void __launch_bounds__(CSR_THREADS, 1) k_csr_solve(CsrDev D, CsrParam
       if (nf == 0) return k;
       if (lead) cb[(k + 2) % 3] = 0;
       for (int i0 = wslot, i = slot; i0 < nf;) {
-        int a = i < nf ? f.x + sub : 0;
-        const int a1 = i < nf ? f.y : 0;
-        for (; __any_sync(FULL, a < a1); a += W) {
-          bool ok = a < a1;
+        ArcWalk<W> a;
+        if (i < nf) a = ArcWalk<W>(f.x, f.y, sub);
+        for (; __any_sync(FULL, a.on()); a.step()) {
+          bool ok = a.on();
           int2 r = make_int2(0, 0);
           if (ok) {
-            const int v = __ldg(D.to + a);
+            const int v = __ldg(D.to + a.at);
             r = arcs_of(v);
-            ok = take(a, v, k);
+            ok = take(a.at, v, k);
           }
           csr_append(ok, r, ln, cb + (k + 1) % 3);
         }
@@ -308,7 +309,7 @@ __global__ void __launch_bounds__(CSR_THREADS, 1) k_csr_solve(CsrDev D, CsrParam
       csr_append(seed, seed ? arcs_of(v) : make_int2(0, 0), D.front, cb + 0);
     }
     if (!sync()) return;
-    const int rounds = bfs([&](int a, int v, int k) {
+    const int rounds = bfs([&](uint32_t a, int v, int k) {
       const int r = __ldcg(D.res + __ldg(D.rev + a));
       // the frontier of round k has height k + 1
       return ldv(D.h + v) == INF && r > 0 && atomicCAS(D.h + v, INF, k + 2) == INF;
@@ -343,11 +344,11 @@ __global__ void __launch_bounds__(CSR_THREADS, 1) k_csr_solve(CsrDev D, CsrParam
       // push step: labels fixed; the vertex's lanes split its excess among the
       // admissible arcs by a saturating prefix sum
       for (int i0 = wslot, i = slot; i0 < ncur; i0 += slots, i += slots) {
-        int a = 0, a1 = 0, ev = 0, hv = INF, rt = 0;
+        ArcWalk<W> a;
+        int ev = 0, hv = INF, rt = 0;
         if (i < ncur) {
           if (i != slot) v = __ldcg(lc + i);
-          a = __ldg(D.row + v) + sub;
-          a1 = __ldg(D.row + v + 1);
+          a = ArcWalk<W>(__ldg(D.row + v), __ldg(D.row + v + 1), sub);
           hv = __ldcg(D.h + v);
           if (sub == 0) {
             ev = __ldcg(D.e + v);
@@ -358,7 +359,7 @@ __global__ void __launch_bounds__(CSR_THREADS, 1) k_csr_solve(CsrDev D, CsrParam
         // lanes share out what is subtracted from it below.
         ev = __shfl_sync(FULL, ev, 0, W);
         rt = __shfl_sync(FULL, rt, 0, W);
-        if (ev <= 0 || hv >= INF) { ev = 0; a1 = 0; }
+        if (ev <= 0 || hv >= INF) { ev = 0; a.stop(); }
         const int e0 = ev;
         if (rt > 0 && hv == 1 && ev > 0) {
           const int dl = min(ev, rt);
@@ -368,13 +369,13 @@ __global__ void __launch_bounds__(CSR_THREADS, 1) k_csr_solve(CsrDev D, CsrParam
             flow += dl;
           }
         }
-        for (; __any_sync(FULL, a < a1 && ev > 0); a += W) {
+        for (; __any_sync(FULL, a.on() && ev > 0); a.step()) {
           unsigned cap = 0;
           int r = 0, u = 0, rv = 0;
-          if (a < a1 && ev > 0) {
-            r = __ldcg(D.res + a);
-            u = __ldg(D.to + a);
-            rv = __ldg(D.rev + a);
+          if (a.on() && ev > 0) {
+            r = __ldcg(D.res + a.at);
+            u = __ldg(D.to + a.at);
+            rv = __ldg(D.rev + a.at);
             if (r > 0 && __ldcg(D.h + u) == hv - 1) cap = (unsigned)min(r, ev);
           }
           unsigned s = cap;
@@ -389,7 +390,7 @@ __global__ void __launch_bounds__(CSR_THREADS, 1) k_csr_solve(CsrDev D, CsrParam
           ev -= (int)__shfl_sync(FULL, s, W - 1, W);
           bool fresh = false;
           if (dl > 0) {
-            D.res[a] = r - dl;  // only v writes this arc in this step
+            D.res[a.at] = r - dl;  // only v writes this arc in this step
             atomicAdd(D.res + rv, dl);
             atomicAdd(D.e + u, dl);
             fresh = atomicExch(D.stamp + u, sid) != sid;
@@ -406,21 +407,21 @@ __global__ void __launch_bounds__(CSR_THREADS, 1) k_csr_solve(CsrDev D, CsrParam
       v = slot < n ? ld_early(ln + slot) : 0;
       const int nn = ldv(cn);
       for (int i0 = wslot, i = slot; i0 < nn; i0 += slots, i += slots) {
-        int a = 0, a1 = 0, hv = INF, mn = INF;
+        ArcWalk<W> a;
+        int hv = INF, mn = INF;
         if (i < nn) {
           if (i != slot) v = __ldcg(ln + i);
-          a = __ldg(D.row + v) + sub;
-          a1 = __ldg(D.row + v + 1);
+          a = ArcWalk<W>(__ldg(D.row + v), __ldg(D.row + v + 1), sub);
           const int ev = __ldcg(D.e + v), rt = __ldcg(D.rT + v);
           hv = __ldcg(D.h + v);
           if (ev <= 0 || (rt > 0 && hv == 1)) hv = INF;
           if (rt > 0) mn = 0;
         }
-        if (hv >= INF) a1 = 0;
-        for (; __any_sync(FULL, a < a1); a += W) {
-          if (a < a1) {
-            const int r = __ldcg(D.res + a);
-            const int hu = ldv(D.h + __ldg(D.to + a));
+        if (hv >= INF) a.stop();
+        for (; __any_sync(FULL, a.on()); a.step()) {
+          if (a.on()) {
+            const int r = __ldcg(D.res + a.at);
+            const int hu = ldv(D.h + __ldg(D.to + a.at));
             if (r > 0) mn = min(mn, hu);
           }
         }
@@ -447,7 +448,7 @@ __global__ void __launch_bounds__(CSR_THREADS, 1) k_csr_solve(CsrDev D, CsrParam
     csr_append(seed, seed ? arcs_of(v) : make_int2(0, 0), D.front, cb + 0);
   }
   if (!sync()) return;
-  const int rrounds = bfs([&](int a, int v, int) {
+  const int rrounds = bfs([&](uint32_t a, int v, int) {
     const int r = __ldcg(D.res + a);
     return ldv(D.reach + v) == 0 && r > 0 && atomicCAS(D.reach + v, 0, 1) == 0;
   });
