@@ -41,24 +41,36 @@ __global__ void __launch_bounds__(256) k_seg_all(DevPool P, uint8_t* const* __re
   }
 }
 
-static int ensure_tables(Pool& p) {
-  if (!p.d_in) {
-    if (!p.bound) CGC_CUDA(cudaEventCreateWithFlags(&p.bound, cudaEventDisableTiming));
-    if (int rc = dev_alloc(p.device, &p.d_in, sizeof(int32_t*) * 8 * p.ninst)) return rc;
-    if (int rc = dev_alloc(p.device, &p.d_out, sizeof(uint8_t*) * 2 * p.ninst)) return rc;
-    p.in_ptrs.assign(8 * (size_t)p.ninst, nullptr);
-    p.out_ptrs.assign(2 * (size_t)p.ninst, nullptr);
-  }
+// `bytes` of a table to the device.  A copy of pageable memory may end after
+// cudaMemcpy returns, and the solve's stream may not be ordered behind it, so
+// its end is waited for.
+static int copy_table(Pool& p, void* dst, const void* src, size_t bytes) {
+  cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
+  if (e != cudaSuccess) p.untracked = true;
+  CGC_CUDA(e);
   return CGC_OK;
 }
 
-// `bytes` of a table to the device; the copy of pageable memory may end after
-// the call returns, so its end is marked.
-static int copy_table(Pool& p, void* dst, const void* src, size_t bytes) {
-  cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaEventRecord(p.bound, cudaStreamLegacy);
-  if (e != cudaSuccess) p.untracked = true;
-  CGC_CUDA(e);
+// The device tables start with null pointers: outputs need not be bound for
+// every instance, and the blocks hold whatever their last handle left there.
+static int ensure_tables(Pool& p) {
+  if (!p.d_out) {
+    p.in_ptrs.assign(8 * (size_t)p.ninst, nullptr);
+    p.out_ptrs.assign(2 * (size_t)p.ninst, nullptr);
+    const size_t in = sizeof(int32_t*) * p.in_ptrs.size(), out = sizeof(uint8_t*) * p.out_ptrs.size();
+    if (!p.d_in) {
+      if (int rc = dev_alloc(p.device, &p.d_in, in)) return rc;
+    }
+    if (int rc = copy_table(p, p.d_in, p.in_ptrs.data(), in)) return rc;
+    uint8_t** d_out = nullptr;
+    if (int rc = dev_alloc(p.device, &d_out, out)) return rc;
+    if (int rc = copy_table(p, d_out, p.out_ptrs.data(), out)) {
+      if (p.idle()) dev_free(d_out);
+      return rc;
+    }
+    p.d_out = d_out;  // both tables are there
+  }
   return CGC_OK;
 }
 
@@ -91,7 +103,7 @@ int pool_bind_outputs(Pool& p, int inst, uint8_t* source_side, uint8_t* sink_sid
 
 // Enqueues one batched solve on `stream` without synchronising the host.
 int pool_enqueue(Pool& p, const cgc_options* opts, int64_t* flows_dev, cudaStream_t stream) {
-  if (!p.d_in) return fail(CGC_ERR_STATE, "enqueue: no device inputs bound");
+  if (!p.d_out) return fail(CGC_ERR_STATE, "enqueue: no device inputs bound");
   if (p.pending) return fail(CGC_ERR_STATE, "enqueue: a host-path solve of this handle was not waited for");
   for (int i = 0; i < p.ninst; ++i)
     if (!p.in_ptrs[8 * (size_t)i]) return fail(CGC_ERR_STATE, "enqueue: instance without bound inputs");

@@ -703,7 +703,7 @@ bool wait_for_device(int device) {
 
 bool Pool::idle() {
   bool told = !untracked;
-  for (cudaEvent_t e : {used, bound, ev[1]})  // no wait for one that was never recorded
+  for (cudaEvent_t e : {used, ev[1]})  // no wait for one that was never recorded
     if (e && cudaEventSynchronize(e) != cudaSuccess) {
       cudaGetLastError();
       told = false;

@@ -73,9 +73,9 @@ struct Pool {
   uint8_t* segtmp = nullptr;     // maxN bytes for remapped masks (mask / background values)
   int32_t* resid = nullptr;      // maxN int32 for cgc_grid_get_residuals
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};  // solve and kernel timing
-  // the end of what the handle queued besides solves (whose end is ev[1])
-  cudaEvent_t used = nullptr;    // on the handle's stream (note_use)
-  cudaEvent_t bound = nullptr;   // on the legacy stream: the copies of the bound pointers
+  // the end of what the handle queued on its stream besides solves, whose end
+  // is ev[1] (note_use)
+  cudaEvent_t used = nullptr;
   bool untracked = false;        // something was queued behind no event (a stream under capture, a failed record)
   bool pending = false;          // a host-path solve was enqueued and not yet waited for
   int pending_persistent = 1;    // its options' persistent field
@@ -118,8 +118,7 @@ struct Pool {
         dev_free(q);
       pinned_give(pinned_cnt);
     }
-    for (auto e : {used, bound})
-      if (e) cudaEventDestroy(e);
+    if (used) cudaEventDestroy(used);
     if (inputs_read) cudaEventDestroy(inputs_read);
     for (auto e : ev)
       if (e) cudaEventDestroy(e);
