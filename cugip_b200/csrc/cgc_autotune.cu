@@ -158,6 +158,7 @@ int pool_autotune(Pool& p, const cgc_options* cands, int32_t n, int32_t repeats,
   if (rc2) return rc2;
   if (best_i < 0) return fail(CGC_ERR_STATE, "autotune: every candidate failed");
   cgc_options b = resolve_options(&cand[best_i]);
+  if (cand[best_i].sweeps_per_relabel < 0) b.sweeps_per_relabel = -b.sweeps_per_relabel;  // exact, as it was timed
   store(size_class(total_voxels(p), p.ninst), b, best_t);
   if (best) *best = b;
   if (best_ms) *best_ms = best_t;

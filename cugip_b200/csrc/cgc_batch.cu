@@ -118,7 +118,7 @@ int pool_enqueue(Pool& p, const cgc_options* opts, int64_t* flows_dev, cudaStrea
   CGC_CUDA(cudaMemsetAsync(p.back_dev, 0, p.back_bytes, stream));  // statistics, barrier, error word, flows
   k_put_all<<<d.nruns, 128, 0, stream>>>(d, p.d_in);
   note_launch();
-  const SolveParams prm = solve_params(o);
+  const SolveParams prm = solve_params(o, opts);
   if (int rc = launch_solve(d, prm, p.device, p.sms, stream)) return rc;
   bool any_out = false;
   for (uint8_t* q : p.out_ptrs) any_out = any_out || q;

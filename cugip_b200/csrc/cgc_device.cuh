@@ -118,6 +118,7 @@ struct SolveParams {
   int L;                 // pulses per tile visit (per region-relabel round)
   int R;                 // region-relabel rounds per tile visit (0: pulses only)
   int K;                 // sweep pairs between global relabels
+  int dense_K;           // the same in cycles with more than 16 active tiles per SM
   int stall;             // relabel after this many sweeps without sink flow (0: never)
   int learned;           // 1: budgets and priorities from the learned scheduler
   int trace_cycles;      // record scheduling traces for the first trace_cycles relabel cycles

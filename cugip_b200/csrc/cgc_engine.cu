@@ -414,16 +414,15 @@ __device__ __forceinline__ void solve_body(const DevPool& P, const SolveParams& 
     if (nact == 0) break;
     // Sweep pairs of this cycle.  Where a sweep costs more than a relabel -- more
     // than 16 active tiles per SM -- a cycle ends after 4 pairs at the latest,
-    // since by then most tiles hold excess that a relabel finds cut off from the
+    // unless the caller asked for an exact number (then dense_K = K), since by then most tiles hold excess that a relabel finds cut off from the
     // sink: 405x377x362 8.9 -> 8.0 ms, 512x512x128 tubes 3.6 -> 3.3, 256^3 3.13
     // -> 3.05, segmentation of 150x140x96 9.1 -> 8.9 (K = 8).  2 pairs are better
     // on balls (7.6 ms) and worse on the segmentation (10.0 ms), whose relabels
     // take long; lower limits on the tiles cost small grids 10 %.
     // A cycle in which the limit on sweeps may be met is a full one, so that a
     // small limit allows the sweeps that it always did.
-    const bool cut = nact > 16 * G && prm.K > 4 &&
-                     sweeps + 2 * prm.K < (int64_t)prm.max_sweeps;
-    const int K = cut ? 4 : prm.K;
+    const bool cut = nact > 16 * G && sweeps + 2 * prm.K < (int64_t)prm.max_sweeps;
+    const int K = cut ? prm.dense_K : prm.K;
     if (sweeps >= prm.max_sweeps) {
       if (b == 0 && tid == 0) raise_error(P, CGC_ERR_NOT_CONVERGED);
       break;
@@ -1060,7 +1059,7 @@ cgc_options resolve_options(const cgc_options* o) {
   r.relabel = 2;
   if (o) {
     if (o->local_pulses > 0) r.local_pulses = std::min(o->local_pulses, 64);
-    if (o->sweeps_per_relabel > 0) r.sweeps_per_relabel = o->sweeps_per_relabel;
+    if (o->sweeps_per_relabel) r.sweeps_per_relabel = (int)std::min<int64_t>(std::abs((int64_t)o->sweeps_per_relabel), 1 << 24);
     if (o->wait_limit_us > 0) r.wait_limit_us = o->wait_limit_us;
     if (o->max_sweeps > 0) r.max_sweeps = o->max_sweeps;
     if (o->persistent) r.persistent = o->persistent;
@@ -1080,12 +1079,14 @@ uint64_t wait_limit_ns(const cgc_options& o) {
   return (uint64_t)(o.wait_limit_us > 0 ? o.wait_limit_us : 20 * 1000 * 1000) * 1000ull;
 }
 
-// Parameters of the persistent solve kernel from resolved options.
-SolveParams solve_params(const cgc_options& o) {
+// Parameters of the persistent solve kernel from resolved options and the
+// caller's (may be null).
+SolveParams solve_params(const cgc_options& o, const cgc_options* given) {
   SolveParams prm;
   prm.L = o.local_pulses;
   prm.R = o.region_relabels;
   prm.K = o.sweeps_per_relabel;
+  prm.dense_K = given && given->sweeps_per_relabel < 0 ? prm.K : std::min(prm.K, 4);
   prm.stall = o.stall_sweeps;
   prm.learned = o.learned;
   prm.trace_cycles = o.trace_cycles > 0 ? o.trace_cycles : 0;
@@ -1140,7 +1141,7 @@ int pool_solve_async(Pool& p, const cgc_options* opts) {
   for (int i = 0; i < p.ninst; ++i)
     for (int a = 0; a < 3; ++a)
       if (!(p.uploaded[i] & (2u << a))) in[8 * (size_t)i + 2 + a] = in[8 * (size_t)i + 5 + a] = nullptr;
-  const SolveParams prm = solve_params(o);
+  const SolveParams prm = solve_params(o, opts);
   NoteUse note(p);
   if (o.persistent > 0 && (prm.learned || prm.trace_cycles))  // buffers and weights before anything is queued
     if (int rc = ensure_sched(p, prm.learned != 0, prm.trace_cycles)) return rc;

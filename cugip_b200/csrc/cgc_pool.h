@@ -151,7 +151,7 @@ int pool_put_tlinks(Pool& p, int inst, const int32_t* capS, const int32_t* capT,
 int pool_put_nlinks(Pool& p, int inst, int axis, const int32_t* fwd, const int32_t* bwd, bool host);
 cgc_options resolve_options(const cgc_options* o);
 uint64_t wait_limit_ns(const cgc_options& o);
-SolveParams solve_params(const cgc_options& o);
+SolveParams solve_params(const cgc_options& o, const cgc_options* given);
 int pool_solve(Pool& p, const cgc_options* opts);
 // host path in two halves: enqueue a solve of the set_* inputs on p.stream
 // (no host synchronisation), then wait for it and read flows and statistics

@@ -66,7 +66,7 @@ typedef struct cgc_options {
   int32_t struct_size;
   int32_t local_pulses;       /* push/relabel pulses per region-relabel round (1..64), default 4 */
   int32_t sweeps_per_relabel; /* sweep pairs between global relabels, default 8 (persistent: at most 4 while there
-                                 are more than 16 active tiles per SM) */
+                                 are more than 16 active tiles per SM; -n asks for n pairs in every cycle) */
   int32_t wait_limit_us;      /* bound of every device-side wait (grid barriers of the persistent
                                  solve), in microseconds; default 20 s.  A wait that runs out ends
                                  the solve with CGC_ERR_TIMEOUT; the handle stays usable */
