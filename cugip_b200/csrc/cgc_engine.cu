@@ -274,7 +274,7 @@ __device__ __forceinline__ void solve_body(const DevPool& P, const SolveParams& 
   int32_t* const sc = P.cnt + C_SW0;
   uint32_t bfs_id = 1;
   int s = 0;        // sweep index; sweep s uses list 3 + (s & 3) and stamp id s + 1
-  int sweeps = 0, rounds = 0, relabels = 0, traced = 0;
+  int sweeps = 0, rounds = 0, relabels = 0, traced = 0, spare = 0;
   // block 0 records one phase step (after the barrier that ended it)
   auto record = [&](unsigned long long kind, long long index, int tiles) {
     if (b == 0 && tid == 0 && P.trace && book.ntrace < TRACE_CAP) {
@@ -419,14 +419,14 @@ __device__ __forceinline__ void solve_body(const DevPool& P, const SolveParams& 
     // -> 3.05, segmentation of 150x140x96 9.1 -> 8.9 (K = 8).  2 pairs are better
     // on balls (7.6 ms) and worse on the segmentation (10.0 ms), whose relabels
     // take long; lower limits on the tiles cost small grids 10 %.
-    // A cycle in which the limit on sweeps may be met is a full one, so that a
-    // small limit allows the sweeps that it always did.
-    const bool cut = nact > 16 * G && sweeps + 2 * prm.K < (int64_t)prm.max_sweeps;
-    const int K = cut ? prm.dense_K : prm.K;
-    if (sweeps >= prm.max_sweeps) {
+    const int K = nact > 16 * G ? prm.dense_K : prm.K;
+    // The limit on sweeps is checked before a cycle, so full cycles run up to
+    // 2 K - 1 sweeps past it; a solve with shorter ones may run as many.
+    if (sweeps >= prm.max_sweeps + spare) {
       if (b == 0 && tid == 0) raise_error(P, CGC_ERR_NOT_CONVERGED);
       break;
     }
+    if (K < prm.K) spare = 2 * prm.K - 1;
     // ------------------------------------------------ learned scheduler
     const int cycle = relabels - 1;
     const bool tracing = prm.trace_cycles > cycle;

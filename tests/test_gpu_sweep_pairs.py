@@ -3,6 +3,7 @@ or, with a negative number, exactly as many as the caller asks for.  Batches of
 chains in which excess moves a tile per sweep tell the cycles apart."""
 import pytest
 
+from cugip_b200._lib import CgcError
 from cugip_b200.graph_cut import Batch, Policy
 
 pytestmark = pytest.mark.gpu
@@ -64,3 +65,20 @@ def test_negative_pairs_elsewhere():
     with GenericGraph(X * Y * Z, *e) as g:
         g.set_tweights(c[0], c[1])
         assert g.max_flow(Policy(sweeps_per_relabel=-3)) == f0
+
+
+@pytest.mark.parametrize("max_sweeps", [1, 16, 17, 32])
+@pytest.mark.parametrize("pairs", [0, 8, 16])
+def test_limit_on_sweeps_allows_what_full_cycles_would(pairs, max_sweeps):
+    """A limit is checked before each cycle, so cycles of n pairs run it up to the
+    next multiple of 2n sweeps; shortened cycles must not stop a solve earlier,
+    and must still stop one that needs much more."""
+    full = 2 * (pairs or 8)
+    allowed = -(-max_sweeps // full) * full
+    with Chains(allowed) as c:  # a tile per sweep: the last allowed sweep delivers the flow
+        c.solve(Policy(sweeps_per_relabel=pairs, max_sweeps=max_sweeps))
+    with Chains(allowed + 2 * full) as c:
+        c.batch.enqueue(Policy(sweeps_per_relabel=pairs, max_sweeps=max_sweeps))
+        with pytest.raises(CgcError) as e:
+            c.batch.wait()
+        assert e.value.code == 5  # CGC_ERR_NOT_CONVERGED
