@@ -202,6 +202,10 @@ union TileShared {  // size a multiple of 16: the members are aligned
   SweepShared sw;
   BfsShared bfs;
 };
+// wide visits and warp visits use the groups' memory together
+static_assert(sizeof(WideShared) <= GROUPS * sizeof(TileShared) &&
+              GROUPS * GROUP / 32 * WREL_SMEM * sizeof(unsigned short) <= GROUPS * sizeof(TileShared) &&
+              sizeof(TileShared) % 16 == 0 && GROUPS * GROUP == WIDE, "shared memory of the solve's visits");
 
 // Bookkeeping of a CTA that one thread updates: kept out of the registers,
 // which the visits need.

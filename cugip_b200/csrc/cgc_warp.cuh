@@ -72,12 +72,16 @@ __device__ inline void bfs_init_tile_w(const DevPool& P, const int t, const bool
 constexpr int WREL_SMEM = HROWS * 8;  // 16-bit heights per warp
 
 // The fixed point of one visit in 32-bit heights on the tile's plane in
-// memory, for a tile with heights beyond 16 bits around it.  Returns the
-// lane's changed faces in bits 0..5, bit 6: something changed.
+// memory, for a tile with heights beyond 16 bits around it.  nb: in lane d the
+// (checked) neighbour along d, or -1.  Returns the lane's changed faces in bits
+// 0..5, bit 6: something changed.
 template <bool INVAL>
-__device__ __noinline__ unsigned relabel_far_w(int32_t* h, const uint8_t* rmask, const int32_t* nbr, int T, int t) {
+__device__ __noinline__ unsigned relabel_far_w(int32_t* h, const uint8_t* rmask, int nb, int t) {
   const int lane = threadIdx.x & 31;
   volatile int32_t* const H = h;
+  int nt[6];
+#pragma unroll
+  for (int d = 0; d < 6; ++d) nt[d] = __shfl_sync(FULL, nb, d);
   unsigned out = 0;
   for (int it = 0; it < 1200; ++it) {
     bool ch = false;
@@ -87,13 +91,13 @@ __device__ __noinline__ unsigned relabel_far_w(int32_t* h, const uint8_t* rmask,
       const unsigned m = rmask[g];
       const int old = H[g];
       int n = INVAL ? ((m & 64u) ? 1 : INF) : old;
+#pragma unroll
       for (int d = 0; d < 6; ++d) {
         if (!((m >> d) & 1u)) continue;
         int64_t u = g + loff(d);
         if (!inside(d, x, y, z)) {
-          const int nt = nbr[d * T + t];
-          if (nt < 0) continue;
-          u = (int64_t)nt * TV + i + xoff(d);
+          if (nt[d] < 0) continue;
+          u = (int64_t)nt[d] * TV + i + xoff(d);
         }
         n = min(n, H[u] + 1);
       }
@@ -164,7 +168,7 @@ __device__ __forceinline__ int relabel_tile_w(const DevPool& P, const int t, uns
   unsigned faces = 0;
   bool act = false;
   if (__any_sync(FULL, far)) {
-    faces = relabel_far_w<INVAL>(P.h, P.rmask, P.nbr, P.T, t);
+    faces = relabel_far_w<INVAL>(P.h, P.rmask, nb, t);
     if (!INVAL) {
       for (int k = 0; k < 16; ++k)
         act = act || ((P.rmask[base + 16 * lane + k] & 128u) && *(volatile int32_t*)(P.h + base + 16 * lane + k) < INF);
