@@ -116,7 +116,8 @@ __global__ void k_csr_degree(int64_t m, const int32_t* __restrict__ a, const int
 // exclusive scan, pass 1: each block scans SCAN_BLOCK entries
 __global__ void __launch_bounds__(SCAN_BLOCK) k_scan_block(const int32_t* in, int32_t* out, int32_t* bsum, int n) {
   __shared__ int32_t ws[SCAN_BLOCK / 32];
-  const int i = blockIdx.x * SCAN_BLOCK + threadIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t i = blockIdx.x * (int64_t)SCAN_BLOCK + threadIdx.x;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int v = i < n ? in[i] : 0;
   int x = v;
 #pragma unroll
@@ -181,8 +182,8 @@ __global__ void __launch_bounds__(SCAN_BLOCK) k_scan_sums(int32_t* bsum, int nb,
 
 // pass 3: add the block offsets
 __global__ void k_scan_add(int32_t* out, const int32_t* bsum, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] += bsum[i / SCAN_BLOCK];
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    out[i] += bsum[i / SCAN_BLOCK];
 }
 
 __global__ void k_csr_scatter(int64_t m, const int32_t* __restrict__ a, const int32_t* __restrict__ b,
