@@ -250,23 +250,6 @@ __device__ __forceinline__ void queue_tile(const DevPool& P, uint32_t* stamp, in
   }
 }
 
-
-// block-wide int64 sum (512 threads); result valid in thread 0
-__device__ __forceinline__ long long block_sum64(long long v, long long* red) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane == 0) red[w] = v;
-  __syncthreads();
-  long long s = 0;
-  if (threadIdx.x < 32) {
-    s = (lane < (int)(blockDim.x >> 5)) ? red[lane] : 0;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-  }
-  return s;
-}
-
 // Shared state of one tile group.
 struct alignas(16) SweepShared {
   int h[2][HROWS * 8];  // heights, double buffered by pulse

@@ -95,7 +95,6 @@ struct Pool {
   std::vector<uint8_t*> out_ptrs;        // 2 per instance: source side, sink side
   const int32_t** d_in = nullptr;        // device copy of in_ptrs
   uint8_t** d_out = nullptr;             // device copy of out_ptrs
-  bool tables_dirty = true;
   cudaStream_t cap_stream = nullptr;     // capture stream (the legacy stream cannot be captured)
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graph_exec = nullptr;

@@ -70,18 +70,19 @@ typedef struct cgc_options {
   int32_t wait_limit_us;      /* bound of every device-side wait (grid barriers of the persistent
                                  solve), in microseconds; default 20 s.  A wait that runs out ends
                                  the solve with CGC_ERR_TIMEOUT; the handle stays usable */
-  int32_t max_sweeps;         /* safety cap on sweeps, default 1<<17; CGC_ERR_NOT_CONVERGED when reached */
+  int32_t max_sweeps;         /* safety cap on sweeps, default 1<<17, checked before each relabel cycle (a solve may run
+                                 2 * sweeps_per_relabel - 1 past it); CGC_ERR_NOT_CONVERGED when reached */
   int32_t persistent;         /* 1 = one cooperative launch per solve (default), -1 = host loop */
   int32_t region_relabels;    /* region-relabel rounds per tile visit (default 2, -1 = none) */
   int32_t stall_sweeps;       /* persistent: relabel early after this many sweep pairs without sink flow (0 = never) */
   int32_t ctas_per_sm;        /* accepted and without effect: the solve runs one CTA of four 128-thread tile groups
                                  per SM, which is the fastest shape for every workload this selected between */
   int32_t learned;            /* persistent: learned scheduler, 1 = budgets + priorities, 2 = budgets only
-                                 (both only in cycles with more active tiles than twice the CTAs), 3 = budgets
+                                 (both only in cycles with more than 8 active tiles per SM), 3 = budgets
                                  capped at local_pulses in every cycle + priorities where 1 uses them */
   int32_t trace_cycles;       /* persistent: record scheduling traces of the first trace_cycles relabel cycles */
   int32_t bfs_warp_min;       /* accepted and without effect: BFS rounds visit a tile with a 128-thread group,
-                                 or, where tiles outnumber the SMs, with a warp */
+                                 or, from more than 4 tiles per SM on, with a warp */
   int32_t exclusive;          /* persistent: 1 = every sweep visits each queued tile, except a tile that has a
                                  face neighbour of the sweep's parity queued for the same sweep (which waits one
                                  sweep); 0 = checkerboard sweeps, one parity at a time (the default) */
@@ -128,7 +129,11 @@ int cgc_init(int device);
  * Replaces cugip::Graph<TFlow>::set_vertex_count
  * (include/cugip/advanced_operations/graph_cut.hpp:213-237): allocates all
  * device state for an X*Y*Z grid (about 40 bytes per voxel, padded to 8^3
- * tiles).  stream may be NULL (legacy default stream). */
+ * tiles).  stream may be NULL (legacy default stream).
+ * Destroying a grid, batch or graph waits for the work it has queued.  Freed
+ * blocks of at most 128 MB are kept for later handles, up to 256 MB per device;
+ * the driver takes them back when another allocation of the process needs the
+ * memory. */
 int cgc_grid_create(int32_t X, int32_t Y, int32_t Z, void* stream, cgc_grid** out);
 int cgc_grid_destroy(cgc_grid* g);
 
@@ -293,11 +298,11 @@ int cgc_batch_wait(cgc_batch* b, int64_t* flows);
 /* Autotuner (replaces the compile-time policies of
  * detail/graph_cut_policies.hpp:23-89 with measured choices).  Times each
  * candidate option set (n == 0: a built-in grid over local_pulses,
- * region_relabels, sweeps_per_relabel and ctas_per_sm) `repeats` times on the
- * grid's or batch's current capacities (set with the set_* calls, or bound
- * device inputs), writes the fastest to *best (and its time in ms to
- * *best_ms, either may be NULL) and caches it for the size class; the
- * capacities are restored, so maxflow can follow directly.  With the
+ * region_relabels and sweeps_per_relabel) `repeats` times on the grid's or
+ * batch's current capacities (set with the set_* calls, or bound device
+ * inputs), writes the fastest to *best (and its time in ms to *best_ms, either
+ * may be NULL) and caches it for the size class; the capacities are restored,
+ * so maxflow can follow directly.  With the
  * environment variable CGC_AUTOTUNE_CACHE naming a file, results are appended
  * to it and read back by cgc_autotune_lookup in later processes. */
 int cgc_grid_autotune(cgc_grid* g, const cgc_options* candidates, int32_t n, int32_t repeats,
