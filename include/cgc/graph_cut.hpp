@@ -52,7 +52,7 @@ static_assert(sizeof(EdgeRecord) == 8, "EdgeRecord layout");
 struct GraphCutPolicy {
   int local_pulses = 0;        // pulses per region-relabel round of a tile visit
   int region_relabels = 0;     // region relabels per tile visit (-1: none)
-  int sweeps_per_relabel = 0;  // sweep pairs between exact global relabels
+  int sweeps_per_relabel = 0;  // sweep pairs between exact global relabels (-n: n in every cycle)
   int persistent = 0;          // 1: one cooperative launch, -1: host loop
   int wait_limit_us = 0;       // bound of every device-side wait in microseconds (0: 20 s)
   int max_sweeps = 0;          // safety cap (0: default)
